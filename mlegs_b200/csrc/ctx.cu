@@ -10,6 +10,10 @@
 
 thread_local std::vector<void*>* mlegs_host::g_allocs = nullptr;
 
+// A PFF image up to this size: TOFP of several fields as one launch per stage
+// (tofp_pipe); above it, groups of three fields with the stages overlapped.
+static constexpr size_t PIPE_ALL_BYTES = (size_t)8 << 20;
+
 // ====================================================================== set-up
 namespace {
 
@@ -283,14 +287,14 @@ void mlegs_ctx::init(const mlegs_params& prm) {
         k_proj_comp(g, D, 1, compD, s);
         k_proj_comp(g, T, 0, compT, s);
     }
-    if (p.precision == MLEGS_PREC_FP64 && fold_bulk_supported(g, d.NRCHOPDIM + 1)) {
-        fc_pf = dalloc<double>(fold_table_doubles(g, d.NRCHOPDIM + 1));
-        k_fold_table(g, pf, d.NRCHOPDIM + 1, 1, fc_pf, s);
+    if (p.precision == MLEGS_PREC_FP64 && fold_bulk_supported(g, d.NRCHOPDIM)) {
+        fc_pf = dalloc<double>(fold_table_doubles(g, d.NRCHOPDIM));
+        k_fold_table(g, pf, d.NRCHOPDIM + 1, d.NRCHOPDIM, 1, fc_pf, s);
         double** fcs[3] = {&fc_V, &fc_D, &fc_T};
         const double* W[3] = {V, D, T};
         for (int q = 0; q < 3; ++q) {
             *fcs[q] = dalloc<double>(fold_table_doubles(g, d.NRCHOPDIM));
-            k_fold_table(g, W[q], d.NRCHOPDIM, 0, *fcs[q], s);
+            k_fold_table(g, W[q], d.NRCHOPDIM, d.NRCHOPDIM, 0, *fcs[q], s);
         }
     }
 
@@ -409,7 +413,8 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     lnslots = dalloc<double>(nslots);
     CK(cudaMemsetAsync(lnslots, 0, nslots * sizeof(double), s));
     scratch = dalloc<double2>(d.cap());
-    for (double2*& q : pbuf) q = dalloc<double2>(d.cap());
+    pipe_group = d.pff() * sizeof(double2) <= PIPE_ALL_BYTES ? BATCH : 3;
+    for (int q = 0; q < (pipe_group == BATCH ? BATCH : 2 * pipe_group); ++q) pbuf[q] = dalloc<double2>(d.pff());
     size_t nsys = (size_t)d.NTCHOPDIM * d.NXCHOPDIM;
     solve_scr = dalloc<double>((size_t)d.NRCHOPDIM * 4 * nsys);
     size_t ref_max = (size_t)d.NDIMR * d.NDIMTH * d.NX;
@@ -484,6 +489,7 @@ void mlegs_ctx::ln_from_coef(double* ln, const double2* data, double scale) {
 }
 
 // ====================================================================== physics
+// PSIN, CHIN, BNout may share buffers with the inputs (written after the last read).
 // CALC_BOUSSI_FORCE(PSI, CHI, B, PSIN, CHIN, BN), mod_boussinesq.f90:317-410.
 void mlegs_ctx::force(const Field* PSI, const Field* CHI, const Field* B, Field* PSIN, Field* CHIN, Field* BNout) {
     Field *RUR = tmp(), *RUP = tmp(), *UZ = tmp(), *ROR = tmp(), *ROP = tmp(), *OZ = tmp(), *RBR = tmp(),
@@ -492,12 +498,19 @@ void mlegs_ctx::force(const Field* PSI, const Field* CHI, const Field* B, Field*
     grad(B, RBR, RBP, BZ, P3);
     pc2vel(PSI, CHI, RUR, RUP, UZ, P3);
     pc2vor(PSI, CHI, ROR, ROP, OZ, P3);
-    copy0(W, B, 0);  // W = B; TOFP(W) after CHOPSET(-3)
-    // TOFP up to PFP; the HORFFT(+1) of each field happens inside the fused kernel
+    // TOFP up to PFP; the HORFFT(+1) of each field happens inside the fused kernel.
+    // W = B, TOFP(W) after CHOPSET(-3): the FP64 GEMM reads only the rows that COPY0
+    // keeps, so it takes B itself; the derivative fields carry no log term.
+    if (split_S) copy0(W, B, 0);
     {
         Field* const fs[10] = {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ, W};
         const int pads[10] = {P3, P3, P3, P3, P3, P3, P3, P3, P3, 0};
-        tofp_pipe(fs, pads, 10);
+        const double2* src[10];
+        const double* ln[10] = {};
+        for (int q = 0; q < 10; ++q) src[q] = fs[q]->data;
+        if (!split_S) src[9] = B->data;
+        ln[9] = B->ln;
+        tofp_pipe(fs, pads, 10, nullptr, src, ln);
     }
     // VPRODSUB + VDOTPSUB + the linear terms (385-391), then HORFFT(-1) of the results
     Field *NR = tmp(), *NP = tmp(), *NZ = tmp(), *BN = tmp();
@@ -505,12 +518,20 @@ void mlegs_ctx::force(const Field* PSI, const Field* CHI, const Field* B, Field*
                              OZ->data,  RBR->data, RBP->data, BZ->data,  W->data};
     double2* out[4] = {NR->data, NP->data, NZ->data, BN->data};
     k_theta_fused(g, fft, in, out, p.omega, p.bv0, 1, s);
+    Field* Wf = W;  // W = DEL2(CHIN) in FFF
+    if (!split_S && fc_V) {
+        for (Field* f : {NR, NP, NZ, BN}) f->space = MLEGS_PFP;
+        double2* const pff[4] = {RUR->data, RUP->data, UZ->data, ROR->data};
+        project_toff(NR, NP, NZ, BN, pff, PSIN, Wf, BNout);
+        idel2ln(Wf, CHIN, 0);
+        for (Field* f : {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ, W, NR, NP, NZ, BN}) rel(f);
+        return;
+    }
     for (Field* f : {NR, NP, NZ, BN}) {
         f->space = MLEGS_PFP;
         ln_zero(f);
     }
-    for (Field* f : {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ, W}) rel(f);
-    Field* Wf = tmp();  // W = DEL2(CHIN) in FFF
+    for (Field* f : {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ}) rel(f);
     project(NR, NP, NZ, PSIN, Wf, 1, 0.0);
     idel2ln(Wf, CHIN, 0);
     toff(BN, 0);
@@ -957,7 +978,13 @@ void mlegs_ctx::nonlin(const Field* B, Field* RUR, Field* RUP, Field* UZ, Field*
         f->space = MLEGS_PFP;
         CK(cudaMemsetAsync(f->ln, 0, sizeof(double), s2));
     }
-    if (!k_verfft4(g, fft, BN->data, pbuf[0], -1, s2)) k_verfft_f(g, fft, BN->data, pbuf[0], s2);
+    {
+        VerBatch v{};
+        v.n = 1;
+        v.src[0] = BN->data;
+        v.dst[0] = pbuf[0];
+        verfft_batch(v, -1, s2);
+    }
     fold(0, pf, d.NRCHOPDIM + 1, pbuf[0], BN->data, 0 | 2, 0, 0, 0, s2);
     CK(cudaMemsetAsync(BN->ln, 0, sizeof(double), s2));
     BN->space = MLEGS_FFF;

@@ -69,7 +69,11 @@ struct mlegs_ctx {
     cudaStream_t s2 = nullptr;         // second stream of the RTRAN(+1) -> VERFFT(+1) pipeline
     cudaEvent_t evs[64] = {};          // fork/join events, used in rotation
     int ev_next = 0;
-    double2* pbuf[3] = {};             // PFF images in flight between the two stages
+    // TOFP of several fields (tofp_pipe): fields per launch, and the PFF images
+    // between RTRAN(+1) and VERFFT(+1) (pipe_group of them, twice that when the
+    // two stages overlap)
+    int pipe_group = 1;
+    double2* pbuf[BATCH] = {};
     int dev = 0;
     std::string err;
     int64_t launches = 0;
@@ -122,10 +126,10 @@ struct mlegs_ctx {
         }
         // RTRAN(-1) (PF with the Gauss weights) on the bulk-copy pipeline when its table exists
         if (w == 0 && (mode & 2) && Wt == pf && fc_pf) {
-            const double* wc[1] = {fc_pf};
-            const double2* x[1] = {in};
-            const int md[1] = {mode & 1}, sc[1] = {scale};
-            k_fold_bulk(g, wc, x, md, sc, 1, 1, out, nullptr, wt_rows, pad, accumulate, st);
+            const FoldSeg seg[1] = {{fc_pf, in, mode & 1, scale}};
+            const int first[2] = {0, 1};
+            double2* const outs[1] = {out};
+            k_fold_bulk(g, seg, first, 1, outs, d.NRCHOPDIM, pad, accumulate, st);
             return;
         }
         k_fold_gemm(g, Wt, wt_rows, in, out, mode, scale, accumulate, pad, st);
@@ -304,39 +308,79 @@ struct mlegs_ctx {
     }
 
     // TOFP of FFF fields up to PFP (RTRAN(+1) then VERFFT(+1), the reference's
-    // order per field) as a two-stream pipeline: the RTRAN(+1) GEMM of field
-    // i + 1 on s runs beside the VERFFT(+1) of field i on s2, through three
-    // rotating PFF buffers.  Each field ends in its own buffer, in PFP, LN 0.
+    // order per field).  Each field ends in its own buffer, in PFP, LN 0; src and
+    // ln, when given, are the FFF data and LN slots read instead of the fields' own
+    // (null ln entries: no log term).  Small grids (pipe_group = BATCH) run all
+    // fields in one launch per stage: one field alone leaves most of the chip idle
+    // and each launch costs a few us.  Large ones run groups of pipe_group fields
+    // as a two-stream pipeline, the GEMM of a group on s beside the VERFFT of the
+    // group before it on s2, through two sets of PFF images.
     cudaEvent_t next_event() {
         cudaEvent_t e = evs[ev_next];
         ev_next = (ev_next + 1) % 64;
         return e;
     }
-    void tofp_pipe(Field* const* fs, const int* pads, int n, const cudaEvent_t* ready = nullptr) {
-        for (int i = 0; i < n; ++i) require(fs[i], MLEGS_FFF, "RTRAN");
-        cudaEvent_t e0 = next_event();
-        CK(cudaEventRecord(e0, s));
-        CK(cudaStreamWaitEvent(s2, e0, 0));
-        cudaEvent_t done[3] = {nullptr, nullptr, nullptr};  // last VERFFT reading pbuf[j]
-        for (int i = 0; i < n; ++i) {
-            Field* f = fs[i];
-            double2* buf = pbuf[i % 3];
-            if (done[i % 3]) CK(cudaStreamWaitEvent(s, done[i % 3], 0));
-            if (ready && ready[i]) CK(cudaStreamWaitEvent(s, ready[i], 0));  // field made on s2
-            if (split_S)
-                k_split_b2p(g, split_S, split_img, split_eA, f->data, buf, f->ln, pads[i], split_err, split_wait, s);
-            else
-                k_rtran_b2p(g, f->data, buf, f->ln, pads[i], s);
-            cudaEvent_t eb = next_event();
-            CK(cudaEventRecord(eb, s));
-            CK(cudaStreamWaitEvent(s2, eb, 0));
-            if (!k_verfft4(g, fft, buf, f->data, +1, s2)) k_verfft_b(g, fft, buf, f->data, s2);
-            CK(cudaMemsetAsync(f->ln, 0, sizeof(double), s2));  // RTRAN zeroes LN (off the GEMM stream)
-            cudaEvent_t ev = next_event();
-            CK(cudaEventRecord(ev, s2));
-            done[i % 3] = ev;
-            f->space = MLEGS_PFP;
+    void rtran_batch(const B2PBatch& f, cudaStream_t st) {
+        if (!split_S) {
+            k_rtran_b2p_batch(g, f, st);
+            return;
         }
+        for (int q = 0; q < f.n; ++q)
+            k_split_b2p(g, split_S, split_img, split_eA, f.in[q], f.out[q], f.ln[q], f.pad[q], split_err, split_wait,
+                        st);
+    }
+    void verfft_batch(const VerBatch& f, int dir, cudaStream_t st) {
+        if (k_verfft4_batch(g, fft, f, dir, st)) return;
+        for (int q = 0; q < f.n; ++q) {
+            if (dir > 0) k_verfft_b(g, fft, f.src[q], f.dst[q], st);
+            else k_verfft_f(g, fft, f.src[q], f.dst[q], st);
+            if (f.zln[q]) CK(cudaMemsetAsync(f.zln[q], 0, sizeof(double), st));
+        }
+    }
+    void tofp_pipe(Field* const* fs, const int* pads, int n, const cudaEvent_t* ready = nullptr,
+                   const double2* const* src = nullptr, const double* const* ln = nullptr) {
+        if (!src)
+            for (int i = 0; i < n; ++i) require(fs[i], MLEGS_FFF, "RTRAN");
+        const bool all = pipe_group >= BATCH;
+        if (!all) {
+            cudaEvent_t e0 = next_event();
+            CK(cudaEventRecord(e0, s));
+            CK(cudaStreamWaitEvent(s2, e0, 0));
+        }
+        cudaEvent_t done[2] = {nullptr, nullptr};  // last VERFFT reading image set j
+        for (int i0 = 0, set = 0; i0 < n; i0 += pipe_group, set ^= 1) {
+            const int cnt = std::min(pipe_group, n - i0);
+            B2PBatch b{};
+            VerBatch v{};
+            b.n = v.n = cnt;
+            for (int q = 0; q < cnt; ++q) {
+                Field* f = fs[i0 + q];
+                double2* buf = pbuf[(all ? 0 : set * pipe_group) + q];
+                b.in[q] = src ? src[i0 + q] : f->data;
+                b.out[q] = buf;
+                b.ln[q] = ln ? ln[i0 + q] : f->ln;
+                b.pad[q] = pads[i0 + q];
+                v.src[q] = buf;
+                v.dst[q] = f->data;
+                v.zln[q] = f->ln;  // RTRAN zeroes LN
+                if (ready && ready[i0 + q]) CK(cudaStreamWaitEvent(s, ready[i0 + q], 0));  // field made on s2
+            }
+            if (done[set]) CK(cudaStreamWaitEvent(s, done[set], 0));
+            rtran_batch(b, s);
+            if (all) {
+                verfft_batch(v, +1, s);
+            } else {
+                cudaEvent_t eb = next_event();
+                CK(cudaEventRecord(eb, s));
+                CK(cudaStreamWaitEvent(s2, eb, 0));
+                verfft_batch(v, +1, s2);
+                cudaEvent_t ev = next_event();
+                CK(cudaEventRecord(ev, s2));
+                done[set] = ev;
+            }
+            for (int q = 0; q < cnt; ++q) fs[i0 + q]->space = MLEGS_PFP;
+        }
+        if (all) return;
         cudaEvent_t ej = next_event();
         CK(cudaEventRecord(ej, s2));
         CK(cudaStreamWaitEvent(s, ej, 0));
@@ -569,14 +613,33 @@ struct mlegs_ctx {
     }
 
     // PROJECT's five fold products of PFF inputs (mod_legops.f90:2497-2535) on
-    // the bulk-copy pipeline: PSI = -(i m) EO(V, RUR) - OE(D, RUP),
-    // CHI = (i k) OE(D, RUR) + m k EO(V, RUP) - EO(T, UZ).
+    // the bulk-copy pipeline: CHI = (i k) OE(D, RUR) + m k EO(V, RUP) - EO(T, UZ),
+    // PSI = -(i m) EO(V, RUR) - OE(D, RUP); with bn, the RTRAN(-1) of bn into bn_out
+    // in the same launch.
     void project_bulk(const double2* rur, const double2* rup, const double2* uz, double2* psi_, double2* chi_,
-                      cudaStream_t st) {
-        const double* wc[5] = {fc_V, fc_D, fc_D, fc_V, fc_T};
-        const double2* x[5] = {rur, rup, rur, rup, uz};
-        const int md[5] = {0, 1, 1, 0, 0}, sc[5] = {2, 1, 3, 4, 1};
-        k_fold_bulk(g, wc, x, md, sc, 5, 2, psi_, chi_, d.NRCHOPDIM, 0, 0, st);
+                      cudaStream_t st, const double2* bn = nullptr, double2* bn_out = nullptr) {
+        const FoldSeg seg[6] = {{fc_D, rur, 1, 3}, {fc_V, rup, 0, 4}, {fc_T, uz, 0, 1},
+                                {fc_V, rur, 0, 2}, {fc_D, rup, 1, 1}, {fc_pf, bn, 0, 0}};
+        const int first[4] = {0, 3, 5, 6};
+        double2* const outs[3] = {chi_, psi_, bn_out};
+        k_fold_bulk(g, seg, first, bn ? 3 : 2, outs, d.NRCHOPDIM, 0, 0, st);
+    }
+    // PROJECT(NR, NP, NZ, PSI, W, 0.0) and BN = TOFF(BN) (pad 0) of PFP results of
+    // the theta stage, whose PFF images go to pff[0..3]; PSI, W, BNout in FFF.
+    void project_toff(Field* NR, Field* NP, Field* NZ, Field* BN, double2* const* pff, Field* PSI, Field* W,
+                      Field* BNout) {
+        VerBatch v{};
+        v.n = 4;
+        Field* const f[4] = {NR, NP, NZ, BN};
+        for (int q = 0; q < 4; ++q) {
+            v.src[q] = f[q]->data;
+            v.dst[q] = pff[q];
+        }
+        verfft_batch(v, -1, s);
+        launch_vel2pln(g, pff[1], PSI->ln, 1, 0.0, v2p_pff, s, W->ln, BNout->ln);
+        project_bulk(pff[0], pff[1], pff[2], PSI->data, W->data, s, pff[3], BNout->data);
+        k_farfield_fix(g, PSI->data, d.NRCHOP, s);
+        PSI->space = W->space = BNout->space = MLEGS_FFF;
     }
     // PROJECT(RUR, RUP, UZ, PSI, CHI) with PSI%LN by reference (ln_mode 2) for
     // FFF inputs whose LN terms are zero: one composite FFF -> FFF product per m

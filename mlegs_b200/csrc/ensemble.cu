@@ -204,12 +204,16 @@ void phase0(mlegs_ensemble& E, EnsInst& I) {
 void phase1(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
     const DevGrid& g = c->g;
+    VerBatch v{};
+    v.n = 10;
     for (int q = 0; q < 10; ++q) {
-        if (!k_verfft4(g, c->fft, I.T[q]->data, I.f[q]->data, +1, c->s)) k_verfft_b(g, c->fft, I.T[q]->data, I.f[q]->data, c->s);
-        c->ln_zero(I.f[q]);
+        v.src[q] = I.T[q]->data;
+        v.dst[q] = I.f[q]->data;
+        v.zln[q] = I.f[q]->ln;
         I.f[q]->space = MLEGS_PFP;
-        c->rel(I.T[q]);
     }
+    c->verfft_batch(v, +1, c->s);
+    for (Field* x : I.T) c->rel(x);
     I.NR = c->tmp();
     I.NP = c->tmp();
     I.NZ = c->tmp();

@@ -103,7 +103,13 @@ __global__ void __launch_bounds__(128) rtran_b2p_kernel(DevGrid g, const double*
 
 void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
     if (b2p_bulk_supported(g)) {
-        k_rtran_b2p_bulk(g, a, b, ln, pad, s);
+        B2PBatch f{};
+        f.n = 1;
+        f.in[0] = a;
+        f.out[0] = b;
+        f.ln[0] = ln;
+        f.pad[0] = pad;
+        k_rtran_b2p_bulk(g, f, s);
         return;
     }
     if (dmma_supported(g)) {
@@ -114,6 +120,14 @@ void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* l
     dim3 grid((ncol + TN - 1) / TN, (g.NRH + TM - 1) / TM, g.NTCHOPDIM);
     rtran_b2p_kernel<<<grid, 128, 0, s>>>(g, (const double*)a, (double*)b, ln, pad);
     count_launch();
+}
+
+void k_rtran_b2p_batch(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
+    if (b2p_bulk_supported(g)) {
+        k_rtran_b2p_bulk(g, f, s);
+        return;
+    }
+    for (int q = 0; q < f.n; ++q) k_rtran_b2p(g, f.in[q], f.out[q], f.ln[q], f.pad[q], s);
 }
 
 namespace {

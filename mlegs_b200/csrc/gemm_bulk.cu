@@ -5,7 +5,9 @@
 // m and parity p of n,
 //     C_p(i, c) = sum_t PF(i, 2t+p) A(2t+p, c),  B(i) = C_0 + C_1,
 //     B(NR-1-i) = C_0 - C_1,  plus the (m, k) = (0, 0) log term.
-// One CTA computes a 32-column tile of one m for all NRH output rows:
+// One launch runs up to ten fields (each with its own chop): a single small
+// field fills a fraction of the chip and costs a launch of its own.  One CTA
+// computes a 32-column tile of one m of one field for all NRH output rows:
 //   warps 0..3   consumers: m8n8k4 FP64 MMAs over their MTW m-tiles x four
 //                n-tiles, both parities' accumulators in registers;
 //   warp 4       producer: per 16-row K chunk, one 1-D bulk copy
@@ -116,16 +118,15 @@ __device__ __forceinline__ void chunk_mma(double (&acc)[MTW][4][2], const double
 // Per-stage work description the producer hands to the consumers with the
 // stage's data (written before the stage's arrive, read after its wait).
 struct StageInfo {
-    int tile;    // tile index (m * ntx + column tile), -1: no more work
+    int tile;    // tile index ((m * fields + field) * ntx + column tile), -1: no more work
     int p;       // parity of the K rows
     int kvalid;  // valid K rows in this chunk (0: a tile without K rows)
     int last;    // 1: the tile's last chunk (the consumers write the tile out)
 };
 
 template <int MTW, int NST>
-__global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_kernel(DevGrid g, const double* __restrict__ A,
-                                                                               double* __restrict__ out,
-                                                                               const double* ln, int pad) {
+__global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
+    b2p_bulk_kernel(DevGrid g, const __grid_constant__ B2PBatch fb_) {
     constexpr int SA = BNW * MTW * 8 + (((BNW * MTW) & 1) ? 0 : 8);  // PF row stride, = 8 mod 16
     constexpr int STG = BK * SA + BK * BSB;                          // doubles per stage
     extern __shared__ __align__(128) double smd[];
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
     __shared__ int abort_f;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ncol = 2 * g.NXCHOPDIM;
-    const int ntx = (ncol + BCT - 1) / BCT, ntiles = ntx * g.NTCHOPDIM;
+    const int ntx = (ncol + BCT - 1) / BCT, ntf = ntx * fb_.n, ntiles = ntf * g.NTCHOPDIM;
     // zeroed ring (rows that are never copied stay finite), barriers
     for (int e = tid; e < NST * STG; e += blockDim.x) smd[e] = 0.0;
     if (tid == 0) {
@@ -151,9 +152,9 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
 
     if (warp == BNW) {
         // ---------------------------------------------------------------- producer
-        // The CTA's tiles are blockIdx.x, + gridDim.x, ... (m ascending: the
-        // largest K first); their chunks form one stream through the ring, so
-        // the next tile's rows arrive while the current one is finishing.
+        // The CTA's tiles are blockIdx.x, + gridDim.x, ... (m ascending over all
+        // fields: the largest K first); their chunks form one stream through the
+        // ring, so the next tile's rows arrive while the current one is finishing.
         const int ne = g.NRCHOPDIM + 1;
         const uint32_t abytes = (uint32_t)g.NRH * 8u;
         int seq = 0;  // chunks handed over so far
@@ -166,14 +167,14 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
             return w && !*(volatile int*)&abort_f;
         };
         for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-            const int m = tile / ntx, c0 = (tile - m * ntx) * BCT;
-            int nn = g.NRCHOP + pad - m;
+            const int m = tile / ntf, fi = (tile - m * ntf) / ntx, c0 = (tile - m * ntf - fi * ntx) * BCT;
+            int nn = g.NRCHOP + fb_.pad[fi] - m;
             if (nn < 0) nn = 0;
             const int kp0 = (nn + 1) / 2, kp1 = nn / 2;
             const int nc0 = (kp0 + BK - 1) / BK, nc1 = (kp1 + BK - 1) / BK;
             const int total = max(1, nc0 + nc1);  // a tile without K rows still hands over one empty chunk
             const double* pf = g.pf + (size_t)m * ne * g.NRH;
-            const double* a = A + (size_t)m * g.NRCHOPDIM * ncol;
+            const double* a = (const double*)fb_.in[fi] + (size_t)m * g.NRCHOPDIM * ncol;
             const uint32_t bbytes = (uint32_t)min(BCT, ncol - c0) * 8u;
             for (int c = 0; c < total; ++c) {
                 const int st = seq % NST;
@@ -258,9 +259,9 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
         if (lane == 0) bar_arrive(empty + st);
         if (!inf.last) continue;
         // the tile's butterfly + log term, then fresh accumulators
-        const int m = inf.tile / ntx, c0 = (inf.tile - m * ntx) * BCT;
-        const double lnv = (m == 0 && ln) ? *ln : 0.0;
-        double* o = out + (size_t)m * g.NR * ncol;
+        const int m = inf.tile / ntf, fi = (inf.tile - m * ntf) / ntx, c0 = (inf.tile - m * ntf - fi * ntx) * BCT;
+        const double lnv = (m == 0 && fb_.ln[fi]) ? *fb_.ln[fi] : 0.0;
+        double* o = (double*)fb_.out[fi] + (size_t)m * g.NR * ncol;
 #pragma unroll
         for (int i = 0; i < MTW; ++i) {
             const int row = (warp + BNW * i) * 8 + gq;
@@ -288,7 +289,9 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
 // products, mod_legops.f90:2497-2535, 2548-2648) with the same pipeline:
 //   out(n, c) (+)= sum_seg sum_{i < NRH} W_seg(n, i) s_seg(c) F_seg(i, c),
 //   F = x(i) +/- x(NR-1-i), the sign by output-row parity xor the segment's mode.
-// One CTA tile = (m, output parity pr, 64 columns): each of four consumer
+// A launch has up to three outputs, each the sum of its own segments: PROJECT's
+// PSI and CHI and the RTRAN(-1) of a fourth field go together, as separate tiles.
+// One CTA tile = (m, output, output parity pr, 64 columns): each of four consumer
 // warps folds its own 16 columns once per chunk and multiplies them by every
 // valid output-row tile (8 rows) of the weights, so the fold work is not
 // repeated across warps.  A K chunk (16 rows i of one
@@ -304,31 +307,21 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2) b2p_bulk_ker
 // each B fragment as it is read: -1, m k and the fold sign are real factors,
 // -i m and i k read the partner column (re <-> im) with a per-lane sign.
 struct FoldBulkArgs {
-    const double* wc[5];  // chunked weight tables
-    int mode[5];          // 0: EO fold, 1: OE fold
-    int scale[5];         // 0 none, 1 -v, 2 -i m v, 3 i k v, 4 m k v
-    int nseg, split;      // segments [0, split) -> out0, [split, nseg) -> out1
-    double* out0;
-    double* out1;
-    int wt_rows, pad, accumulate, RB;  // RB: rows per (m, pr) block of the tables
+    const double* wc[FOLD_SEGS];    // chunked weight tables
+    int mode[FOLD_SEGS];            // 0: EO fold, 1: OE fold
+    int scale[FOLD_SEGS];           // 0 none, 1 -v, 2 -i m v, 3 i k v, 4 m k v
+    int first[FOLD_OUTS + 1];       // output o sums the segments [first[o], first[o + 1])
+    double* out[FOLD_OUTS];
+    int nout, wt_rows, pad, accumulate, RB;  // RB: rows per (m, pr) block of the tables
 };
 // The segments' input fields as 2-D tensor maps: columns (2 NXCHOPDIM) x rows (NTCHOPDIM NR).
 struct alignas(64) FoldMaps {
-    CUtensorMap x[5];
+    CUtensorMap x[FOLD_SEGS];
 };
 constexpr int WCS = 20;           // chunked weight row stride (doubles), = 4 mod 16
 constexpr int FNW = 4;            // consumer warps, 16 columns each
 constexpr int FCT = 16 * FNW;     // columns per tile
 constexpr int XW = FCT + 8;       // field box width (doubles), = 8 mod 16
-
-template <class T>
-__device__ __forceinline__ T sel5(const T (&a)[5], int i) {
-    T v = a[0];
-#pragma unroll
-    for (int j = 1; j < 5; ++j)
-        if (i == j) v = a[j];
-    return v;
-}
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -339,8 +332,8 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 }
 
 struct FoldInfo {
-    int tile;    // (m, pr, column tile) index, -1: no more work
-    int gc;      // chunk index within the tile (segment * nch + chunk)
+    int tile;    // (m, output, pr, column tile) index, -1: no more work
+    int gc;      // chunk index within the tile (the output's segment * nch + chunk)
     int kvalid;  // valid K rows in the chunk
     int last;    // 1: the tile's last chunk
 };
@@ -377,7 +370,8 @@ __device__ __forceinline__ void fold_chunk_mma(double (&acc)[MT][2][2], const do
 }
 
 template <int MT, int NST>
-__global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g, FoldBulkArgs fa,
+__global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
+                                                                      const __grid_constant__ FoldBulkArgs fa,
                                                                       const __grid_constant__ FoldMaps tm) {
     extern __shared__ __align__(128) double smd[];
     const int STG = fa.RB * WCS + 2 * BK * XW;  // doubles per stage (a multiple of 16)
@@ -387,8 +381,8 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
     __shared__ int abort_f;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ncol = 2 * g.NXCHOPDIM;
-    const int ntx = (ncol + FCT - 1) / FCT, ntiles = ntx * 2 * g.NTCHOPDIM;
-    const int nch = (g.NRH + BK - 1) / BK, nchunks = fa.nseg * nch;
+    const int ntx = (ncol + FCT - 1) / FCT, ntiles = ntx * 2 * fa.nout * g.NTCHOPDIM;
+    const int nch = (g.NRH + BK - 1) / BK;
     for (int e = tid; e < NST * STG; e += blockDim.x) smd[e] = 0.0;
     if (tid == 0) {
         abort_f = 0;
@@ -400,10 +394,12 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    // per tile: m, parity, first column, valid row tiles (rows n < min(NRCHOPS(m), wt_rows))
-    auto decode = [&](int tile, int& m, int& pr, int& c0, int& nn, int& RTv) {
-        m = tile / (2 * ntx);
-        const int rem = tile - m * 2 * ntx;
+    // per tile: m, output, parity, first column, valid row tiles (rows n < min(NRCHOPS(m), wt_rows))
+    auto decode = [&](int tile, int& m, int& ou, int& pr, int& c0, int& nn, int& RTv) {
+        m = tile / (2 * ntx * fa.nout);
+        int rem = tile - m * 2 * ntx * fa.nout;
+        ou = rem / (2 * ntx);
+        rem -= ou * 2 * ntx;
         pr = rem / ntx;
         c0 = (rem - pr * ntx) * FCT;
         nn = g.NRCHOP + fa.pad - m;
@@ -427,16 +423,17 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
         };
         constexpr uint32_t xbytes = (uint32_t)(BK * XW * 8);
         for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-            int m, pr, c0, nn, RTv;
-            decode(tile, m, pr, c0, nn, RTv);
+            int m, ou, pr, c0, nn, RTv;
+            decode(tile, m, ou, pr, c0, nn, RTv);
             const uint32_t abytes = (uint32_t)RTv * 8u * WCS * 8u;
+            const int s0 = fa.first[ou], nchunks = (fa.first[ou + 1] - s0) * nch;
             for (int gc = 0; gc < nchunks; ++gc) {
                 const int st = seq % NST;
                 if (!acquire(st)) {
                     ok = false;
                     break;
                 }
-                const int sg = gc / nch, ch = gc - sg * nch, i0 = ch * BK;
+                const int sl = gc / nch, sg = s0 + sl, ch = gc - sl * nch, i0 = ch * BK;
                 const int kv = min(BK, g.NRH - i0);
                 double* As = smd + (size_t)st * STG;
                 double* Xs = As + fa.RB * WCS;
@@ -444,12 +441,10 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
                     info[st] = FoldInfo{tile, gc, kv, gc == nchunks - 1 ? 1 : 0};
                     bar_expect_tx(full + st, abytes + 2u * xbytes);
                     if (abytes) {
-                        const double* wc = sel5(fa.wc, sg) + (((size_t)m * 2 + pr) * nch + ch) * fa.RB * WCS;
+                        const double* wc = fa.wc[sg] + (((size_t)m * 2 + pr) * nch + ch) * fa.RB * WCS;
                         bulk_copy(As, wc, abytes, full + st);
                     }
-                    const CUtensorMap* map = &tm.x[0];
-                    for (int j = 1; j < 5; ++j)
-                        if (sg == j) map = &tm.x[j];
+                    const CUtensorMap* map = &tm.x[sg];
                     tma_load_2d(Xs, map, c0, m * g.NR + i0, full + st);
                     tma_load_2d(Xs + BK * XW, map, c0, m * g.NR + g.NR - BK - i0, full + st);
                 }
@@ -485,7 +480,7 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
     double fac[2] = {1.0, 1.0}, fsg[2] = {1.0, 1.0};
     int gsel = gq;
     int cur_tile = -2, cur_sg = -1;
-    int m = 0, pr = 0, c0 = 0, nn = 0, RTv = 0;
+    int m = 0, ou = 0, pr = 0, c0 = 0, nn = 0, RTv = 0;
     auto epilogue = [&](double* out) {
         double* o = out + (size_t)m * g.NRCHOPDIM * ncol;
 #pragma unroll
@@ -524,13 +519,13 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
         if (inf.tile != cur_tile) {
             cur_tile = inf.tile;
             cur_sg = -1;
-            decode(inf.tile, m, pr, c0, nn, RTv);
+            decode(inf.tile, m, ou, pr, c0, nn, RTv);
         }
-        const int sg = inf.gc / nch;
+        const int sg = fa.first[ou] + inf.gc / nch;
         if (sg != cur_sg) {  // the segment's fold sign, column factors and column selection
             cur_sg = sg;
-            const int sc = sel5(fa.scale, sg);
-            const double sgn = (pr ^ sel5(fa.mode, sg)) ? -1.0 : 1.0;
+            const int sc = fa.scale[sg];
+            const double sgn = (pr ^ fa.mode[sg]) ? -1.0 : 1.0;
             const bool rot = sc == 2 || sc == 3;
             const double odd = (gq & 1) ? 1.0 : -1.0;  // lanes on imaginary columns
 #pragma unroll
@@ -558,15 +553,13 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
         else fold_chunk_mma<MT, true>(acc, As + fa_ofs, Xt, Xb, fac, fsg, inf.kvalid, q, RTv);
         __syncwarp();
         if (lane == 0) bar_arrive(empty + st);
-        const int ch_last = (inf.gc % nch) == nch - 1;
-        if (ch_last && sg == fa.split - 1) epilogue(fa.out0);
-        else if (inf.last) epilogue(fa.out1);
+        if (inf.last) epilogue(fa.out[ou]);
     }
 }
 
 // Chunked weight table of a fold GEMM: Wc[m][pr][chunk][r][WCS] = W(n = 2r + pr,
 // i = 16 chunk + kk) (times w_i when use_w), zero past NRH, wt_rows and kk >= 16.
-__global__ void fold_table_kernel(DevGrid g, const double* __restrict__ W, int wt_rows, int use_w, int RB,
+__global__ void fold_table_kernel(DevGrid g, const double* __restrict__ W, int src_rows, int wt_rows, int use_w, int RB,
                                   double* __restrict__ Wc) {
     const int nch = (g.NRH + BK - 1) / BK;
     const size_t total = (size_t)g.NTCHOPDIM * 2 * nch * RB * WCS;
@@ -580,7 +573,7 @@ __global__ void fold_table_kernel(DevGrid g, const double* __restrict__ W, int w
     const int n = 2 * r + pr, i = ch * BK + kk;
     double v = 0.0;
     if (kk < BK && n < wt_rows && i < g.NRH) {
-        v = W[((size_t)m * wt_rows + n) * g.NRH + i];
+        v = W[((size_t)m * src_rows + n) * g.NRH + i];
         if (use_w) v *= g.w[i];
     }
     Wc[t] = v;
@@ -598,8 +591,7 @@ int bulk_sm_count() {
 }
 
 template <int MTW, int NST>
-void launch_b2p_bulk_n(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, int per_sm,
-                       cudaStream_t s) {
+void launch_b2p_bulk_n(const DevGrid& g, const B2PBatch& f, int per_sm, cudaStream_t s) {
     constexpr int SA = BNW * MTW * 8 + (((BNW * MTW) & 1) ? 0 : 8);
     constexpr size_t smem = (size_t)NST * (BK * SA + BK * BSB) * sizeof(double) + 2 * NST * sizeof(uint64_t);
     static bool attr = false;
@@ -608,9 +600,9 @@ void launch_b2p_bulk_n(const DevGrid& g, const double2* a, double2* b, const dou
         attr = true;
     }
     const int ncol = 2 * g.NXCHOPDIM;
-    const int ntiles = ((ncol + BCT - 1) / BCT) * g.NTCHOPDIM;
+    const int ntiles = ((ncol + BCT - 1) / BCT) * g.NTCHOPDIM * f.n;
     const int grid = std::min(ntiles, bulk_sm_count() * per_sm);
-    b2p_bulk_kernel<MTW, NST><<<grid, (BNW + 1) * 32, smem, s>>>(g, (const double*)a, (double*)b, ln, pad);
+    b2p_bulk_kernel<MTW, NST><<<grid, (BNW + 1) * 32, smem, s>>>(g, f);
     count_launch();
 }
 
@@ -618,8 +610,8 @@ void launch_b2p_bulk_n(const DevGrid& g, const double2* a, double2* b, const dou
 // SM for a VERFFT(+1) CTA, which runs beside the GEMM on the other stream in
 // TOFP; four stages filled the SM (545 vs 541 steps/s at 192x128x256).
 template <int MTW>
-void launch_b2p_bulk(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
-    launch_b2p_bulk_n<MTW, 3>(g, a, b, ln, pad, MTW <= 3 ? 3 : 2, s);
+void launch_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
+    launch_b2p_bulk_n<MTW, 3>(g, f, MTW <= 3 ? 3 : 2, s);
 }
 
 template <int MT>
@@ -633,7 +625,7 @@ void launch_fold_bulk(const DevGrid& g, const FoldBulkArgs& fa, const FoldMaps& 
             attr = smem;
     }
     const int ncol = 2 * g.NXCHOPDIM;
-    const int ntiles = ((ncol + FCT - 1) / FCT) * 2 * g.NTCHOPDIM;
+    const int ntiles = ((ncol + FCT - 1) / FCT) * 2 * fa.nout * g.NTCHOPDIM;
     const int grid = std::min(ntiles, bulk_sm_count() * 3);
     fold_bulk_kernel<MT, NST><<<grid, (FNW + 1) * 32, smem, s>>>(g, fa, tm);
     count_launch();
@@ -702,13 +694,13 @@ bool b2p_bulk_supported(const DevGrid& g) {
     return (g.NRH % 2) == 0 && RT <= 4 * BNW;
 }
 
-void k_rtran_b2p_bulk(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
+void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
     const int RT = (g.NRH + 7) / 8;
     switch ((RT + BNW - 1) / BNW) {
-        case 1: launch_b2p_bulk<1>(g, a, b, ln, pad, s); break;
-        case 2: launch_b2p_bulk<2>(g, a, b, ln, pad, s); break;
-        case 3: launch_b2p_bulk<3>(g, a, b, ln, pad, s); break;
-        default: launch_b2p_bulk<4>(g, a, b, ln, pad, s); break;
+        case 1: launch_b2p_bulk<1>(g, f, s); break;
+        case 2: launch_b2p_bulk<2>(g, f, s); break;
+        case 3: launch_b2p_bulk<3>(g, f, s); break;
+        default: launch_b2p_bulk<4>(g, f, s); break;
     }
 }
 
@@ -730,10 +722,11 @@ size_t fold_table_doubles(const DevGrid& g, int wt_rows) {
     return (size_t)g.NTCHOPDIM * 2 * nch * fold_table_rows(g, wt_rows) * WCS;
 }
 
-void k_fold_table(const DevGrid& g, const double* W, int wt_rows, int use_w, double* Wc, cudaStream_t s) {
+void k_fold_table(const DevGrid& g, const double* W, int src_rows, int wt_rows, int use_w, double* Wc,
+                  cudaStream_t s) {
     const size_t n = fold_table_doubles(g, wt_rows);
-    fold_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, W, wt_rows, use_w, fold_table_rows(g, wt_rows),
-                                                                   Wc);
+    fold_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, W, src_rows, wt_rows, use_w,
+                                                                   fold_table_rows(g, wt_rows), Wc);
     count_launch();
 }
 
@@ -745,26 +738,25 @@ bool fold_bulk_supported(const DevGrid& g, int wt_rows) {
     return RB <= 12 * 8 && smem <= 227 * 1024 / 2 - 1024 && g.NRH >= BK && tmap_encoder() != nullptr;
 }
 
-// out (+)= sum over segments; wc: chunked tables of k_fold_table (wt_rows rows).
-void k_fold_bulk(const DevGrid& g, const double* const* wc, const double2* const* x, const int* mode,
-                 const int* scale, int nseg, int split, double2* out0, double2* out1, int wt_rows, int pad,
-                 int accumulate, cudaStream_t s) {
+// outs[o] (+)= sum over the segments [first[o], first[o + 1]); the segments' tables
+// come from k_fold_table with the same wt_rows.
+void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nout, double2* const* outs, int wt_rows,
+                 int pad, int accumulate, cudaStream_t s) {
     FoldBulkArgs fa{};
     FoldMaps tm;
     memset(&tm, 0, sizeof(tm));
-    for (int q = 0; q < 5; ++q) {
-        const int src = q < nseg ? q : 0;
-        fa.wc[q] = wc[src];
-        fa.mode[q] = q < nseg ? mode[q] : 0;
-        fa.scale[q] = q < nseg ? scale[q] : 0;
-        if (q < nseg && !field_map(g, (const double*)x[q], &tm.x[q]))
+    const int nseg = first[nout];
+    for (int q = 0; q < nseg; ++q) {
+        fa.wc[q] = seg[q].wc;
+        fa.mode[q] = seg[q].mode;
+        fa.scale[q] = seg[q].scale;
+        if (!field_map(g, (const double*)seg[q].x, &tm.x[q]))
             throw std::runtime_error("fold GEMM: cuTensorMapEncodeTiled failed");
     }
-    for (int q = nseg; q < 5; ++q) tm.x[q] = tm.x[0];
-    fa.nseg = nseg;
-    fa.split = split;
-    fa.out0 = (double*)out0;
-    fa.out1 = (double*)(out1 ? out1 : out0);
+    for (int q = nseg; q < FOLD_SEGS; ++q) tm.x[q] = tm.x[0];
+    for (int o = 0; o <= FOLD_OUTS; ++o) fa.first[o] = first[std::min(o, nout)];
+    for (int o = 0; o < nout; ++o) fa.out[o] = (double*)outs[o];
+    fa.nout = nout;
     fa.wt_rows = wt_rows;
     fa.pad = pad;
     fa.accumulate = accumulate;

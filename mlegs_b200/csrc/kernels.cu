@@ -345,7 +345,7 @@ __device__ double vel2pln_dot(const double* L, const double2* line, size_t st, i
 }
 
 __global__ void vel2pln_kernel(DevGrid g, double2* rup, double* psi_ln, int mode, double ln_in, const double* Lpff,
-                               double* zero_ln) {
+                               double* zero_ln, double* zero_ln2) {
     __shared__ double part[8];
     const size_t st = g.NXCHOPDIM;  // PFF row stride for m = 0 ([0][r][k])
     const double pln = vel2pln_dot(Lpff, rup, st, g.NR, part);
@@ -359,11 +359,12 @@ __global__ void vel2pln_kernel(DevGrid g, double2* rup, double* psi_ln, int mode
     if (threadIdx.x == 0) {
         *psi_ln = (mode == 1) ? ln_in : pln;
         if (zero_ln) *zero_ln = 0.0;
+        if (zero_ln2) *zero_ln2 = 0.0;
     }
 }
 void launch_vel2pln(const DevGrid& g, double2* rup_pff, double* psi_ln, int mode, double ln, const double* Lpff,
-                    cudaStream_t s, double* zero_ln) {
-    vel2pln_kernel<<<1, 256, 0, s>>>(g, rup_pff, psi_ln, mode, ln, Lpff, zero_ln);
+                    cudaStream_t s, double* zero_ln, double* zero_ln2) {
+    vel2pln_kernel<<<1, 256, 0, s>>>(g, rup_pff, psi_ln, mode, ln, Lpff, zero_ln, zero_ln2);
     count_launch();
 }
 

@@ -106,6 +106,18 @@ void k_split_fold(const DevGrid& g, int S, const uint8_t* img, const int* eA, in
                   double2* out, int mode, int scale, int accumulate, int pad, int use_w, int* err,
                   uint64_t wait_cycles, cudaStream_t s);
 void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
+// RTRAN(+1) of up to ten fields, each at its own CHOPSET(pad), in one launch when
+// the bulk-copy form runs (one launch per field otherwise).  ln: the fields' LN
+// slots (null: no log term).
+constexpr int BATCH = 10;
+struct B2PBatch {
+    const double2* in[BATCH];
+    double2* out[BATCH];
+    const double* ln[BATCH];
+    int pad[BATCH];
+    int n;
+};
+void k_rtran_b2p_batch(const DevGrid& g, const B2PBatch& f, cudaStream_t s);
 // Fold GEMM arguments (gemm_dmma.cu): RTRAN(-1) and PROJECT's five EOMUL/OEMUL
 // products as K-concatenated segments.
 struct FoldArgs {
@@ -166,19 +178,25 @@ bool b2p_bulk_supported(const DevGrid& g);
 // FP64 tensor-path ceiling microbenchmark (register-only MMAs); FLOPs per launch
 double k_dmma_peak(double* out, cudaStream_t s);
 double dmma_peak_flops();
-void k_rtran_b2p_bulk(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
+void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s);
 int bulk_gemm_error(bool reset);
 // Fold GEMMs (RTRAN(-1), PROJECT's products) on the same pipeline: weight
-// tables re-laid per (m, parity, 16-row chunk) by k_fold_table (times w_i when
-// use_w), then k_fold_bulk over nseg segments (mode / scale as in FoldArgs;
-// segments [0, split) -> out0, the rest -> out1).
+// tables re-laid per (m, parity, 16-row chunk) by k_fold_table (rows n < wt_rows of
+// W[m][src_rows][NRH], times w_i when use_w), then k_fold_bulk: output o sums the
+// segments [first[o], first[o + 1]) (mode / scale as in FoldArgs).
+constexpr int FOLD_SEGS = 6, FOLD_OUTS = 3;
+struct FoldSeg {
+    const double* wc;
+    const double2* x;
+    int mode, scale;
+};
 int fold_table_rows(const DevGrid& g, int wt_rows);
 size_t fold_table_doubles(const DevGrid& g, int wt_rows);
-void k_fold_table(const DevGrid& g, const double* W, int wt_rows, int use_w, double* Wc, cudaStream_t s);
+void k_fold_table(const DevGrid& g, const double* W, int src_rows, int wt_rows, int use_w, double* Wc,
+                  cudaStream_t s);
 bool fold_bulk_supported(const DevGrid& g, int wt_rows);
-void k_fold_bulk(const DevGrid& g, const double* const* wc, const double2* const* x, const int* mode,
-                 const int* scale, int nseg, int split, double2* out0, double2* out1, int wt_rows, int pad,
-                 int accumulate, cudaStream_t s);
+void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nout, double2* const* outs, int wt_rows,
+                 int pad, int accumulate, cudaStream_t s);
 // FP64 tensor-path (mma.sync m8n8k4.f64) forms used by k_rtran_b2p / k_fold_gemm when supported.
 bool dmma_supported(const DevGrid& g);
 void k_rtran_b2p_dmma(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
@@ -224,6 +242,14 @@ void k_theta_fused(const DevGrid& g, const FFTPlan& p, const double2* const in[1
 void k_horfft_warp(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s);
 // Four-step VERFFT (dir +1: PFF -> PFP, -1: PFP -> PFF); false if NX has no specialisation.
 bool k_verfft4(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s);
+// The same for up to ten fields in one launch; zln: LN slots set to 0 (null entries: none).
+struct VerBatch {
+    const double2* src[BATCH];
+    double2* dst[BATCH];
+    double* zln[BATCH];
+    int n;
+};
+bool k_verfft4_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s);
 
 // Spectral operators on FFF.
 void k_delsqh(const DevGrid& g, const double2* a, const double* ln_a, double2* b, int pad, cudaStream_t s);
@@ -250,9 +276,9 @@ void k_ihelmp(const DevGrid& g, int P, const double* dq, int rows, double2* a, c
 // on the PFF line of RUP (Lpff, NR entries), or on RUP's FFF (0, 0) column
 // (Lfff, NRCHOP entries; mode 0, applied to that column).
 void k_vel2pln_coef(const DevGrid& g, const double* explog0, int nn, double* Lpff, double* Lfff, cudaStream_t s);
-// zero_ln (optional): one more LN slot set to 0 by the same launch.
+// zero_ln, zero_ln2 (optional): further LN slots set to 0 by the same launch.
 void launch_vel2pln(const DevGrid& g, double2* rup_pff, double* psi_ln, int mode, double ln, const double* Lpff,
-                    cudaStream_t s, double* zero_ln = nullptr);
+                    cudaStream_t s, double* zero_ln = nullptr, double* zero_ln2 = nullptr);
 void launch_vel2pln_fff(const DevGrid& g, double2* rup_fff, double* psi_ln, const double* Lfff, cudaStream_t s,
                         double* zero_ln = nullptr);
 

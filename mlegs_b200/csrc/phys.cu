@@ -799,10 +799,13 @@ void phys_set_attributes() {
 // group (warp w, gid) owns line m0 + w*G + gid.  PFP rows [r][z][m0..m0+MB)
 // move through a shared tile T[z][mloc] so global accesses stay contiguous.
 template <int N1, int N2>
-__global__ void __launch_bounds__(256) verfft4_kernel(DevGrid g, const double2* src, double2* dst,
+__global__ void __launch_bounds__(256) verfft4_kernel(DevGrid g, const __grid_constant__ VerBatch f,
                                                       const double2* tw_g, int dir) {
     constexpr int N = N1 * N2, G = 32 / N2;
     extern __shared__ double2 sm[];
+    const double2* src = f.src[blockIdx.z];
+    double2* dst = f.dst[blockIdx.z];
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && f.zln[blockIdx.z]) *f.zln[blockIdx.z] = 0.0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int gid = lane / N2, t = lane % N2;
     const int MB = nw * G;
@@ -871,8 +874,7 @@ __global__ void __launch_bounds__(256) verfft4_kernel(DevGrid g, const double2* 
 }
 
 template <int N1, int N2>
-static void launch_verfft4(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir,
-                           cudaStream_t s) {
+static void launch_verfft4(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
     constexpr int N = N1 * N2, G = 32 / N2;
     // (+1): MB = 4 G lines per CTA, more and smaller CTAs per SM overlapping their
     // load, FFT and store phases; (-1): 8 warps, longer tile rows per cp.async pass
@@ -888,21 +890,29 @@ static void launch_verfft4(const DevGrid& g, const FFTPlan& p, const double2* sr
         attr = true;
     }
     const int MB = warps * G;
-    dim3 grid((g.NTCHOPDIM + MB - 1) / MB, g.NR);
-    verfft4_kernel<N1, N2><<<grid, warps * 32, need(warps), s>>>(g, src, dst, p.tw_x, dir);
+    dim3 grid((g.NTCHOPDIM + MB - 1) / MB, g.NR, f.n);
+    verfft4_kernel<N1, N2><<<grid, warps * 32, need(warps), s>>>(g, f, p.tw_x, dir);
     count_launch();
 }
 
-bool k_verfft4(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s) {
+bool k_verfft4_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
     switch (g.NX) {
-        case 16: launch_verfft4<4, 4>(g, p, src, dst, dir, s); return true;
-        case 32: launch_verfft4<8, 4>(g, p, src, dst, dir, s); return true;
-        case 64: launch_verfft4<8, 8>(g, p, src, dst, dir, s); return true;
-        case 128: launch_verfft4<16, 8>(g, p, src, dst, dir, s); return true;
-        case 256: launch_verfft4<16, 16>(g, p, src, dst, dir, s); return true;
-        case 512: launch_verfft4<32, 16>(g, p, src, dst, dir, s); return true;
+        case 16: launch_verfft4<4, 4>(g, p, f, dir, s); return true;
+        case 32: launch_verfft4<8, 4>(g, p, f, dir, s); return true;
+        case 64: launch_verfft4<8, 8>(g, p, f, dir, s); return true;
+        case 128: launch_verfft4<16, 8>(g, p, f, dir, s); return true;
+        case 256: launch_verfft4<16, 16>(g, p, f, dir, s); return true;
+        case 512: launch_verfft4<32, 16>(g, p, f, dir, s); return true;
         default: return false;
     }
+}
+
+bool k_verfft4(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s) {
+    VerBatch f{};
+    f.n = 1;
+    f.src[0] = src;
+    f.dst[0] = dst;
+    return k_verfft4_batch(g, p, f, dir, s);
 }
 
 template <int N1, int N2>
