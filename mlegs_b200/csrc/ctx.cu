@@ -1111,6 +1111,51 @@ void mlegs_ctx::rich_fe_be() {
     rel(B2);
 }
 
+// The AB2 update, the history and CALC_BOUSSI_VISC_CN (mod_march.f90:636-654) of
+// the fields that have viscosity, as one pass (k_ab2_visc_rhs) and one launch of
+// their IHELM solves.  False, and nothing done, unless VISC%SW = 1 with every
+// coefficient non-zero and the factors at hand.
+bool mlegs_ctx::ab2_visc_fused(Field* PN, Field* CN, Field* BN) {
+    if (p.visc_sw != 1 || p.nu == 0.0 || p.kappa == 0.0) return false;
+    Field* const A[3] = {psi, chi, b};
+    Field* const N1[3] = {PN, CN, BN};
+    const double nu[3] = {p.nu, p.nu, p.kappa};
+    Ab2Args a{};
+    SolveBatch sb{};
+    a.n = sb.n = 3;
+    a.c1 = 1.5 * p.dt;
+    a.c0 = -0.5 * p.dt;
+    for (int q = 0; q < 3; ++q) {
+        a.alp[q] = 2 / nu[q] / p.dt;
+        const SolveFactors* f = factors(2, 0, a.alp[q]);
+        if (!f) return false;
+        sb.p[q].F5 = f->F5;
+        sb.p[q].F7 = f->F7;
+    }
+    Field* WK[3] = {tmp(), tmp(), tmp()};
+    for (int q = 0; q < 3; ++q) {
+        a.a[q] = A[q]->data;
+        a.n1[q] = N1[q]->data;
+        a.n0[q] = hist[q]->data;
+        a.rhs[q] = WK[q]->data;
+        a.a_ln[q] = A[q]->ln;
+        a.n1_ln[q] = q < 2 ? N1[q]->ln : nullptr;
+        a.n0_ln[q] = hist[q]->ln;
+        a.rhs_ln[q] = WK[q]->ln;
+        SolveItem& it = sb.p[q];
+        it.src = WK[q]->data;
+        it.dst = A[q]->data;
+        it.ln_src[0] = WK[q]->ln;
+        it.ln_dst[0] = A[q]->ln;
+        it.ln_src[1] = N1[q]->ln;
+        it.ln_dst[1] = hist[q]->ln;
+    }
+    k_ab2_visc_rhs(g, a, s);
+    k_solve_factored_batch(g, sb, 2, 0, 0.0, 0, 0, s);
+    for (Field* f : WK) rel(f);
+    return true;
+}
+
 // STEP_BOUSSI_AB_CN (mod_march.f90:609-661).
 void mlegs_ctx::step_ab_cn() {
     const double dt = p.dt;
@@ -1119,6 +1164,12 @@ void mlegs_ctx::step_ab_cn() {
     Field *NP = hist[0], *NC = hist[1], *NB = hist[2];
     Field *PN = tmp(), *CN = tmp(), *BN = tmp();
     force(psi, chi, b, PN, CN, BN);
+    if (ab2_visc_fused(PN, CN, BN)) {
+        rel(PN);
+        rel(CN);
+        rel(BN);
+        return;
+    }
     Field *P0 = tmp(), *C0 = tmp(), *B0 = tmp();
     copy0(P0, psi, 0);
     copy0(C0, chi, 0);

@@ -669,6 +669,7 @@ struct mlegs_ctx {
                 Field* BN, cudaEvent_t vor_ready = nullptr, Field* PSIN = nullptr, Field* CHIN = nullptr);
     void visc1(Field* A, double nu, double dt);
     void visc2(Field* A, const Field* AO, double nu, double dt);
+    bool ab2_visc_fused(Field* PN, Field* CN, Field* BN);
     void visc_be(Field* P, Field* C, Field* B, double dt);
     void visc_cn(Field* P, Field* C, Field* B, const Field* PO, const Field* CO, const Field* BO);
     void hyperv3(Field* P, Field* C, Field* B, double tf);

@@ -1223,6 +1223,68 @@ void k_mulr(const DevGrid& g, const double2* src, double2* dst, int mode, cudaSt
     count_launch();
 }
 
+// STEP_BOUSSI_AB_CN from its nonlinear terms to IHELM's right-hand sides
+// (mod_march.f90:636-647, VISC2 1579-1636, IHELM's log rows mod_legops.f90:
+// 1244-1255) in one pass per field:
+//   A1 = A + c1 N1 + c0 N0,  rhs = -DEL2(A chopped at pad 0) - alp A1 (chopped),
+//   rhs -= the DEL2 image of A1's log term at (m, k) = (0, 0),  N0 <- N1 chopped.
+// As copies, AXPBYs, DEL2 and chops this was thirteen launches a field, each a few
+// us on the small grids and a full pass over memory on the large ones; here each
+// element is read once (DEL2's row neighbours from L1: a block is 32 k by 8 rows).
+// The new LN goes to rhs_ln: the slots a_ln, n1_ln, n0_ln are read by several
+// blocks, so the solve that follows moves it to the state.
+__global__ void __launch_bounds__(256) ab2_visc_rhs_kernel(DevGrid g, const __grid_constant__ Ab2Args A) {
+    const int nkb = (g.NXCHOPDIM + 31) / 32;
+    const int f = blockIdx.x / nkb, k = (blockIdx.x - f * nkb) * 32 + threadIdx.x;
+    const int n = blockIdx.y * 8 + threadIdx.y, m = blockIdx.z;
+    if (k >= g.NXCHOPDIM || n >= g.NRCHOPDIM) return;
+    const size_t st = g.NXCHOPDIM;
+    const size_t t = ((size_t)m * g.NRCHOPDIM + n) * st + k;
+    const int nn = m < g.NTCHOP ? nrchops(g, m, 0) : 0;
+    const bool log = m == 0 && k == 0 && n < 3;
+    const double alp = A.alp[f];
+    double ln0 = 0.0, ln1 = 0.0;  // the state's LN before and after
+    if (log) {
+        ln0 = *A.a_ln[f];
+        double v = ln0;
+        if (A.n1_ln[f]) v = v + A.c1 * (*A.n1_ln[f]) + A.c0 * (*A.n0_ln[f]);
+        ln1 = (-alp * v) * (-1.0 / alp);
+        if (n == 0) *A.rhs_ln[f] = ln1;
+    }
+    if (n >= nn) {
+        A.rhs[f][t] = make_double2(0.0, 0.0);
+        A.n0[f][t] = make_double2(0.0, 0.0);
+        return;
+    }
+    const double2* a = A.a[f] + t;
+    const double2 a0 = *a, x1 = A.n1[f][t], x0 = A.n0[f][t];
+    A.n0[f][t] = x1;
+    const double* tb = g.del2h + ((size_t)m * g.NB + n) * 5;
+    double2 d = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        const int r = n + j - 2;
+        if (r < 0 || r >= nn) continue;
+        const double2 v = j == 2 ? a0 : a[((ptrdiff_t)j - 2) * (ptrdiff_t)st];
+        d.x += tb[j] * v.x;
+        d.y += tb[j] * v.y;
+    }
+    const double k2 = g.ak[k] * g.ak[k];
+    d.x -= k2 * a0.x;
+    d.y -= k2 * a0.y;
+    const double c[3] = {4.0 / 3, -2.0, 2.0 / 3};
+    if (log) d.x += c[n] * ln0 / g.ELL2 / g.norm0[n];
+    double2 v = make_double2(a0.x + A.c1 * x1.x + A.c0 * x0.x, a0.y + A.c1 * x1.y + A.c0 * x0.y);
+    v = make_double2(-d.x - alp * v.x, -d.y - alp * v.y);
+    if (log) v.x -= ln1 * (c[n] / g.ELL2) / g.norm0[n];
+    A.rhs[f][t] = v;
+}
+void k_ab2_visc_rhs(const DevGrid& g, const Ab2Args& a, cudaStream_t s) {
+    const dim3 grid(((g.NXCHOPDIM + 31) / 32) * a.n, (g.NRCHOPDIM + 7) / 8, g.NTCHOPDIM);
+    ab2_visc_rhs_kernel<<<grid, dim3(32, 8), 0, s>>>(g, a);
+    count_launch();
+}
+
 void k_etd_ab_fused(const DevGrid& g, const EtdAbArgs& a, cudaStream_t s) {
     const size_t n = g.NTCHOPDIM * (size_t)g.NRCHOPDIM * g.NXCHOPDIM;
     etd_ab_fused_kernel<<<nblk(n, 256), 256, 0, s>>>(g, a);

@@ -292,6 +292,38 @@ void solve_factor_sizes(const DevGrid& g, size_t* f5, size_t* f7);
 void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F5, double* F7, cudaStream_t s);
 void k_solve_factored(const DevGrid& g, const double* F5, const double* F7, const double2* src, double2* dst,
                       double* ln_out, int kind, int has_ln, double ln_in, int pad, int farfield, cudaStream_t s);
+// Several fields' solves of one kind and pad in one launch; ln_dst[j] <- ln_src[j]
+// (null: none) are LN copies the launch makes on the side.
+struct SolveItem {
+    const double* F5;
+    const double* F7;
+    const double2* src;
+    double2* dst;
+    double* ln_out;
+    const double* ln_src[2];
+    double* ln_dst[2];
+};
+struct SolveBatch {
+    SolveItem p[3];
+    int n;
+};
+void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
+                            int farfield, cudaStream_t s);
+// The AB2 update with VISC2's right-hand side for up to three fields (kernels.cu).
+struct Ab2Args {
+    const double2* a[3];     // state before the step
+    const double2* n1[3];    // nonlinear terms of this step
+    double2* n0[3];          // history: read, then set to n1 chopped
+    double2* rhs[3];         // IHELM's right-hand side
+    const double* a_ln[3];
+    const double* n1_ln[3];  // null: the state's LN is not updated by them
+    const double* n0_ln[3];
+    double* rhs_ln[3];       // the state's LN after the step
+    double alp[3];           // 2 / (NU DT)
+    double c1, c0;           // AB2 weights times DT
+    int n;
+};
+void k_ab2_visc_rhs(const DevGrid& g, const Ab2Args& a, cudaStream_t s);
 // Fixed __device__ solve scratch (solve_static.cu) for the allocation-free
 // IDEL2LN entry point: returns 0 and its address on `device` (the current
 // device), 1 if need_doubles exceeds kStaticSolveBytes, 2 on a CUDA error;

@@ -494,10 +494,19 @@ void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F5,
     count_launch();
 }
 
-__global__ void __launch_bounds__(128) solve_factored_kernel(DevGrid g, const double* __restrict__ F5,
-                                                             const double* __restrict__ F7, const double2* src,
-                                                             double2* dst, double* ln_out, int kind, int has_ln,
-                                                             double ln_in, int pad, int farfield, int wpad) {
+// LN slots a solve sets besides its own (thread 0 of the problem's first block).
+__device__ __forceinline__ void solve_ln_copies(const SolveItem& p) {
+    for (int j = 0; j < 2; ++j)
+        if (p.ln_dst[j]) *p.ln_dst[j] = *p.ln_src[j];
+}
+
+// blockIdx.y: the problem (fields with factors of one kind and pad: a step's
+// three viscous solves in one launch, each latency-bound alone).
+__global__ void __launch_bounds__(128) solve_factored_kernel(DevGrid g, const __grid_constant__ SolveBatch b, int kind,
+                                                             int has_ln, double ln_in, int pad, int farfield,
+                                                             int wpad) {
+    const SolveItem& p = b.p[blockIdx.y];
+    if (blockIdx.x == 0 && threadIdx.x == 0) solve_ln_copies(p);
     // kinds 1 and 2: the 7-band m = 0 systems (u < 2 NXCHOPDIM) take whole
     // warps, the 5-band ones start after wpad idle threads, so that no warp
     // runs both substitutions one after the other
@@ -507,7 +516,7 @@ __global__ void __launch_bounds__(128) solve_factored_kernel(DevGrid g, const do
         if (u >= nw && u < nw + wpad) return;
         if (u >= nw) u -= wpad;
     }
-    solve_factored_sys<16>(g, F5, F7, src, dst, ln_out, kind, has_ln, ln_in, pad, farfield, u);
+    solve_factored_sys<16>(g, p.F5, p.F7, p.src, p.dst, p.ln_out, kind, has_ln, ln_in, pad, farfield, u);
 }
 
 // Small systems (NRCHOP + pad <= SMALL_R rows): one warp takes 16 systems
@@ -529,11 +538,17 @@ __device__ __forceinline__ void cpa16(double2* d, const double2* src) {
                  : "memory");
 }
 
-__global__ void __launch_bounds__(32) solve_small_kernel(DevGrid g, const double* __restrict__ F5,
-                                                         const double* __restrict__ F7, const double2* src,
-                                                         double2* dst, double* ln_out, int kind, int has_ln,
-                                                         double ln_in, int pad, int farfield, int t_begin, int nb0) {
+__global__ void __launch_bounds__(32) solve_small_kernel(DevGrid g, const __grid_constant__ SolveBatch b, int kind,
+                                                         int has_ln, double ln_in, int pad, int farfield,
+                                                         int t_begin, int nb0) {
     extern __shared__ __align__(16) double sms[];
+    const SolveItem& p = b.p[blockIdx.y];
+    const double* __restrict__ F5 = p.F5;
+    const double* __restrict__ F7 = p.F7;
+    const double2* src = p.src;
+    double2* dst = p.dst;
+    double* ln_out = p.ln_out;
+    if (blockIdx.x == 0 && threadIdx.x == 0) solve_ln_copies(p);
     const int R = g.NRCHOP + pad;
     double* Fs = sms;                         // [R][7][16]
     double2* Xs = (double2*)(sms + R * 112);  // [R][16]
@@ -655,8 +670,8 @@ __global__ void __launch_bounds__(32) solve_small_kernel(DevGrid g, const double
 
 bool solve_small_ok(const DevGrid& g, int pad) { return g.NRCHOP + pad <= SMALL_R; }
 
-void k_solve_small(const DevGrid& g, const double* F5, const double* F7, const double2* src, double2* dst,
-                   double* ln_out, int kind, int has_ln, double ln_in, int pad, int farfield, cudaStream_t s) {
+void k_solve_small(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad, int farfield,
+                   cudaStream_t s) {
     const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
     const int t_begin = kind == 0 ? 0 : g.NXCHOPDIM;
     const int nb0 = (t_begin + 15) / 16, nb1 = (nsys - t_begin + 15) / 16;
@@ -667,22 +682,32 @@ void k_solve_small(const DevGrid& g, const double* F5, const double* F7, const d
         cudaFuncSetAttribute(solve_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = smem;
     }
-    solve_small_kernel<<<nb0 + nb1, 32, smem, s>>>(g, F5, F7, src, dst, ln_out, kind, has_ln, ln_in, pad, farfield,
-                                                   t_begin, nb0);
+    solve_small_kernel<<<dim3(nb0 + nb1, b.n), 32, smem, s>>>(g, b, kind, has_ln, ln_in, pad, farfield, t_begin, nb0);
+    count_launch();
+}
+
+void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
+                            int farfield, cudaStream_t s) {
+    if (solve_small_ok(g, pad)) {  // the whole system fits in shared memory
+        k_solve_small(g, b, kind, has_ln, ln_in, pad, farfield, s);
+        return;
+    }
+    const int wpad = kind == 0 ? 0 : (32 - (2 * g.NXCHOPDIM) % 32) % 32;
+    const int n = 2 * g.NTCHOPDIM * g.NXCHOPDIM + wpad;
+    solve_factored_kernel<<<dim3((n + 127) / 128, b.n), 128, 0, s>>>(g, b, kind, has_ln, ln_in, pad, farfield, wpad);
     count_launch();
 }
 
 void k_solve_factored(const DevGrid& g, const double* F5, const double* F7, const double2* src, double2* dst,
                       double* ln_out, int kind, int has_ln, double ln_in, int pad, int farfield, cudaStream_t s) {
-    if (solve_small_ok(g, pad)) {  // the whole system fits in shared memory
-        k_solve_small(g, F5, F7, src, dst, ln_out, kind, has_ln, ln_in, pad, farfield, s);
-        return;
-    }
-    const int wpad = kind == 0 ? 0 : (32 - (2 * g.NXCHOPDIM) % 32) % 32;
-    const int n = 2 * g.NTCHOPDIM * g.NXCHOPDIM + wpad;
-    solve_factored_kernel<<<(n + 127) / 128, 128, 0, s>>>(g, F5, F7, src, dst, ln_out, kind, has_ln, ln_in, pad,
-                                                          farfield, wpad);
-    count_launch();
+    SolveBatch b{};
+    b.n = 1;
+    b.p[0].F5 = F5;
+    b.p[0].F7 = F7;
+    b.p[0].src = src;
+    b.p[0].dst = dst;
+    b.p[0].ln_out = ln_out;
+    k_solve_factored_batch(g, b, kind, has_ln, ln_in, pad, farfield, s);
 }
 
 void k_solve_del2(const DevGrid& g, double2* a, double* ln_out, int kind, double alp, int has_ln, double ln_in,
