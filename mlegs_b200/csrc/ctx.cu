@@ -225,6 +225,11 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     tb_xxdx = up(h_xxdx);
     tb_xm = up(h_xm);
     tb_del2h = up(h_del2h);
+    {
+        std::vector<double> h(d.NTCHOPDIM + d.NRCHOPDIM + 2);
+        for (size_t N = 0; N < h.size(); ++N) h[N] = -(double)(N * (N + 1)) / d.ELL2;
+        lap = up(h);
+    }
 
     g.NR = d.NR;
     g.NRH = d.NRH;
@@ -250,6 +255,7 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     g.xm = tb_xm;
     g.del2h = tb_del2h;
     g.NB = NB;
+    g.lap = lap;
 
     // --- PROJECT weights (device, from PF)
     size_t vsz = (size_t)d.NTCHOPDIM * d.NRCHOPDIM * d.NRH;
@@ -495,9 +501,10 @@ void mlegs_ctx::force(const Field* PSI, const Field* CHI, const Field* B, Field*
     Field *RUR = tmp(), *RUP = tmp(), *UZ = tmp(), *ROR = tmp(), *ROP = tmp(), *OZ = tmp(), *RBR = tmp(),
           *RBP = tmp(), *BZ = tmp(), *W = tmp();
     const int P3 = 3;  // CHOPSET(3) ... CHOPSET(-3)
-    grad(B, RBR, RBP, BZ, P3);
-    pc2vel(PSI, CHI, RUR, RUP, UZ, P3);
-    pc2vor(PSI, CHI, ROR, ROP, OZ, P3);
+    {
+        Field* const fs[9] = {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ};
+        derivatives(PSI, CHI, B, fs, P3);
+    }
     // TOFP up to PFP; the HORFFT(+1) of each field happens inside the fused kernel.
     // W = B, TOFP(W) after CHOPSET(-3): the FP64 GEMM reads only the rows that COPY0
     // keeps, so it takes B itself; the derivative fields carry no log term.
@@ -1342,7 +1349,12 @@ void mlegs_ctx::step_etdab_cn() {
     rel(RURN);
     rel(RUPN);
     rel(UZN);
-    k_pc2vel_fused(g, psi->data, psi->ln, chi->data, chi->ln, hist[4]->data, hist[5]->data, hist[6]->data, 3, s, 1);
+    {
+        DerivArgs v = deriv_in(psi, chi, 3);
+        for (int q = 0; q < 3; ++q) v.out[q] = hist[4 + q]->data;
+        v.sub = 1;
+        k_deriv(g, v, 1, s);
+    }
     if (p.visc_sw == 1) {
         visc_cn(psi, chi, b, P0, C0, B0);
         rel(P0);

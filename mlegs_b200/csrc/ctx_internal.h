@@ -83,7 +83,7 @@ struct mlegs_ctx {
     // device tables
     double *x = nullptr, *w = nullptr, *r = nullptr, *lnx = nullptr, *pf = nullptr, *ak = nullptr;
     double *norm0 = nullptr, *explog0 = nullptr, *at1 = nullptr, *tb_xxdx = nullptr, *tb_xm = nullptr,
-           *tb_del2h = nullptr;
+           *tb_del2h = nullptr, *lap = nullptr;
     double *V = nullptr, *D = nullptr, *T = nullptr;
     double *hv[3] = {nullptr, nullptr, nullptr}, *hd[3] = {nullptr, nullptr, nullptr};
     // HYP3SET masks (VISC%MASK_R/T/X) and the adaptive state of VISC
@@ -543,17 +543,20 @@ struct mlegs_ctx {
         require(a, MLEGS_FFF, "GRAD");
         distinct({a}, {rr, rp, gz}, "GRAD");
         if (!st) st = s;
-        k_grad_fused(g, a->data, a->ln, rr->data, rp->data, gz->data, pad, st);
-        rr->space = rp->space = gz->space = MLEGS_FFF;
-        for (Field* f : {rr, rp, gz}) CK(cudaMemsetAsync(f->ln, 0, sizeof(double), st));
+        DerivArgs v{};
+        v.b = a->data;
+        v.b_ln = a->ln;
+        v.pad_b = pad;
+        deriv_out(v, 6, rr, rp, gz);
+        k_deriv(g, v, 4, st);
     }
     void pc2vel(const Field* psi_, const Field* chi_, Field* rur, Field* rup, Field* uz, int pad) {  // 1789-1853
         require(psi_, MLEGS_FFF, "PC2VEL");
         require(chi_, MLEGS_FFF, "PC2VEL");
         distinct({psi_, chi_}, {rur, rup, uz}, "PC2VEL");
-        double* zl[3] = {rur->ln, rup->ln, uz->ln};  // set to 0 by the kernel
-        k_pc2vel_fused(g, psi_->data, psi_->ln, chi_->data, chi_->ln, rur->data, rup->data, uz->data, pad, s, 0, zl);
-        rur->space = rup->space = uz->space = MLEGS_FFF;
+        DerivArgs v = deriv_in(psi_, chi_, pad);
+        deriv_out(v, 0, rur, rup, uz);
+        k_deriv(g, v, 1, s);
     }
     void pc2vor(const Field* psi_, const Field* chi_, Field* ror, Field* rop, Field* oz, int pad,
                 cudaStream_t st = nullptr) {  // 1856-1919
@@ -561,9 +564,41 @@ struct mlegs_ctx {
         require(chi_, MLEGS_FFF, "PC2VOR");
         distinct({psi_, chi_}, {ror, rop, oz}, "PC2VOR");
         if (!st) st = s;
-        k_pc2vor_fused(g, psi_->data, psi_->ln, chi_->data, chi_->ln, ror->data, rop->data, oz->data, pad, st);
-        ror->space = rop->space = oz->space = MLEGS_FFF;
-        for (Field* f : {ror, rop, oz}) CK(cudaMemsetAsync(f->ln, 0, sizeof(double), st));
+        DerivArgs v = deriv_in(psi_, chi_, pad);
+        deriv_out(v, 3, ror, rop, oz);
+        k_deriv(g, v, 2, st);
+    }
+    // PC2VEL and PC2VOR of (psi, chi) and GRAD of b at one pad, in one launch
+    // (f[0..8]: RUR RUP UZ ROR ROP OZ RBR RBP BZ).
+    void derivatives(const Field* psi_, const Field* chi_, const Field* b_, Field* const* f, int pad) {
+        for (const Field* q : {psi_, chi_, b_}) {
+            require(q, MLEGS_FFF, "CALC_BOUSSI_FORCE");
+            distinct({q}, {f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], f[8]}, "CALC_BOUSSI_FORCE");
+        }
+        DerivArgs v = deriv_in(psi_, chi_, pad);
+        v.b = b_->data;
+        v.b_ln = b_->ln;
+        v.pad_b = pad;
+        for (int q = 0; q < 9; q += 3) deriv_out(v, q, f[q], f[q + 1], f[q + 2]);
+        k_deriv(g, v, 7, s);
+    }
+    DerivArgs deriv_in(const Field* psi_, const Field* chi_, int pad) const {
+        DerivArgs v{};
+        v.psi = psi_->data;
+        v.psi_ln = psi_->ln;
+        v.chi = chi_->data;
+        v.chi_ln = chi_->ln;
+        v.pad = pad;
+        return v;
+    }
+    // outputs at o .. o + 2: FFF, LN set to 0 by the kernel
+    static void deriv_out(DerivArgs& v, int o, Field* a, Field* b_, Field* c) {
+        Field* const f[3] = {a, b_, c};
+        for (int q = 0; q < 3; ++q) {
+            v.out[o + q] = f[q]->data;
+            v.zln[o + q] = f[q]->ln;
+            f[q]->space = MLEGS_FFF;
+        }
     }
     // PROJECT (mod_legops.f90:2397-2545).  ln_mode: 0 none, 1 value, 2 PSI%LN by reference.
     void project(Field* rur, Field* rup, Field* uz, Field* psi_, Field* chi_, int ln_mode, double ln) {

@@ -182,9 +182,7 @@ void phase0(mlegs_ensemble& E, EnsInst& I) {
     I.BN = c->tmp();
     for (Field*& f : I.f) f = c->tmp();
     Field **f = I.f;
-    c->grad(c->b, f[6], f[7], f[8], P3);
-    c->pc2vel(c->psi, c->chi, f[0], f[1], f[2], P3);
-    c->pc2vor(c->psi, c->chi, f[3], f[4], f[5], P3);
+    c->derivatives(c->psi, c->chi, c->b, f, P3);
     c->copy0(f[9], c->b, 0);
     for (int q = 0; q < 10; ++q) {
         I.T[q] = c->tmp(MLEGS_PFF);

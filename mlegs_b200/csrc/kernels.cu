@@ -100,10 +100,7 @@ __global__ void delsqh_kernel(DevGrid g, const double2* a, const double* ln, dou
     int n = (int)((t / g.NXCHOPDIM) % g.NRCHOPDIM);
     int m = (int)(t / ((size_t)g.NXCHOPDIM * g.NRCHOPDIM));
     double2 v = make_double2(0.0, 0.0);
-    if (n < nrchops(g, m, pad)) {
-        int N = m + n;
-        v = cscale(a[t], -(double)(N * (N + 1)) / g.ELL2);
-    }
+    if (n < nrchops(g, m, pad)) v = cscale(a[t], g.lap[m + n]);
     if (m == 0 && n == 0 && k == 0) v = make_double2((ln ? *ln : 0.0) / g.ELL2 / g.norm0[0], 0.0);
     b[t] = v;
 }
@@ -769,8 +766,7 @@ __device__ __forceinline__ double2 xxdx_row(const DevGrid& g, int m, int k, cons
 __device__ __forceinline__ double2 delsqh_row(const DevGrid& g, int m, int k, const Col& c, int n, double ln) {
     if (m == 0 && n == 0 && k == 0) return make_double2(ln / g.ELL2 / g.norm0[0], 0.0);
     if (n < 0 || n >= c.nn) return make_double2(0.0, 0.0);
-    const int N = m + n;
-    return cscale(c.p[(size_t)n * c.st], -(double)(N * (N + 1)) / g.ELL2);
+    return cscale(c.p[(size_t)n * c.st], g.lap[m + n]);
 }
 
 // DEL2 of column c at row n (zero outside [0, nn)), log rows at (0, 0)
@@ -832,6 +828,22 @@ __device__ __forceinline__ double2 neg_xm2_delsqh(const DevGrid& g, int m, int k
     return make_double2(-v.x, -v.y);
 }
 
+// Launches over (m, n, k) tiles of 32 k by 8 rows n (fff_tiles): no division per
+// element, and a column's row neighbours are mostly the block's own rows, so they
+// come from L1.  (One flat index per thread, divided by run-time extents, and a
+// divide per row by L^2 made these kernels ALU-bound: at 192x128x256 PC2VOR took
+// 63 us, PC2VEL 51 us for 124-154 MB.)
+__device__ __forceinline__ bool tile_index(const DevGrid& g, size_t& t, int& m, int& n, int& k) {
+    k = blockIdx.x * 32 + threadIdx.x;
+    n = blockIdx.y * 8 + threadIdx.y;
+    m = blockIdx.z;
+    t = ((size_t)m * g.NRCHOPDIM + n) * g.NXCHOPDIM + k;
+    return k < g.NXCHOPDIM && n < g.NRCHOPDIM;
+}
+inline dim3 fff_tiles(const DevGrid& g) {
+    return dim3((g.NXCHOPDIM + 31) / 32, (g.NRCHOPDIM + 7) / 8, g.NTCHOPDIM);
+}
+
 __device__ __forceinline__ bool fff_index(const DevGrid& g, size_t t, int& m, int& n, int& k) {
     const size_t total = (size_t)g.NTCHOPDIM * g.NRCHOPDIM * g.NXCHOPDIM;
     if (t >= total) return false;
@@ -851,87 +863,89 @@ __device__ __forceinline__ Col column(const DevGrid& g, const double2* a, int m,
 
 }  // namespace
 
-__global__ void grad_fused_kernel(DevGrid g, const double2* a, const double* ln, double2* rr, double2* rp,
-                                  double2* gz, int pad) {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    int m, n, k;
-    if (!fff_index(g, t, m, n, k)) return;
-    const Col c = column(g, a, m, k, pad);
-    double2 v0 = make_double2(0.0, 0.0), v1 = v0, v2 = v0;
-    if (n < c.nn) {
-        const double2 an = c.p[(size_t)n * c.st];
-        v0 = xxdx_row(g, m, k, c, n, ln ? *ln : 0.0);
-        v1 = cmuli(an, (double)m);
-        v2 = cmuli(an, g.ak[k]);
-    }
-    rr[t] = v0;
-    rp[t] = v1;
-    gz[t] = v2;
+// PC2VEL (mod_legops.f90:1789-1853) of the columns (psi, chi) at row n < nn.
+__device__ __forceinline__ void pc2vel_row(const DevGrid& g, int m, int n, int k, const Col& cp, double lp,
+                                           const Col& cc, double lc, double2 (&u)[3]) {
+    const double mv = (double)m, kv = g.ak[k];
+    const double2 ps = cp.p[(size_t)n * cp.st], ch = cc.p[(size_t)n * cc.st];
+    const double2 xc = xxdx_row(g, m, k, cc, n, lc);
+    const double2 xp = xxdx_row(g, m, k, cp, n, lp);
+    u[0] = cadd(cmuli(ps, mv), cmuli(xc, kv));
+    u[1] = make_double2(-xp.x - (mv * kv) * ch.x, -xp.y - (mv * kv) * ch.y);
+    u[2] = neg_xm2_delsqh(g, m, k, cc, n, lc);
 }
 
-// sub = 1: the outputs are decremented by the velocity instead of set to it
-__global__ void pc2vel_fused_kernel(DevGrid g, const double2* psi, const double* psi_ln, const double2* chi,
-                                    const double* chi_ln, double2* rur, double2* rup, double2* uz, int pad, int sub,
-                                    double* zl0, double* zl1, double* zl2) {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+// WHICH: 1 PC2VEL -> out[0..2], 2 PC2VOR -> out[3..5], 4 GRAD -> out[6..8], any
+// of them together (a step's nine derivative fields in one launch).  sub (PC2VEL
+// alone): the outputs are decremented by the velocity instead of set to it.
+template <int WHICH>
+__global__ void __launch_bounds__(256) deriv_kernel(DevGrid g, const __grid_constant__ DerivArgs A) {
+    size_t t;
     int m, n, k;
-    if (!fff_index(g, t, m, n, k)) return;
-    // the outputs' LN slots (PC2VEL results carry no log term); read by no thread here
-    if (t < 3 && zl0) *(t == 0 ? zl0 : (t == 1 ? zl1 : zl2)) = 0.0;
-    const Col cp = column(g, psi, m, k, pad), cc = column(g, chi, m, k, pad);
-    double2 v0 = make_double2(0.0, 0.0), v1 = v0, v2 = v0;
-    if (n < cp.nn) {
-        const double lp = psi_ln ? *psi_ln : 0.0, lc = chi_ln ? *chi_ln : 0.0;
-        const double mv = (double)m, kv = g.ak[k];
-        const double2 ps = cp.p[(size_t)n * cp.st], ch = cc.p[(size_t)n * cc.st];
-        const double2 xc = xxdx_row(g, m, k, cc, n, lc);
-        const double2 xp = xxdx_row(g, m, k, cp, n, lp);
-        v0 = cadd(cmuli(ps, mv), cmuli(xc, kv));
-        v1 = make_double2(-xp.x - (mv * kv) * ch.x, -xp.y - (mv * kv) * ch.y);
-        v2 = neg_xm2_delsqh(g, m, k, cc, n, lc);
+    if (!tile_index(g, t, m, n, k)) return;
+    // the outputs' LN slots (these fields carry no log term); read by no thread here
+    if (t < 9) {
+        double* z = A.zln[t];
+        if (z) *z = 0.0;
     }
-    if (sub) {
-        v0 = csub(rur[t], v0);
-        v1 = csub(rup[t], v1);
-        v2 = csub(uz[t], v2);
+    double2 u[3], w[3], d[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) u[q] = w[q] = d[q] = make_double2(0.0, 0.0);
+    if constexpr ((WHICH & 3) != 0) {
+        const Col cp = column(g, A.psi, m, k, A.pad), cc = column(g, A.chi, m, k, A.pad);
+        if (n < cp.nn) {
+            const bool log = m == 0 && k == 0;
+            const double lp = log && A.psi_ln ? *A.psi_ln : 0.0, lc = log && A.chi_ln ? *A.chi_ln : 0.0;
+            if constexpr ((WHICH & 1) != 0) pc2vel_row(g, m, n, k, cp, lp, cc, lc, u);
+            if constexpr ((WHICH & 2) != 0) {
+                const double mv = (double)m, kv = g.ak[k];
+                const double2 ps = cp.p[(size_t)n * cp.st];
+                // oz' = DEL2(chi) at rows n-1, n, n+1; XXDX(oz') has no log rows (oz'%LN = 0)
+                const double2 dm = del2_row(g, m, k, cc, n - 1, lc), d0 = del2_row(g, m, k, cc, n, lc),
+                              dp = del2_row(g, m, k, cc, n + 1, lc);
+                const double* tb = g.xxdx + ((size_t)m * g.NB + n) * 2;
+                double2 xo = make_double2(0.0, 0.0);
+                if (n >= 1) {
+                    xo.x += tb[0] * dm.x;
+                    xo.y += tb[0] * dm.y;
+                }
+                if (n + 1 < cp.nn) {
+                    xo.x += tb[1] * dp.x;
+                    xo.y += tb[1] * dp.y;
+                }
+                const double2 xp = xxdx_row(g, m, k, cp, n, lp);
+                w[0] = cadd(cmuli(d0, -mv), cmuli(xp, kv));
+                w[1] = make_double2(xo.x - (kv * mv) * ps.x, xo.y - (kv * mv) * ps.y);
+                w[2] = neg_xm2_delsqh(g, m, k, cp, n, lp);
+            }
+        }
     }
-    rur[t] = v0;
-    rup[t] = v1;
-    uz[t] = v2;
+    if constexpr ((WHICH & 4) != 0) {
+        const Col c = column(g, A.b, m, k, A.pad_b);
+        if (n < c.nn) {
+            const double2 an = c.p[(size_t)n * c.st];
+            d[0] = xxdx_row(g, m, k, c, n, (m == 0 && k == 0 && A.b_ln) ? *A.b_ln : 0.0);
+            d[1] = cmuli(an, (double)m);
+            d[2] = cmuli(an, g.ak[k]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        if constexpr ((WHICH & 1) != 0) A.out[q][t] = A.sub ? csub(A.out[q][t], u[q]) : u[q];
+        if constexpr ((WHICH & 2) != 0) A.out[3 + q][t] = w[q];
+        if constexpr ((WHICH & 4) != 0) A.out[6 + q][t] = d[q];
+    }
 }
 
-__global__ void pc2vor_fused_kernel(DevGrid g, const double2* psi, const double* psi_ln, const double2* chi,
-                                    const double* chi_ln, double2* ror, double2* rop, double2* oz, int pad) {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    int m, n, k;
-    if (!fff_index(g, t, m, n, k)) return;
-    const Col cp = column(g, psi, m, k, pad), cc = column(g, chi, m, k, pad);
-    double2 v0 = make_double2(0.0, 0.0), v1 = v0, v2 = v0;
-    if (n < cp.nn) {
-        const double lp = psi_ln ? *psi_ln : 0.0, lc = chi_ln ? *chi_ln : 0.0;
-        const double mv = (double)m, kv = g.ak[k];
-        const double2 ps = cp.p[(size_t)n * cp.st];
-        // oz' = DEL2(chi) at rows n-1, n, n+1; XXDX(oz') has no log rows (oz'%LN = 0)
-        const double2 dm = del2_row(g, m, k, cc, n - 1, lc), d0 = del2_row(g, m, k, cc, n, lc),
-                      dp = del2_row(g, m, k, cc, n + 1, lc);
-        const double* tb = g.xxdx + ((size_t)m * g.NB + n) * 2;
-        double2 xo = make_double2(0.0, 0.0);
-        if (n >= 1) {
-            xo.x += tb[0] * dm.x;
-            xo.y += tb[0] * dm.y;
-        }
-        if (n + 1 < cp.nn) {
-            xo.x += tb[1] * dp.x;
-            xo.y += tb[1] * dp.y;
-        }
-        const double2 xp = xxdx_row(g, m, k, cp, n, lp);
-        v0 = cadd(cmuli(d0, -mv), cmuli(xp, kv));
-        v1 = make_double2(xo.x - (kv * mv) * ps.x, xo.y - (kv * mv) * ps.y);
-        v2 = neg_xm2_delsqh(g, m, k, cp, n, lp);
+void k_deriv(const DevGrid& g, const DerivArgs& a, int which, cudaStream_t s) {
+    const dim3 grid = fff_tiles(g), block(32, 8);
+    switch (which) {
+        case 1: deriv_kernel<1><<<grid, block, 0, s>>>(g, a); break;
+        case 2: deriv_kernel<2><<<grid, block, 0, s>>>(g, a); break;
+        case 4: deriv_kernel<4><<<grid, block, 0, s>>>(g, a); break;
+        default: deriv_kernel<7><<<grid, block, 0, s>>>(g, a); break;
     }
-    ror[t] = v0;
-    rop[t] = v1;
-    oz[t] = v2;
+    count_launch();
 }
 
 // The coefficient update of STEP_BOUSSI_ETDAB_CN (mod_march.f90:811-901) from
@@ -948,24 +962,16 @@ __device__ __forceinline__ void pc2vel_at(const DevGrid& g, int m, int n, int k,
                                           const double2* chi, double lc, int pad, double2 (&u)[3]) {
     const Col cp = column(g, psi, m, k, pad), cc = column(g, chi, m, k, pad);
     u[0] = u[1] = u[2] = make_double2(0.0, 0.0);
-    if (n < cp.nn) {
-        const double mv = (double)m, kv = g.ak[k];
-        const double2 ps = cp.p[(size_t)n * cp.st], ch = cc.p[(size_t)n * cc.st];
-        const double2 xc = xxdx_row(g, m, k, cc, n, lc);
-        const double2 xp = xxdx_row(g, m, k, cp, n, lp);
-        u[0] = cadd(cmuli(ps, mv), cmuli(xc, kv));
-        u[1] = make_double2(-xp.x - (mv * kv) * ch.x, -xp.y - (mv * kv) * ch.y);
-        u[2] = neg_xm2_delsqh(g, m, k, cc, n, lc);
-    }
+    if (n < cp.nn) pc2vel_row(g, m, n, k, cp, lp, cc, lc, u);
 }
 
 // Three 256-thread blocks per SM (at most 80 registers; a few bytes spill):
 // the kernel is bound by memory-level parallelism, and this beats the 98-register
 // form at two blocks per SM.
 __global__ void __launch_bounds__(256, 3) etd_ab_fused_kernel(DevGrid g, EtdAbArgs a) {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    size_t t;
     int m, n, k;
-    if (!fff_index(g, t, m, n, k)) return;
+    if (!tile_index(g, t, m, n, k)) return;
     if (t < 3) *a.out_ln[t] = 0.0;
     double fv = 1.0, fd = 1.0;
     if (a.hyper) {
@@ -1286,31 +1292,7 @@ void k_ab2_visc_rhs(const DevGrid& g, const Ab2Args& a, cudaStream_t s) {
 }
 
 void k_etd_ab_fused(const DevGrid& g, const EtdAbArgs& a, cudaStream_t s) {
-    const size_t n = g.NTCHOPDIM * (size_t)g.NRCHOPDIM * g.NXCHOPDIM;
-    etd_ab_fused_kernel<<<nblk(n, 256), 256, 0, s>>>(g, a);
-    count_launch();
-}
-
-void k_grad_fused(const DevGrid& g, const double2* a, const double* ln, double2* rr, double2* rp, double2* gz, int pad,
-                  cudaStream_t s) {
-    const size_t n = g.NTCHOPDIM * (size_t)g.NRCHOPDIM * g.NXCHOPDIM;
-    grad_fused_kernel<<<nblk(n, 256), 256, 0, s>>>(g, a, ln, rr, rp, gz, pad);
-    count_launch();
-}
-
-void k_pc2vel_fused(const DevGrid& g, const double2* psi, const double* psi_ln, const double2* chi, const double* chi_ln,
-                    double2* rur, double2* rup, double2* uz, int pad, cudaStream_t s, int sub, double* const* zero_ln) {
-    const size_t n = g.NTCHOPDIM * (size_t)g.NRCHOPDIM * g.NXCHOPDIM;
-    pc2vel_fused_kernel<<<nblk(n, 256), 256, 0, s>>>(g, psi, psi_ln, chi, chi_ln, rur, rup, uz, pad, sub,
-                                                     zero_ln ? zero_ln[0] : nullptr, zero_ln ? zero_ln[1] : nullptr,
-                                                     zero_ln ? zero_ln[2] : nullptr);
-    count_launch();
-}
-
-void k_pc2vor_fused(const DevGrid& g, const double2* psi, const double* psi_ln, const double2* chi, const double* chi_ln,
-                    double2* ror, double2* rop, double2* oz, int pad, cudaStream_t s) {
-    const size_t n = g.NTCHOPDIM * (size_t)g.NRCHOPDIM * g.NXCHOPDIM;
-    pc2vor_fused_kernel<<<nblk(n, 256), 256, 0, s>>>(g, psi, psi_ln, chi, chi_ln, ror, rop, oz, pad);
+    etd_ab_fused_kernel<<<fff_tiles(g), dim3(32, 8), 0, s>>>(g, a);
     count_launch();
 }
 

@@ -64,6 +64,7 @@ struct DevGrid {
     const double* xm;       // [NTCHOPDIM][NB][2]  (sub, super)     diag = 1
     const double* del2h;    // [NTCHOPDIM][NB][5]
     int NB;                 // NRCHOPDIM + 2
+    const double* lap;      // -N (N + 1) / ELL2 by degree N = m + n (DELSQH's diagonal)
 };
 
 struct Field {
@@ -258,14 +259,16 @@ void k_band3(const DevGrid& g, const double2* a, double2* b, int which /*0 xxdx,
 void k_del2(const DevGrid& g, const double2* a, double2* b, int pad, cudaStream_t s);
 void k_logterm_rows(const DevGrid& g, double2* b, const double* ln, int which, double coef, cudaStream_t s);
 void k_mk_combine(const DevGrid& g, int op, const double2* x, const double2* y, double2* out, int pad, cudaStream_t s);
-// GRAD, PC2VEL, PC2VOR each in one pass (kernels.cu); outputs FFF, log terms read from *ln.
-void k_grad_fused(const DevGrid& g, const double2* a, const double* ln, double2* rr, double2* rp, double2* gz, int pad,
-                  cudaStream_t s);
-void k_pc2vel_fused(const DevGrid& g, const double2* psi, const double* psi_ln, const double2* chi, const double* chi_ln,
-                    double2* rur, double2* rup, double2* uz, int pad, cudaStream_t s, int sub = 0,
-                    double* const* zero_ln = nullptr);
-void k_pc2vor_fused(const DevGrid& g, const double2* psi, const double* psi_ln, const double2* chi, const double* chi_ln,
-                    double2* ror, double2* rop, double2* oz, int pad, cudaStream_t s);
+// GRAD, PC2VEL, PC2VOR (kernels.cu), alone or in one pass; outputs FFF.  which:
+// 1 PC2VEL -> out[0..2], 2 PC2VOR -> out[3..5], 4 GRAD -> out[6..8], 7 all.
+struct DerivArgs {
+    const double2 *psi, *chi, *b;
+    const double *psi_ln, *chi_ln, *b_ln;  // log terms (null: none)
+    double2* out[9];
+    double* zln[9];                        // LN slots set to 0 (null: none)
+    int pad, pad_b, sub;                   // sub (which = 1): out -= instead of out =
+};
+void k_deriv(const DevGrid& g, const DerivArgs& a, int which, cudaStream_t s);
 void k_farfield_fix(const DevGrid& g, double2* a, int nr_sum, cudaStream_t s, int by_pf = 0);
 // IHELMP (solve.cu): dq = DEL2H power tables [m][q][rows][4q+1], scratch of
 // ihelmp_scratch_doubles(g, P) doubles; a is solved in place, ln = A%LN.
