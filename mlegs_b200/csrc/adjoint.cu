@@ -141,290 +141,6 @@ __global__ void __launch_bounds__(256) farfield_T_kernel(const DevGrid g, double
     if (ny == 0) y[k] = make_double2(0.0, 0.0);
 }
 
-// Transposed banded solves with the stored unpivoted factors A = L U of the
-// forward solves (solve.cu: F5 [row][5][system] = L(r, r-2), L(r, r-1),
-// U(r, r), U(r, r+1), U(r, r+2); F7 [row][7][k] = L(r, r-3 .. r-1), U(r, r ..
-// r+3)).  A^T x = y is U^T z = y, then L^T x = z.  One thread per (system, real
-// or imaginary part), in place on the FFF field, rows from the system size on
-// left as they are.
-//   kind 0  IDEL2LN: 5-band factors for every (m, k);
-//   kind 2  IHELM: m >= 1 5-band; m = 0 the forward solves (H XM) v = rhs on
-//           NN - 1 rows and returns XM v (NN rows), so the transpose forms
-//           w = XM^T y, solves (H XM)^T on NN - 1 rows and zeroes row NN - 1.
-// The substitutions run in load blocks of TB (TW for the 7-band systems)
-// rows: a block's right-hand sides and factors are loaded together, the
-// diagonal's reciprocal and the scaled off-diagonals are formed off the
-// recurrence, which then costs one dependent FMA per row.  wpad idle threads
-// after the 7-band m = 0 systems of kind 2 keep them in warps of their own.
-__global__ void __launch_bounds__(128) solve_T_kernel(const DevGrid g, const double* __restrict__ F5,
-                                                      const double* __restrict__ F7, double2* yfield, int kind,
-                                                      int pad, int wpad) {
-    constexpr int TB = 16, TW = 8;
-    const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    int u = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nw = 2 * g.NXCHOPDIM;
-    if (wpad) {
-        if (u >= nw && u < nw + wpad) return;
-        if (u >= nw) u -= wpad;
-    }
-    const int t = u >> 1, comp = u & 1;
-    if (t >= nsys) return;
-    const int k = t % g.NXCHOPDIM, m = t / g.NXCHOPDIM;
-    const int nn = nrc(g, m, pad);
-    double* col = (double*)(yfield + (size_t)m * g.NRCHOPDIM * g.NXCHOPDIM + k) + comp;
-    const size_t st = 2 * (size_t)g.NXCHOPDIM;
-    if (!(m == 0 && kind == 2)) {
-        const int size = nn;
-        // U^T z = y: z(r) = (y(r) - U(r-1, r) z(r-1) - U(r-2, r) z(r-2)) / U(r, r)
-        double z1 = 0.0, z2 = 0.0;
-        for (int r0 = 0; r0 < size; r0 += TB) {
-            double yv[TB], a1[TB], a2[TB];
-#pragma unroll
-            for (int q = 0; q < TB; ++q) {
-                const int r = r0 + q;
-                const bool ok = r < size;
-                yv[q] = ok ? col[(size_t)r * st] : 0.0;
-                const double d = ok ? F5[((size_t)r * 5 + 2) * nsys + t] : 1.0;
-                a1[q] = (ok && r >= 1) ? F5[((size_t)(r - 1) * 5 + 3) * nsys + t] : 0.0;
-                a2[q] = (ok && r >= 2) ? F5[((size_t)(r - 2) * 5 + 4) * nsys + t] : 0.0;
-                const double ri = 1.0 / d;
-                yv[q] = __dmul_rn(yv[q], ri);
-                a1[q] = __dmul_rn(a1[q], ri);
-                a2[q] = __dmul_rn(a2[q], ri);
-            }
-#pragma unroll
-            for (int q = 0; q < TB; ++q) {
-                if (r0 + q >= size) break;
-                const double v = __fma_rn(-a1[q], z1, __fma_rn(-a2[q], z2, yv[q]));
-                col[(size_t)(r0 + q) * st] = v;
-                z2 = z1;
-                z1 = v;
-            }
-        }
-        // L^T x = z: x(r) = z(r) - L(r+1, r) x(r+1) - L(r+2, r) x(r+2)
-        double x1 = 0.0, x2 = 0.0;
-        for (int r1 = size - 1; r1 >= 0; r1 -= TB) {
-            double zv[TB], e1[TB], e2[TB];
-#pragma unroll
-            for (int q = 0; q < TB; ++q) {
-                const int r = r1 - q;
-                const bool ok = r >= 0;
-                zv[q] = ok ? col[(size_t)r * st] : 0.0;
-                e1[q] = (ok && r + 1 < size) ? F5[((size_t)(r + 1) * 5 + 1) * nsys + t] : 0.0;
-                e2[q] = (ok && r + 2 < size) ? F5[((size_t)(r + 2) * 5 + 0) * nsys + t] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < TB; ++q) {
-                const int r = r1 - q;
-                if (r < 0) break;
-                const double v = __fma_rn(-e1[q], x1, __fma_rn(-e2[q], x2, zv[q]));
-                col[(size_t)r * st] = v;
-                x2 = x1;
-                x1 = v;
-            }
-        }
-        return;
-    }
-    if (nn <= 0) return;
-    // w = XM^T y: w(r) = y(r) + XM(r+1, r) y(r+1) + XM(r-1, r) y(r-1), with
-    // XM(l, l-1) = sub(l), XM(l, l+1) = super(l) (the m = 0 table [row][2])
-    const double* xm = g.xm;
-    {
-        double prev = 0.0;
-        for (int r0 = 0; r0 < nn; r0 += TW) {
-            double yv[TW + 1];
-#pragma unroll
-            for (int q = 0; q <= TW; ++q) yv[q] = (r0 + q < nn) ? col[(size_t)(r0 + q) * st] : 0.0;
-#pragma unroll
-            for (int q = 0; q < TW; ++q) {
-                const int r = r0 + q;
-                if (r >= nn) break;
-                double v = yv[q];
-                if (r + 1 < nn) v = __fma_rn(xm[(size_t)(r + 1) * 2 + 0], yv[q + 1], v);
-                if (r >= 1) v = __fma_rn(xm[(size_t)(r - 1) * 2 + 1], prev, v);
-                col[(size_t)r * st] = v;
-                prev = yv[q];
-            }
-        }
-    }
-    const int size = nn - 1;
-    const size_t NK = g.NXCHOPDIM;
-    auto f7 = [&](int r, int j) { return F7[((size_t)r * 7 + j) * NK + k]; };
-    double z1 = 0.0, z2 = 0.0, z3 = 0.0;
-    for (int r0 = 0; r0 < size; r0 += TW) {
-        double yv[TW], a1[TW], a2[TW], a3[TW];
-#pragma unroll
-        for (int q = 0; q < TW; ++q) {
-            const int r = r0 + q;
-            const bool ok = r < size;
-            yv[q] = ok ? col[(size_t)r * st] : 0.0;
-            const double d = ok ? f7(r, 3) : 1.0;
-            a1[q] = (ok && r >= 1) ? f7(r - 1, 4) : 0.0;
-            a2[q] = (ok && r >= 2) ? f7(r - 2, 5) : 0.0;
-            a3[q] = (ok && r >= 3) ? f7(r - 3, 6) : 0.0;
-            const double ri = 1.0 / d;
-            yv[q] = __dmul_rn(yv[q], ri);
-            a1[q] = __dmul_rn(a1[q], ri);
-            a2[q] = __dmul_rn(a2[q], ri);
-            a3[q] = __dmul_rn(a3[q], ri);
-        }
-#pragma unroll
-        for (int q = 0; q < TW; ++q) {
-            if (r0 + q >= size) break;
-            const double v = __fma_rn(-a1[q], z1, __fma_rn(-a2[q], z2, __fma_rn(-a3[q], z3, yv[q])));
-            col[(size_t)(r0 + q) * st] = v;
-            z3 = z2;
-            z2 = z1;
-            z1 = v;
-        }
-    }
-    double x1 = 0.0, x2 = 0.0, x3 = 0.0;
-    for (int r1 = size - 1; r1 >= 0; r1 -= TW) {
-        double zv[TW], c1[TW], c2[TW], c3[TW];
-#pragma unroll
-        for (int q = 0; q < TW; ++q) {
-            const int r = r1 - q;
-            const bool ok = r >= 0;
-            zv[q] = ok ? col[(size_t)r * st] : 0.0;
-            c1[q] = (ok && r + 1 < size) ? f7(r + 1, 2) : 0.0;
-            c2[q] = (ok && r + 2 < size) ? f7(r + 2, 1) : 0.0;
-            c3[q] = (ok && r + 3 < size) ? f7(r + 3, 0) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < TW; ++q) {
-            const int r = r1 - q;
-            if (r < 0) break;
-            const double v = __fma_rn(-c1[q], x1, __fma_rn(-c2[q], x2, __fma_rn(-c3[q], x3, zv[q])));
-            col[(size_t)r * st] = v;
-            x3 = x2;
-            x2 = x1;
-            x1 = v;
-        }
-    }
-    col[(size_t)size * st] = 0.0;
-}
-
-// solve_T_kernel for small systems (NRCHOP + pad <= 72 rows): one warp takes 16
-// systems, copies their factor rows and columns into shared memory in one
-// burst of cp.async copies, and runs the same substitutions there; rows from
-// the system size on are left as they are.  Blocks [0, nb0) hold the 7-band
-// m = 0 systems of kind 2.  Shared memory per block: R x 144 doubles.
-__global__ void __launch_bounds__(32) solve_T_small_kernel(const DevGrid g, const double* __restrict__ F5,
-                                                           const double* __restrict__ F7, double2* yfield, int kind,
-                                                           int pad, int t_begin, int nb0) {
-    extern __shared__ __align__(16) double sms[];
-    const int R = g.NRCHOP + pad;
-    double* Fs = sms;                         // [R][7][16]
-    double2* Xs = (double2*)(sms + R * 112);  // [R][16]
-    const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    const int lane = threadIdx.x, sy = lane >> 1, comp = lane & 1;
-    const bool wide = (int)blockIdx.x < nb0;
-    const int tb = wide ? blockIdx.x * 16 : t_begin + (blockIdx.x - nb0) * 16;
-    const int nsb = min(16, (wide ? t_begin : nsys) - tb);
-    const size_t NK = g.NXCHOPDIM;
-    if (wide) {
-        for (int e = lane; e < R * 112; e += 32) {
-            const int r = e / 112, j = (e / 16) % 7, q = e % 16;
-            if (q < nsb)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(Fs + e)),
-                             "l"(F7 + ((size_t)r * 7 + j) * NK + tb + q)
-                             : "memory");
-        }
-    } else {
-        for (int e = lane; e < R * 80; e += 32) {
-            const int r = e / 80, j = (e / 16) % 5, q = e % 16;
-            if (q < nsb)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(Fs + (r * 7 + j) * 16 + q)),
-                             "l"(F5 + ((size_t)r * 5 + j) * nsys + tb + q)
-                             : "memory");
-        }
-    }
-    for (int e = lane; e < R * 16; e += 32) {
-        const int r = e / 16, q = e % 16;
-        if (q < nsb) {
-            const int tq = tb + q, mq = tq / g.NXCHOPDIM, kq = tq - mq * g.NXCHOPDIM;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(Xs + e)),
-                         "l"(yfield + (size_t)mq * g.NRCHOPDIM * NK + (size_t)r * NK + kq)
-                         : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-    if (sy >= nsb) return;
-    const int t = tb + sy, k = t % g.NXCHOPDIM, m = t / g.NXCHOPDIM;
-    const int nn = nrc(g, m, pad);
-    double* X = (double*)Xs + sy * 2 + comp;  // row r at X[r * 32]
-    auto F = [&](int r, int j) { return Fs[(r * 7 + j) * 16 + sy]; };
-    int rows_out = 0;
-    if (!wide) {
-        const int size = nn;
-        double z1 = 0.0, z2 = 0.0;
-        for (int r = 0; r < size; ++r) {
-            const double ri = 1.0 / F(r, 2);
-            const double a1 = r >= 1 ? __dmul_rn(F(r - 1, 3), ri) : 0.0;
-            const double a2 = r >= 2 ? __dmul_rn(F(r - 2, 4), ri) : 0.0;
-            const double v = __fma_rn(-a1, z1, __fma_rn(-a2, z2, __dmul_rn(X[r * 32], ri)));
-            X[r * 32] = v;
-            z2 = z1;
-            z1 = v;
-        }
-        double x1 = 0.0, x2 = 0.0;
-        for (int r = size - 1; r >= 0; --r) {
-            const double e1 = r + 1 < size ? F(r + 1, 1) : 0.0;
-            const double e2 = r + 2 < size ? F(r + 2, 0) : 0.0;
-            const double v = __fma_rn(-e1, x1, __fma_rn(-e2, x2, X[r * 32]));
-            X[r * 32] = v;
-            x2 = x1;
-            x1 = v;
-        }
-        rows_out = size;
-    } else if (nn > 0) {
-        // w = XM^T y, then the transposed 7-band solve on NN - 1 rows, row NN - 1 zeroed
-        const double* xm = g.xm;
-        double prev = 0.0;
-        for (int r = 0; r < nn; ++r) {
-            const double yr = X[r * 32];
-            double v = yr;
-            if (r + 1 < nn) v = __fma_rn(xm[(size_t)(r + 1) * 2 + 0], X[(r + 1) * 32], v);
-            if (r >= 1) v = __fma_rn(xm[(size_t)(r - 1) * 2 + 1], prev, v);
-            X[r * 32] = v;
-            prev = yr;
-        }
-        const int size = nn - 1;
-        double z1 = 0.0, z2 = 0.0, z3 = 0.0;
-        for (int r = 0; r < size; ++r) {
-            const double ri = 1.0 / F(r, 3);
-            const double a1 = r >= 1 ? __dmul_rn(F(r - 1, 4), ri) : 0.0;
-            const double a2 = r >= 2 ? __dmul_rn(F(r - 2, 5), ri) : 0.0;
-            const double a3 = r >= 3 ? __dmul_rn(F(r - 3, 6), ri) : 0.0;
-            const double v = __fma_rn(-a1, z1, __fma_rn(-a2, z2, __fma_rn(-a3, z3, __dmul_rn(X[r * 32], ri))));
-            X[r * 32] = v;
-            z3 = z2;
-            z2 = z1;
-            z1 = v;
-        }
-        double x1 = 0.0, x2 = 0.0, x3 = 0.0;
-        for (int r = size - 1; r >= 0; --r) {
-            const double c1 = r + 1 < size ? F(r + 1, 2) : 0.0;
-            const double c2 = r + 2 < size ? F(r + 2, 1) : 0.0;
-            const double c3 = r + 3 < size ? F(r + 3, 0) : 0.0;
-            const double v = __fma_rn(-c1, x1, __fma_rn(-c2, x2, __fma_rn(-c3, x3, X[r * 32])));
-            X[r * 32] = v;
-            x3 = x2;
-            x2 = x1;
-            x1 = v;
-        }
-        X[size * 32] = 0.0;
-        rows_out = nn;
-    }
-    double* col = (double*)(yfield + (size_t)m * g.NRCHOPDIM * NK + k) + comp;
-    const size_t st = 2 * NK;
-    for (int r = 0; r < rows_out; ++r) col[(size_t)r * st] = X[r * 32];
-}
-
 // Adjoints of VPRODSUB's cross product and VDOTPSUB's dot product
 // (mod_legops.f90:2105-2130, 2207-2225), pointwise on the packed physical
 // samples [r][z][j] (real and imaginary parts are separate samples):
@@ -802,25 +518,7 @@ struct Adj {
         if (!f) throw ApiError(MLEGS_ERR_STATE, "adjoint: banded-solve factors unavailable");
         return f;
     }
-    void solve_T(const mlegs_ctx::SolveFactors* f, Field* y, int kind) {
-        if (c->d.NRCHOP <= 72) {  // the whole system fits in shared memory
-            const int nsys = c->d.NTCHOPDIM * c->d.NXCHOPDIM, t_begin = kind == 2 ? c->d.NXCHOPDIM : 0;
-            const int nb0 = (t_begin + 15) / 16, nb1 = (nsys - t_begin + 15) / 16;
-            const size_t smem = (size_t)c->d.NRCHOP * 144 * sizeof(double);
-            static size_t attr = 0;
-            if (smem > attr && smem > 48 * 1024) {
-                cudaFuncSetAttribute(solve_T_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                attr = smem;
-            }
-            solve_T_small_kernel<<<nb0 + nb1, 32, smem, s()>>>(g(), f->F5, f->F7, y->data, kind, 0, t_begin, nb0);
-            count_launch();
-            return;
-        }
-        const int nw = 2 * c->d.NXCHOPDIM, wpad = kind == 2 ? (32 - nw % 32) % 32 : 0;
-        const int n = 2 * c->d.NTCHOPDIM * c->d.NXCHOPDIM + wpad;
-        solve_T_kernel<<<nb(n, 128), 128, 0, s()>>>(g(), f->F5, f->F7, y->data, kind, 0, wpad);
-        count_launch();
-    }
+    void solve_T(const mlegs_ctx::SolveFactors* f, Field* y, int kind) { k_solve_T(g(), f->F, y->data, kind, 0, s()); }
     // IDEL2LN(B, A) (mod_legops.f90:1013-1176) as B -> (A, A%LN): A_bar -> B_bar (LN 0)
     void idel2ln_T(const Field* ab, Field* out) {
         const auto* f = factors(0, 0.0);

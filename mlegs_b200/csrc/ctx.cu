@@ -420,7 +420,11 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     CK(cudaMemsetAsync(lnslots, 0, nslots * sizeof(double), s));
     scratch = dalloc<double2>(d.cap());
     pipe_group = d.pff() * sizeof(double2) <= PIPE_ALL_BYTES ? BATCH : 3;
-    for (int q = 0; q < (pipe_group == BATCH ? BATCH : 2 * pipe_group); ++q) pbuf[q] = dalloc<double2>(d.pff());
+    {
+        const int images = pipe_group == BATCH ? BATCH : 2 * pipe_group;
+        double2* slab = dalloc<double2>(images * d.pff());
+        for (int q = 0; q < images; ++q) pbuf[q] = slab + q * d.pff();
+    }
     size_t nsys = (size_t)d.NTCHOPDIM * d.NXCHOPDIM;
     solve_scr = dalloc<double>((size_t)d.NRCHOPDIM * 4 * nsys);
     size_t ref_max = (size_t)d.NDIMR * d.NDIMTH * d.NX;
@@ -430,6 +434,7 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     dflag = dalloc<int>(1);
     split_err = dalloc<int>(1);
     CK(cudaMemsetAsync(split_err, 0, sizeof(int), s));
+    g.err = split_err;
     if (p.precision == MLEGS_PREC_SPLIT) {
         const int S = p.split_slices > 0 ? p.split_slices : 6;
         if (!split_supported(g, S, d.NRCHOPDIM + 1))
@@ -1136,8 +1141,7 @@ bool mlegs_ctx::ab2_visc_fused(Field* PN, Field* CN, Field* BN) {
         a.alp[q] = 2 / nu[q] / p.dt;
         const SolveFactors* f = factors(2, 0, a.alp[q]);
         if (!f) return false;
-        sb.p[q].F5 = f->F5;
-        sb.p[q].F7 = f->F7;
+        sb.p[q].F = f->F;
     }
     Field* WK[3] = {tmp(), tmp(), tmp()};
     for (int q = 0; q < 3; ++q) {
@@ -1422,7 +1426,7 @@ int mlegs_sync(mlegs_ctx* ctx) {
         CK(cudaMemcpy(&e, ctx->split_err, sizeof(int), cudaMemcpyDeviceToHost));
         if (e) {  // reported once; the context stays usable
             CK(cudaMemset(ctx->split_err, 0, sizeof(int)));
-            throw ApiError(MLEGS_ERR_TIMEOUT, "tensor-core GEMM: a bounded wait timed out (results invalid)");
+            throw ApiError(MLEGS_ERR_TIMEOUT, "a bounded pipeline wait timed out (results invalid)");
         }
         if (bulk_gemm_error(true) > 0)
             throw ApiError(MLEGS_ERR_TIMEOUT, "RTRAN(+1) GEMM: a bounded pipeline wait timed out (results invalid)");
@@ -2189,7 +2193,7 @@ int mlegs_kernel_time(mlegs_ctx* ctx, int kernel, int reps, double* ms_per_launc
                     break;
                 case 7: {
                     const auto* f = ctx->factors(0, 0, 0.0);
-                    if (f) k_solve_factored(g, f->F5, f->F7, a->data, b->data, c->ln, 0, 0, 0.0, 0, 1, s);
+                    if (f) k_solve_factored(g, f->F, a->data, b->data, c->ln, 0, 0, 0.0, 0, 1, s);
                     else k_solve_del2(g, a->data, c->ln, 0, 0.0, 0, 0.0, nullptr, ctx->solve_scr, 0, s);
                 } break;
                 case 8: {

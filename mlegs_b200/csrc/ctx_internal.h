@@ -427,7 +427,7 @@ struct mlegs_ctx {
     struct SolveFactors {
         int kind, pad;
         double alp;
-        double *F5, *F7;
+        double* F;
     };
     std::deque<SolveFactors> sfac;  // a deque: entries stay put as the cache grows
     const SolveFactors* factors(int kind, int pad, double alp) {
@@ -437,17 +437,15 @@ struct mlegs_ctx {
         CK(cudaStreamIsCapturing(s, &cs));
         if (cs != cudaStreamCaptureStatusNone || sfac.size() >= 16 || pad < 0 || d.NRCHOP + pad > d.NRCHOPDIM)
             return nullptr;
-        size_t n5, n7;
-        solve_factor_sizes(g, &n5, &n7);
-        SolveFactors f{kind, pad, alp, dalloc<double>(n5), dalloc<double>(n7)};
-        k_solve_factor(g, kind, alp, pad, f.F5, f.F7, s);
+        SolveFactors f{kind, pad, alp, dalloc<double>(solve_factor_doubles(g))};
+        k_solve_factor(g, kind, alp, pad, f.F, s);
         sfac.push_back(f);
         return &sfac.back();
     }
     void idel2(const Field* bb, Field* a, int has_ln, double ln, int pad) {
         require(bb, MLEGS_FFF, "IDEL2");
         if (const SolveFactors* f = factors(1, pad, 0.0)) {
-            k_solve_factored(g, f->F5, f->F7, bb->data, a->data, a->ln, 1, has_ln, ln, pad, 1, s);
+            k_solve_factored(g, f->F, bb->data, a->data, a->ln, 1, has_ln, ln, pad, 1, s);
             a->space = MLEGS_FFF;
             return;
         }
@@ -460,7 +458,7 @@ struct mlegs_ctx {
     void idel2ln(const Field* bb, Field* a, int pad) {  // 1013-1176
         require(bb, MLEGS_FFF, "IDEL2LN");
         if (const SolveFactors* f = factors(0, pad, 0.0)) {
-            k_solve_factored(g, f->F5, f->F7, bb->data, a->data, a->ln, 0, 0, 0.0, pad, 1, s);
+            k_solve_factored(g, f->F, bb->data, a->data, a->ln, 0, 0, 0.0, pad, 1, s);
             a->space = MLEGS_FFF;
             return;
         }
@@ -473,13 +471,15 @@ struct mlegs_ctx {
     void ihelm(const Field* bb, Field* a, double alp, int pad) {  // 1204-1354
         require(bb, MLEGS_FFF, "IHELM");
         if (alp == 0.0) throw ApiError(MLEGS_ERR_LEGOPERATOR, "IHELM: ALP CAN'T BE ZERO");
+        if (const SolveFactors* f = factors(2, pad, alp)) {
+            k_solve_factored(g, f->F, bb->data, a->data, a->ln, 2, 0, 0.0, pad, 0, s, bb->ln, -1.0 / alp);
+            a->space = MLEGS_FFF;
+            return;
+        }
         copy0(a, bb, pad);
-        k_ln_copy(a->ln, bb->ln, -1.0 / alp, s);      // A%LN = -B%LN/ALP
+        k_ln_copy(a->ln, bb->ln, -1.0 / alp, s);       // A%LN = -B%LN/ALP
         k_logterm_rows(g, a->data, a->ln, 2, 1.0, s);  // rhs -= LN * DEL2(log)
-        if (const SolveFactors* f = factors(2, pad, alp))
-            k_solve_factored(g, f->F5, f->F7, a->data, a->data, nullptr, 2, 0, 0.0, pad, 0, s);
-        else
-            k_solve_del2(g, a->data, nullptr, 2, alp, 0, 0.0, nullptr, solve_scr, pad, s);
+        k_solve_del2(g, a->data, nullptr, 2, alp, 0, 0.0, nullptr, solve_scr, pad, s);
         chopdo(a, pad);
     }
     // IHELMP (mod_legops.f90:1409-1592): DEL2H power tables per P (built on the

@@ -157,7 +157,9 @@ struct mlegs_ensemble {
     }
     void launch_solve(Group<GroupSolve>& G) {
         upload<GroupSolve>(G, [](GroupSolve& p) { return group_solve_blocks(p); });
-        if (G.total) k_grouped_solve(G.d, G.d_first, (int)G.up.size(), G.total, gs);
+        G.smem = 0;
+        for (const GroupSolve& p : G.up) G.smem = std::max(G.smem, group_solve_smem(p));
+        if (G.total) k_grouped_solve(G.d, G.d_first, (int)G.up.size(), G.total, G.smem, gs);
     }
 
     void prepare();
@@ -277,11 +279,10 @@ void phase2(mlegs_ensemble& E, EnsInst& I) {
     if (!fc) throw ApiError(MLEGS_ERR_STATE, "ensemble: IDEL2LN factors missing");
     GroupSolve p{};
     p.g = c->g;
-    p.F5 = fc->F5;
-    p.F7 = fc->F7;
-    p.src = I.Wf->data;
-    p.dst = I.CN->data;
-    p.ln_out = I.CN->ln;
+    p.it.F = fc->F;
+    p.it.src = I.Wf->data;
+    p.it.dst = I.CN->data;
+    p.it.ln_out = I.CN->ln;
     p.kind = 0;
     p.farfield = 1;
     I.CN->space = MLEGS_FFF;
@@ -336,10 +337,9 @@ void phase3(mlegs_ensemble& E, EnsInst& I) {
         if (!fh) throw ApiError(MLEGS_ERR_STATE, "ensemble: IHELM factors missing");
         GroupSolve p{};
         p.g = g;
-        p.F5 = fh->F5;
-        p.F7 = fh->F7;
-        p.src = A[q]->data;
-        p.dst = A[q]->data;
+        p.it.F = fh->F;
+        p.it.src = A[q]->data;
+        p.it.dst = A[q]->data;
         p.kind = 2;
         E.gs2.h.push_back(p);
         I.WK[q] = WK;

@@ -65,6 +65,7 @@ struct DevGrid {
     const double* del2h;    // [NTCHOPDIM][NB][5]
     int NB;                 // NRCHOPDIM + 2
     const double* lap;      // -N (N + 1) / ELL2 by degree N = m + n (DELSQH's diagonal)
+    int* err;               // the context's error word: set to 1 when a bounded wait runs out
 };
 
 struct Field {
@@ -156,22 +157,36 @@ void k_grouped_b2p(const GroupB2P* d, const int* first, int np, int total, size_
                    cudaStream_t s);
 void k_grouped_fold(const GroupFold* d, const int* first, int np, int total, size_t smem, int ctas, int* next,
                     cudaStream_t s);
-// Grouped banded substitutions (solve.cu): one problem per (instance, solve);
-// 64 systems (128 threads: real and imaginary parts) per block, `first` =
-// the problem's first block.
-struct GroupSolve {
-    DevGrid g;
-    const double* F5;
-    const double* F7;
+// Grouped banded substitutions (solve.cu): one problem per (instance, solve),
+// 16 systems per block, `first` = the problem's first block.
+// Several fields' solves of one kind and pad in one launch; ln_dst[j] <- ln_src[j]
+// (null: none) are LN copies the launch makes on the side.  ln_rhs (IHELM, null:
+// none): the right-hand side's LN, times ln_scale the solution's, which goes to
+// ln_out and whose DEL2 image is taken off the right-hand side.
+struct SolveItem {
+    const double* F;  // k_solve_factor's table
     const double2* src;
     double2* dst;
     double* ln_out;
+    const double* ln_rhs;
+    double ln_scale;
+    const double* ln_src[2];
+    double* ln_dst[2];
+};
+struct SolveBatch {
+    SolveItem p[3];
+    int n;
+};
+struct GroupSolve {
+    DevGrid g;
+    SolveItem it;
     int kind, has_ln;
     double ln_in;
     int pad, farfield, first;
 };
 int group_solve_blocks(const GroupSolve& p);
-void k_grouped_solve(const GroupSolve* d, const int* first, int np, int total_blocks, cudaStream_t s);
+size_t group_solve_smem(const GroupSolve& p);
+void k_grouped_solve(const GroupSolve* d, const int* first, int np, int total_blocks, size_t smem, cudaStream_t s);
 // RTRAN(+1) with bulk-copy staging and a warp-specialised mbarrier pipeline
 // (gemm_bulk.cu), the form k_rtran_b2p takes when supported; a timed-out
 // wait raises the module's error word, read (and cleared) by bulk_gemm_error.
@@ -291,25 +306,13 @@ void k_solve_del2(const DevGrid& g, double2* a, double* ln_out, int kind, double
 // Factor-once form of the same solves (solve.cu): LU factors of every (m, k)
 // system for one (kind, pad, alp), then substitutions only; src -> dst with
 // rows past the system size zeroed, farfield = 1 adds the CALCAT1 row-0 fix.
-void solve_factor_sizes(const DevGrid& g, size_t* f5, size_t* f7);
-void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F5, double* F7, cudaStream_t s);
-void k_solve_factored(const DevGrid& g, const double* F5, const double* F7, const double2* src, double2* dst,
-                      double* ln_out, int kind, int has_ln, double ln_in, int pad, int farfield, cudaStream_t s);
-// Several fields' solves of one kind and pad in one launch; ln_dst[j] <- ln_src[j]
-// (null: none) are LN copies the launch makes on the side.
-struct SolveItem {
-    const double* F5;
-    const double* F7;
-    const double2* src;
-    double2* dst;
-    double* ln_out;
-    const double* ln_src[2];
-    double* ln_dst[2];
-};
-struct SolveBatch {
-    SolveItem p[3];
-    int n;
-};
+size_t solve_factor_doubles(const DevGrid& g);
+void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F, cudaStream_t s);
+void k_solve_factored(const DevGrid& g, const double* F, const double2* src, double2* dst, double* ln_out, int kind,
+                      int has_ln, double ln_in, int pad, int farfield, cudaStream_t s, const double* ln_rhs = nullptr,
+                      double ln_scale = 0.0);
+// The transposed systems (adjoint), in place: kind 0 IDEL2LN, 2 IHELM.
+void k_solve_T(const DevGrid& g, const double* F, double2* y, int kind, int pad, cudaStream_t s);
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
                             int farfield, cudaStream_t s);
 // The AB2 update with VISC2's right-hand side for up to three fields (kernels.cu).

@@ -14,7 +14,10 @@
 //  kind 1  IDEL2:   m = 0 uses the 7-band row-shifted system (k = 0: row 0 is
 //                   the log-term boundary condition)
 //  kind 2  IHELM:   m = 0 solves (H XM) y = rhs on NN-1 rows, A = XM y
+#include "bulk.cuh"
 #include "mlegs_internal.h"
+
+#include <algorithm>
 
 namespace mlegs {
 
@@ -222,18 +225,32 @@ __global__ void solve_kernel(DevGrid g, double2* A, double* ln_out, int kind, do
 // Factor once, solve many.  For a fixed (kind, pad, alp) the system matrices
 // do not change from call to call, so their LU factors (the same unpivoted
 // elimination as solve_kernel, LUDCMPB of mod_bandmat.f90:65-155) are stored
-// once and every later solve is only the substitutions of LUBKSBB (320-401):
-//   F5 [row][5][system]  f2 = L(r, r-2), f1 = L(r, r-1), U(r, r), U(r, r+1), U(r, r+2)
-//                        for the 5-band systems;
-//   F7 [row][7][k]       f3, f2, f1, U(r, r .. r+3) for the 7-band m = 0 systems
-//                        of kinds 1 and 2.
-// The multipliers and pivots are the ones solve_kernel forms, and the
-// substitutions apply them in the same order.  The two kernels are compiled
-// separately (solve_kernel's elimination is unrolled in register windows), so
-// the compiler contracts different products into FMAs: the results agree to a
-// few units in the last place (about 2e-16 relative to the field, 1e-15 at
-// most, measured on B200), not bit for bit.
-__global__ void factor_kernel(DevGrid g, int kind, double alp, int pad, double* F5, double* F7) {
+// once and every later solve is only the substitutions of LUBKSBB (320-401).
+// The table holds blocks of 16 systems of one m (consecutive k), per row the
+// sub-diagonal multipliers f_d = L(r, r-d) and the scaled U row u_d =
+// U(r, r+d)/U(r, r), ri = 1/U(r, r) (formed here, off the substitution's
+// recurrence), the 16 systems side by side and the entries in pairs for 16-byte loads:
+//   5-band, HB = 2: L5 [block][row] {f2, f1}[16], U5 [block][row] {u2, u1}[16] ri[16],
+//     block = (m, k / 16);
+//   7-band m = 0 systems of kinds 1 and 2, HB = 3: L7 [k / 16][row] {f3, f2}[16] f1[16],
+//     U7 [k / 16][row] {u3, u2}[16] {u1, ri}[16];
+// so a run of rows is one contiguous piece, one bulk copy.
+struct FactorTable {
+    size_t u5, l7, u7, total;  // offsets (doubles); L5 starts at 0
+    int nkb, R;                // blocks per m, rows per block
+    __host__ __device__ explicit FactorTable(const DevGrid& g) {
+        nkb = (g.NXCHOPDIM + 15) / 16;
+        R = g.NRCHOPDIM;
+        const size_t b = (size_t)nkb * R;
+        u5 = g.NTCHOPDIM * b * 32;
+        l7 = u5 + g.NTCHOPDIM * b * 48;
+        u7 = l7 + b * 48;
+        total = u7 + b * 64;
+    }
+};
+
+__global__ void factor_kernel(DevGrid g, int kind, double alp, int pad, double* F) {
+    const FactorTable ft(g);
     const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nsys) return;
@@ -254,6 +271,10 @@ __global__ void factor_kernel(DevGrid g, int kind, double alp, int pad, double* 
     const bool wide = (m == 0 && kind != 0);
     const int lo = wide ? 3 : 2, up = wide ? 3 : 2;
     const int size = (m == 0 && kind == 2) ? nn - 1 : nn;
+    const size_t blk = wide ? (size_t)(k / 16) : (size_t)m * ft.nkb + k / 16;
+    double* L = F + (wide ? ft.l7 : 0) + blk * ft.R * (wide ? 48 : 32);
+    double* UU = F + (wide ? ft.u7 : ft.u5) + blk * ft.R * (wide ? 64 : 48);
+    const int sy = k % 16;
     double U[3][4] = {};
     for (int r = 0; r < size; ++r) {
         double w[MAXW];
@@ -273,441 +294,546 @@ __global__ void factor_kernel(DevGrid g, int kind, double alp, int pad, double* 
         const int wr = r % 3;
         U[wr][0] = w[3];
         for (int j = 1; j <= 3; ++j) U[wr][j] = (j <= up) ? w[3 + j] : 0.0;
+        const double ri = 1.0 / w[3];
+        double u[4];
+        for (int j = 1; j <= up; ++j) u[j] = (r + j < size) ? __dmul_rn(U[wr][j], ri) : 0.0;
+        double* l = L + (size_t)r * lo * 16;
+        double* o = UU + (size_t)r * (up + 1) * 16;
+        l[2 * sy] = f[lo];
+        l[2 * sy + 1] = f[lo - 1];
+        o[2 * sy] = u[up];
+        o[2 * sy + 1] = u[up - 1];
         if (wide) {
-            double* o = F7 + (size_t)r * 7 * g.NXCHOPDIM + k;
-            o[0] = f[3];
-            o[(size_t)1 * g.NXCHOPDIM] = f[2];
-            o[(size_t)2 * g.NXCHOPDIM] = f[1];
-            for (int j = 0; j < 4; ++j) o[(size_t)(3 + j) * g.NXCHOPDIM] = U[wr][j];
+            l[32 + sy] = f[1];
+            o[32 + 2 * sy] = u[1];
+            o[32 + 2 * sy + 1] = ri;
         } else {
-            double* o = F5 + (size_t)r * 5 * nsys + t;
-            o[0] = f[2];
-            o[(size_t)1 * nsys] = f[1];
-            for (int j = 0; j < 3; ++j) o[(size_t)(2 + j) * nsys] = U[wr][j];
+            o[32 + sy] = ri;
         }
     }
 }
 
-// One thread per (system, real or imaginary part).  Reads the right-hand side
-// from src, writes the solution to dst (rows >= the system size are zeroed),
-// then the per-kind tails of solve_kernel; farfield = 1 also applies the
-// CALCAT1 row-0 correction over n < NRCHOP + pad to the m = 0 columns.
-// One (system, real or imaginary part) u of the factored substitutions: the
-// body of solve_factored_kernel, also run by the grouped ensemble kernel.
-// WB: rows per load block of the 7-band systems (16 where registers allow)
-template <int WB>
-__device__ __forceinline__ void solve_factored_sys(const DevGrid& g, const double* __restrict__ F5,
-                                                   const double* __restrict__ F7, const double2* src, double2* dst,
-                                                   double* ln_out, int kind, int has_ln, double ln_in, int pad,
-                                                   int farfield, int u) {
+size_t solve_factor_doubles(const DevGrid& g) { return FactorTable(g).total; }
+
+// F: solve_factor_doubles(g) entries.
+void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F, cudaStream_t s) {
+    cudaMemsetAsync(F, 0, solve_factor_doubles(g) * sizeof(double), s);  // the blocks' unused columns
     const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    const int t = u >> 1, comp = u & 1;
-    if (t >= nsys) return;
-    const int k = t % g.NXCHOPDIM;
-    const int m = t / g.NXCHOPDIM;
-    int nn = g.NRCHOP + pad - m;
-    if (nn < 0) nn = 0;
-    const bool wide = (m == 0 && kind != 0);
-    int size = (m == 0 && kind == 2) ? nn - 1 : nn;
-    if (size < 0) size = 0;
-    const size_t cofs = (size_t)m * g.NRCHOPDIM * g.NXCHOPDIM + k;
-    const double* in = (const double*)(src + cofs) + comp;
-    double* col = (double*)(dst + cofs) + comp;
-    const size_t st = 2 * (size_t)g.NXCHOPDIM;
-    // IDEL2 (m = 0, k = 0): right-hand side shifted down one row, row 0 <- the LN condition (929-936)
-    const bool shift = (kind == 1 && m == 0 && k == 0);
-    auto rhs = [&](int r) -> double {
-        if (!shift) return in[(size_t)r * st];
-        if (r == 0) return comp ? 0.0 : (has_ln ? ln_in / g.norm0[0] : 0.0);
-        return in[(size_t)(r - 1) * st];
-    };
-    // out of place, the substitution reads the shifted rows directly; in place,
-    // they are shifted first (each row read before it is overwritten)
-    const bool direct = shift && (const void*)src != (const void*)dst;
-    if (shift && !direct) {
-        double prev = rhs(0);
-        for (int r = 0; r < size; ++r) {
-            const double cur = (r + 1 < size) ? rhs(r + 1) : 0.0;
-            col[(size_t)r * st] = prev;
-            prev = cur;
-        }
-        in = col;
-    }
-    constexpr int RBF = 16;
-    if (!wide) {
-        double y1 = 0.0, y2 = 0.0;
-        for (int r0 = 0; r0 < size; r0 += RBF) {
-            double rb[RBF], fa[RBF], fb[RBF];
-#pragma unroll
-            for (int q = 0; q < RBF; ++q) {
-                const int r = r0 + q;
-                const bool ok = r < size;
-                rb[q] = ok ? in[(size_t)r * st] : 0.0;
-                fa[q] = ok ? F5[(size_t)r * 5 * nsys + t] : 0.0;
-                fb[q] = ok ? F5[((size_t)r * 5 + 1) * nsys + t] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < RBF; ++q) {
-                if (r0 + q >= size) break;
-                const double y = __fma_rn(-fb[q], y1, __fma_rn(-fa[q], y2, rb[q]));
-                col[(size_t)(r0 + q) * st] = y;
-                y2 = y1;
-                y1 = y;
-            }
-        }
-        double x1 = 0.0, x2 = 0.0;
-        for (int r1 = size - 1; r1 >= 0; r1 -= RBF) {
-            double vb[RBF], u0[RBF], u1[RBF], u2[RBF];
-#pragma unroll
-            for (int q = 0; q < RBF; ++q) {
-                const int r = r1 - q;
-                const bool ok = r >= 0;
-                vb[q] = ok ? col[(size_t)r * st] : 0.0;
-                u0[q] = ok ? F5[((size_t)r * 5 + 2) * nsys + t] : 1.0;
-                u1[q] = ok ? F5[((size_t)r * 5 + 3) * nsys + t] : 0.0;
-                u2[q] = ok ? F5[((size_t)r * 5 + 4) * nsys + t] : 0.0;
-            }
-            // the diagonal's reciprocal and the scaled row are formed off the
-            // recurrence, which then costs one dependent FMA per row (a divide
-            // on the recurrence made the substitution latency-bound)
-#pragma unroll
-            for (int q = 0; q < RBF; ++q) {
-                const int r = r1 - q;
-                const double ri = 1.0 / u0[q];
-                vb[q] = __dmul_rn(vb[q], ri);
-                u1[q] = (r + 1 < size) ? __dmul_rn(u1[q], ri) : 0.0;
-                u2[q] = (r + 2 < size) ? __dmul_rn(u2[q], ri) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < RBF; ++q) {
-                const int r = r1 - q;
-                if (r < 0) break;
-                const double v = __fma_rn(-u1[q], x1, __fma_rn(-u2[q], x2, vb[q]));
-                col[(size_t)r * st] = v;
-                x2 = x1;
-                x1 = v;
-            }
-        }
-    } else {
-        const size_t NK = g.NXCHOPDIM;
-        constexpr int RBW = WB;
-        double y1 = 0.0, y2 = 0.0, y3 = 0.0;
-        for (int r0 = 0; r0 < size; r0 += RBW) {
-            double rb[RBW], f3[RBW], f2[RBW], f1[RBW];
-#pragma unroll
-            for (int q = 0; q < RBW; ++q) {
-                const int r = r0 + q;
-                const bool ok = r < size;
-                const double* f = F7 + (size_t)r * 7 * NK + k;
-                rb[q] = ok ? (direct ? rhs(r) : in[(size_t)r * st]) : 0.0;
-                f3[q] = ok ? f[0] : 0.0;
-                f2[q] = ok ? f[NK] : 0.0;
-                f1[q] = ok ? f[2 * NK] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < RBW; ++q) {
-                if (r0 + q >= size) break;
-                const double y = __fma_rn(-f1[q], y1, __fma_rn(-f2[q], y2, __fma_rn(-f3[q], y3, rb[q])));
-                col[(size_t)(r0 + q) * st] = y;
-                y3 = y2;
-                y2 = y1;
-                y1 = y;
-            }
-        }
-        double x1 = 0.0, x2 = 0.0, x3 = 0.0;
-        for (int r1 = size - 1; r1 >= 0; r1 -= RBW) {
-            double vb[RBW], u0[RBW], u1[RBW], u2[RBW], u3[RBW];
-#pragma unroll
-            for (int q = 0; q < RBW; ++q) {
-                const int r = r1 - q;
-                const bool ok = r >= 0;
-                const double* f = F7 + (size_t)(ok ? r : 0) * 7 * NK + k;
-                vb[q] = ok ? col[(size_t)r * st] : 0.0;
-                u0[q] = ok ? f[3 * NK] : 1.0;
-                u1[q] = ok ? f[4 * NK] : 0.0;
-                u2[q] = ok ? f[5 * NK] : 0.0;
-                u3[q] = ok ? f[6 * NK] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < RBW; ++q) {
-                const int r = r1 - q;
-                const double ri = 1.0 / u0[q];
-                vb[q] = __dmul_rn(vb[q], ri);
-                u1[q] = (r + 1 < size) ? __dmul_rn(u1[q], ri) : 0.0;
-                u2[q] = (r + 2 < size) ? __dmul_rn(u2[q], ri) : 0.0;
-                u3[q] = (r + 3 < size) ? __dmul_rn(u3[q], ri) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < RBW; ++q) {
-                const int r = r1 - q;
-                if (r < 0) break;
-                const double v = __fma_rn(-u1[q], x1, __fma_rn(-u2[q], x2, __fma_rn(-u3[q], x3, vb[q])));
-                col[(size_t)r * st] = v;
-                x3 = x2;
-                x2 = x1;
-                x1 = v;
-            }
-        }
-    }
-    for (int r = size; r < g.NRCHOPDIM; ++r) col[(size_t)r * st] = 0.0;
-    if (m == 0 && kind == 2 && nn > 0) {
-        // A(NN) = 0; A(:NN) = XM(:NN) y  (1310-1316)
-        const double* xm = g.xm;
-        double prev = 0.0;
-        for (int r = 0; r < nn; ++r) {
-            const double cur = col[(size_t)r * st];
-            const double nxt = (r + 1 < nn) ? col[(size_t)(r + 1) * st] : 0.0;
-            // explicit roundings here and below: every kernel that runs this
-            // body (single and grouped) gives the same bits
-            double v = cur;
-            if (r >= 1) v = __fma_rn(xm[(size_t)r * 2], prev, v);
-            if (r + 1 < nn) v = __fma_rn(xm[(size_t)r * 2 + 1], nxt, v);
-            col[(size_t)r * st] = v;
-            prev = cur;
-        }
-    }
-    if (m == 0 && k == 0 && size > 0) {
-        if (kind == 0) {
-            if (!comp) *ln_out = __dmul_rn(col[0], g.norm0[0]);
-            col[0] = 0.0;
-        } else if (kind == 1 && !comp && ln_out) {
-            *ln_out = has_ln ? __dmul_rn(col[0], g.norm0[0]) : 0.0;
-        }
-    }
-    if (farfield && m == 0) {
-        // a(n=0, m=0, k) -= sum_{n < NRCHOP+pad} AT1(n) a(n, 0, k) / AT1(0)
-        const int nr_sum = g.NRCHOP + pad;
-        double sum = 0.0;
-        for (int r = 0; r < nr_sum && r < g.NRCHOPDIM; ++r) sum = __fma_rn(g.at1[r], col[(size_t)r * st], sum);
-        col[0] = __dsub_rn(col[0], __ddiv_rn(sum, g.at1[0]));
-    }
-}
-
-void solve_factor_sizes(const DevGrid& g, size_t* f5, size_t* f7) {
-    *f5 = (size_t)g.NRCHOPDIM * 5 * g.NTCHOPDIM * g.NXCHOPDIM;
-    *f7 = (size_t)g.NRCHOPDIM * 7 * g.NXCHOPDIM;
-}
-
-void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F5, double* F7, cudaStream_t s) {
-    const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    factor_kernel<<<(nsys + 63) / 64, 64, 0, s>>>(g, kind, alp, pad, F5, F7);
+    factor_kernel<<<(nsys + 63) / 64, 64, 0, s>>>(g, kind, alp, pad, F);
     count_launch();
 }
 
-// LN slots a solve sets besides its own (thread 0 of the problem's first block).
-__device__ __forceinline__ void solve_ln_copies(const SolveItem& p) {
-    for (int j = 0; j < 2; ++j)
-        if (p.ln_dst[j]) *p.ln_dst[j] = *p.ln_src[j];
-}
+// The substitutions: a CTA takes a block of 16 systems.  Warp 0 runs them (lane =
+// system x real or imaginary part); warp 1 streams the factor rows through a
+// ring of SNST chunks of SCH rows in shared memory, ascending for the first
+// substitution and descending for the second, and the right-hand sides with
+// the first pass's chunks.  The column stays in shared memory until both warps
+// write the solution.
+//
+// What bounds it: a system is a serial chain of rows and its warp runs alone,
+// several cycles an instruction, so the launch lasts as long as the
+// instructions of the longest (m = 0) blocks.  Hence the second warp for the
+// copies, one bulk copy a chunk for the factors, the chunk's values in
+// registers before the recurrence (then one dependent FMA per row), and the
+// tables of the m = 0 tails (CALCAT1, XM) in shared memory.  IDEL2 and IDEL2LN at
+// 192x128x256 (139 MB each) take 31 us; 51 us with each thread reading its rows 16
+// at a time from global memory, 34 us with one warp doing both jobs.  A 58-row
+// solve at 64x32x32 takes 11.6 us, 17-19 us in the other forms (ncu, cold cache).
+// The blocks run m ascending: longest first.
+// XG: columns too long for shared memory (more than about 800 rows) stay in
+// global memory, read and written a chunk at a time.
+namespace {
+using namespace bulk;
 
-// blockIdx.y: the problem (fields with factors of one kind and pad: a step's
-// three viscous solves in one launch, each latency-bound alone).
-__global__ void __launch_bounds__(128) solve_factored_kernel(DevGrid g, const __grid_constant__ SolveBatch b, int kind,
-                                                             int has_ln, double ln_in, int pad, int farfield,
-                                                             int wpad) {
-    const SolveItem& p = b.p[blockIdx.y];
-    if (blockIdx.x == 0 && threadIdx.x == 0) solve_ln_copies(p);
-    // kinds 1 and 2: the 7-band m = 0 systems (u < 2 NXCHOPDIM) take whole
-    // warps, the 5-band ones start after wpad idle threads, so that no warp
-    // runs both substitutions one after the other
-    int u = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nw = 2 * g.NXCHOPDIM;
-    if (wpad) {
-        if (u >= nw && u < nw + wpad) return;
-        if (u >= nw) u -= wpad;
-    }
-    solve_factored_sys<16>(g, p.F5, p.F7, p.src, p.dst, p.ln_out, kind, has_ln, ln_in, pad, farfield, u);
-}
+constexpr int SCH = 8;   // rows per chunk
+constexpr int SNST = 5;  // chunks in the ring
+constexpr int SRING = SNST * SCH * 64;  // doubles
 
-// Small systems (NRCHOP + pad <= SMALL_R rows): one warp takes 16 systems
-// (lane = system x real/imaginary part), copies their factor rows and
-// right-hand sides into shared memory in one burst of cp.async copies, and
-// runs the substitutions and the tails of solve_factored_sys there, with the
-// same operations in the same order.  Blocks [0, nb0) hold the t_begin
-// 7-band m = 0 systems of kinds 1 and 2, the rest the 5-band ones, so no
-// warp mixes the two.  Shared memory per block: R x 144 doubles (factor rows
-// [r][7][16], values [r][16] complex), R = NRCHOP + pad.
-constexpr int SMALL_R = 72;
+struct SolveForm {
+    int kind, has_ln;
+    double ln_in;
+    int pad, farfield;
+};
+// A block's shared memory: the ring, the tables of the m = 0 tails (at1 [R],
+// xm [R][2]), the column Xs [R][16].
+struct SolveShared {
+    double* ring;
+    double* at1;
+    double* xm;
+    double2* Xs;
+    uint64_t* full;   // a chunk has arrived: 32 producer lanes and the bulk copy
+    uint64_t* empty;  // the consumer has read it
+    uint64_t* whole;  // the staged column of the transposed m = 0 system
+    int* stop;        // a wait ran out
+};
 
-__device__ __forceinline__ void cpa8(double* d, const double* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cpa16(double2* d, const double2* src) {
+__device__ __forceinline__ void cpa16(void* d, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src)
                  : "memory");
 }
-
-__global__ void __launch_bounds__(32) solve_small_kernel(DevGrid g, const __grid_constant__ SolveBatch b, int kind,
-                                                         int has_ln, double ln_in, int pad, int farfield,
-                                                         int t_begin, int nb0) {
-    extern __shared__ __align__(16) double sms[];
-    const SolveItem& p = b.p[blockIdx.y];
-    const double* __restrict__ F5 = p.F5;
-    const double* __restrict__ F7 = p.F7;
-    const double2* src = p.src;
-    double2* dst = p.dst;
-    double* ln_out = p.ln_out;
-    if (blockIdx.x == 0 && threadIdx.x == 0) solve_ln_copies(p);
-    const int R = g.NRCHOP + pad;
-    double* Fs = sms;                         // [R][7][16]
-    double2* Xs = (double2*)(sms + R * 112);  // [R][16]
-    const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    const int lane = threadIdx.x, sy = lane >> 1, comp = lane & 1;
-    const bool wide_blk = (int)blockIdx.x < nb0;
-    const int tb = wide_blk ? blockIdx.x * 16 : t_begin + (blockIdx.x - nb0) * 16;
-    const int tend = wide_blk ? t_begin : nsys;
-    const int nsb = min(16, tend - tb);
-    const size_t NK = g.NXCHOPDIM;
-    // the burst: factor rows, then the right-hand sides
-    if (wide_blk) {
-        for (int e = lane; e < R * 112; e += 32) {
-            const int r = e / 112, j = (e / 16) % 7, q = e % 16;
-            if (q < nsb) cpa8(Fs + e, F7 + ((size_t)r * 7 + j) * NK + tb + q);
-        }
-    } else {
-        for (int e = lane; e < R * 80; e += 32) {
-            const int r = e / 80, j = (e / 16) % 5, q = e % 16;
-            if (q < nsb) cpa8(Fs + (r * 7 + j) * 16 + q, F5 + ((size_t)r * 5 + j) * nsys + tb + q);
-        }
-    }
-    for (int e = lane; e < R * 16; e += 32) {
-        const int r = e / 16, q = e % 16;
-        if (q < nsb) {
-            const int tq = tb + q, mq = tq / g.NXCHOPDIM, kq = tq - mq * g.NXCHOPDIM;
-            cpa16(Xs + e, src + (size_t)mq * g.NRCHOPDIM * NK + (size_t)r * NK + kq);
-        }
-    }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-    if (sy >= nsb) return;
-    const int t = tb + sy, k = t % g.NXCHOPDIM, m = t / g.NXCHOPDIM;
-    int nn = g.NRCHOP + pad - m;
-    if (nn < 0) nn = 0;
-    const bool wide = wide_blk;
-    int size = (m == 0 && kind == 2) ? nn - 1 : nn;
-    if (size < 0) size = 0;
-    double* X = (double*)Xs + sy * 2 + comp;  // row r at X[r * 32]
-    auto F = [&](int r, int j) { return Fs[(r * 7 + j) * 16 + sy]; };
-    // IDEL2 (m = 0, k = 0): right-hand side shifted down one row, row 0 <- the LN condition
-    if (kind == 1 && m == 0 && k == 0) {
-        for (int r = size - 1; r >= 1; --r) X[r * 32] = X[(r - 1) * 32];
-        if (size > 0) X[0] = comp ? 0.0 : (has_ln ? ln_in / g.norm0[0] : 0.0);
-    }
-    if (!wide) {
-        double y1 = 0.0, y2 = 0.0;
-        for (int r = 0; r < size; ++r) {
-            const double y = __fma_rn(-F(r, 1), y1, __fma_rn(-F(r, 0), y2, X[r * 32]));
-            X[r * 32] = y;
-            y2 = y1;
-            y1 = y;
-        }
-        double x1 = 0.0, x2 = 0.0;
-        for (int r = size - 1; r >= 0; --r) {
-            const double ri = 1.0 / F(r, 2);
-            const double a1 = (r + 1 < size) ? __dmul_rn(F(r, 3), ri) : 0.0;
-            const double a2 = (r + 2 < size) ? __dmul_rn(F(r, 4), ri) : 0.0;
-            const double v = __fma_rn(-a1, x1, __fma_rn(-a2, x2, __dmul_rn(X[r * 32], ri)));
-            X[r * 32] = v;
-            x2 = x1;
-            x1 = v;
-        }
-    } else {
-        double y1 = 0.0, y2 = 0.0, y3 = 0.0;
-        for (int r = 0; r < size; ++r) {
-            const double y = __fma_rn(-F(r, 2), y1, __fma_rn(-F(r, 1), y2, __fma_rn(-F(r, 0), y3, X[r * 32])));
-            X[r * 32] = y;
-            y3 = y2;
-            y2 = y1;
-            y1 = y;
-        }
-        double x1 = 0.0, x2 = 0.0, x3 = 0.0;
-        for (int r = size - 1; r >= 0; --r) {
-            const double ri = 1.0 / F(r, 3);
-            const double a1 = (r + 1 < size) ? __dmul_rn(F(r, 4), ri) : 0.0;
-            const double a2 = (r + 2 < size) ? __dmul_rn(F(r, 5), ri) : 0.0;
-            const double a3 = (r + 3 < size) ? __dmul_rn(F(r, 6), ri) : 0.0;
-            const double v =
-                __fma_rn(-a1, x1, __fma_rn(-a2, x2, __fma_rn(-a3, x3, __dmul_rn(X[r * 32], ri))));
-            X[r * 32] = v;
-            x3 = x2;
-            x2 = x1;
-            x1 = v;
-        }
-    }
-    // the tails of solve_factored_sys, on the staged column
-    for (int r = size; r < R; ++r) X[r * 32] = 0.0;
-    if (m == 0 && kind == 2 && nn > 0) {
-        const double* xm = g.xm;
-        double prev = 0.0;
-        for (int r = 0; r < nn; ++r) {
-            const double cur = X[r * 32];
-            const double nxt = (r + 1 < nn) ? X[(r + 1) * 32] : 0.0;
-            double v = cur;
-            if (r >= 1) v = __fma_rn(xm[(size_t)r * 2], prev, v);
-            if (r + 1 < nn) v = __fma_rn(xm[(size_t)r * 2 + 1], nxt, v);
-            X[r * 32] = v;
-            prev = cur;
-        }
-    }
-    if (m == 0 && k == 0 && size > 0) {
-        if (kind == 0) {
-            if (!comp) *ln_out = __dmul_rn(X[0], g.norm0[0]);
-            X[0] = 0.0;
-        } else if (kind == 1 && !comp && ln_out) {
-            *ln_out = has_ln ? __dmul_rn(X[0], g.norm0[0]) : 0.0;
-        }
-    }
-    if (farfield && m == 0) {
-        double sum = 0.0;
-        for (int r = 0; r < R && r < g.NRCHOPDIM; ++r) sum = __fma_rn(g.at1[r], X[r * 32], sum);
-        X[0] = __dsub_rn(X[0], __ddiv_rn(sum, g.at1[0]));
-    }
-    double* col = (double*)(dst + (size_t)m * g.NRCHOPDIM * NK + k) + comp;
-    const size_t st = 2 * NK;
-    for (int r = 0; r < g.NRCHOPDIM; ++r) col[(size_t)r * st] = r < R ? X[r * 32] : 0.0;
+// arrival once this thread's cp.async copies so far have landed
+__device__ __forceinline__ void cpa_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sa_of(bar)) : "memory");
+}
+// A whole warp's wait; false (for all lanes) when it runs out or the other warp stopped.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, int phase, int* stop) {
+    return __all_sync(0xffffffffu, bar_wait(bar, (uint32_t)(phase & 1))) && !*(volatile int*)stop;
 }
 
-bool solve_small_ok(const DevGrid& g, int pad) { return g.NRCHOP + pad <= SMALL_R; }
-
-void k_solve_small(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad, int farfield,
-                   cudaStream_t s) {
-    const int nsys = g.NTCHOPDIM * g.NXCHOPDIM;
-    const int t_begin = kind == 0 ? 0 : g.NXCHOPDIM;
-    const int nb0 = (t_begin + 15) / 16, nb1 = (nsys - t_begin + 15) / 16;
-    const int R = g.NRCHOP + pad;
-    const size_t smem = (size_t)R * 144 * sizeof(double);
-    static size_t attr = 0;
-    if (smem > attr && smem > 48 * 1024) {
-        cudaFuncSetAttribute(solve_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = smem;
+// Chunk c of 2 nch: rows [lo, lo + rows), ascending in the first pass, descending in the second.
+__device__ __forceinline__ void solve_chunk(int c, int nch, int size, int& lo, int& rows) {
+    if (c < nch) {
+        lo = c * SCH;
+        rows = min(SCH, size - lo);
+    } else {
+        const int hi = size - (c - nch) * SCH;
+        lo = max(0, hi - SCH);
+        rows = hi - lo;
     }
-    solve_small_kernel<<<dim3(nb0 + nb1, b.n), 32, smem, s>>>(g, b, kind, has_ln, ln_in, pad, farfield, t_begin, nb0);
+}
+
+template <int HB, bool TR, bool XG>
+__device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, const double* FL, const double* FU,
+                               int size, int nn, const SolveShared& sh) {
+    constexpr int WL = HB * 16, WU = (HB + 1) * 16, WA = TR ? WU : WL, WB = TR ? WL : WU;
+    const int lane = threadIdx.x & 31;
+    const size_t NK = g.NXCHOPDIM;
+    const int nch = (size + SCH - 1) / SCH;
+    const int q = lane & 15, r0 = lane >> 4;
+    const bool staged = TR && HB == 3;
+    if (staged && !XG) {
+        if (q < nsb)
+            for (int r = r0; r < nn; r += 2) cpa16(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
+        cpa_arrive(sh.whole);
+    }
+    int c = 0;
+    bool ok = true;
+    for (; c < 2 * nch; ++c) {
+        const int st = c % SNST;
+        if (c >= SNST && !warp_wait(sh.empty + st, c / SNST - 1, sh.stop)) {
+            ok = false;
+            break;
+        }
+        int lo, rows;
+        solve_chunk(c, nch, size, lo, rows);
+        const bool up = c < nch;
+        const uint32_t fb = (uint32_t)(rows * (up ? WA : WB)) * 8u;
+        if (lane == 0) {
+            bar_expect_tx(sh.full + st, fb);
+            bulk_copy(sh.ring + st * (SCH * 64), ((up != TR) ? FL : FU) + (size_t)lo * (up ? WA : WB), fb, sh.full + st);
+        }
+        if (up && !XG && !staged && q < nsb) {
+#pragma unroll
+            for (int i = 0; i < SCH / 2; ++i) {
+                const int r = lo + r0 + 2 * i;
+                if (r < lo + rows) cpa16(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
+            }
+        }
+        cpa_arrive(sh.full + st);
+    }
+    if (!ok) {  // the copies in flight land before the CTA ends
+        if (lane == 0) {
+            *sh.stop = 1;
+            if (g.err) *g.err = 1;
+        }
+        for (int b = max(0, c - SNST); b < c; ++b) bar_wait(sh.full + b % SNST, (uint32_t)((b / SNST) & 1));
+    }
+}
+
+// HB: half-bandwidth; TR: the transposed system U^T z = y, L^T x = z (rows from
+// the system size on left as they are), else L y = b, U x = y with the tails.
+// Returns the rows to write, -1 when a wait ran out.
+template <int HB, bool TR, bool XG>
+__device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveForm& fo, int m, int k0, int nsb,
+                              int size, int nn, const SolveShared& sh) {
+    const int lane = threadIdx.x, sy = lane >> 1, comp = lane & 1, k = k0 + sy;
+    const size_t NK = g.NXCHOPDIM, st = 2 * NK, base = (size_t)m * g.NRCHOPDIM * NK + k0;
+    const bool live = sy < nsb;
+    const int kind = fo.kind;
+    const int nch = (size + SCH - 1) / SCH;
+    const double* sc = (const double*)(p.src + base + sy) + comp;
+    double* dc = (double*)(p.dst + base + sy) + comp;
+    double* X = (double*)sh.Xs + lane;
+    const bool c00 = m == 0 && k == 0;
+    constexpr int WL = HB * 16, WU = (HB + 1) * 16;  // doubles per row of L and U
+    // a row's factors from the ring: f[d] = L(r, r-d), or f[0] = 1/U(r, r), f[d] = u_d
+    auto row_l = [&](const double* row, double (&f)[HB + 1]) {
+        const double2 a = *(const double2*)(row + 2 * sy);
+        f[HB] = a.x;
+        f[HB - 1] = a.y;
+        if constexpr (HB == 3) f[1] = row[32 + sy];
+    };
+    auto row_u = [&](const double* row, double (&f)[HB + 1]) {
+        const double2 a = *(const double2*)(row + 2 * sy);
+        f[HB] = a.x;
+        f[HB - 1] = a.y;
+        if constexpr (HB == 3) {
+            const double2 b = *(const double2*)(row + 32 + 2 * sy);
+            f[1] = b.x;
+            f[0] = b.y;
+        } else {
+            f[0] = row[32 + sy];
+        }
+    };
+    auto xget = [&](int r) -> double { return XG ? (live ? dc[(size_t)r * st] : 0.0) : X[r * 32]; };
+    auto xput = [&](int r, double v) {
+        if (!XG) X[r * 32] = v;
+        else if (live) dc[(size_t)r * st] = v;
+    };
+    auto give_up = [&] {
+        if (lane == 0) {
+            *sh.stop = 1;
+            if (g.err) *g.err = 1;
+        }
+        return -1;
+    };
+    // column <- A column for a tri-diagonal A of unit diagonal over rows < nn (XM and XM^T)
+    auto xm_pass = [&](bool transposed) {
+        double prev = 0.0, cur = nn > 0 ? xget(0) : 0.0;
+        for (int r0 = 0; r0 < nn; r0 += SCH) {
+            double nx[SCH], lo[SCH], hi[SCH];
+#pragma unroll
+            for (int q = 0; q < SCH; ++q) {
+                const int r = r0 + q, rl = transposed ? r - 1 : r, rh = transposed ? r + 1 : r;
+                const bool a = r >= 1 && r < nn, b = r + 1 < nn;
+                nx[q] = b ? xget(r + 1) : 0.0;
+                lo[q] = a ? sh.xm[2 * rl + (transposed ? 1 : 0)] : 0.0;
+                hi[q] = b ? sh.xm[2 * rh + (transposed ? 0 : 1)] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < SCH; ++q) {
+                const int r = r0 + q;
+                if (r >= nn) break;
+                // explicit roundings: every launch form gives the same bits
+                double v = transposed ? __fma_rn(lo[q], prev, __fma_rn(hi[q], nx[q], cur))
+                                      : __fma_rn(hi[q], nx[q], __fma_rn(lo[q], prev, cur));
+                xput(r, v);
+                prev = cur;
+                cur = nx[q];
+            }
+        }
+    };
+    // the transposed IHELM system at m = 0 takes w = XM^T y, which couples
+    // neighbouring rows: the column is staged (nn rows) before the passes
+    constexpr bool staged = TR && HB == 3;
+    if constexpr (staged) {
+        if (!XG && !warp_wait(sh.whole, 0, sh.stop)) return give_up();
+        xm_pass(true);
+    }
+    // IHELM of a right-hand side with a log term (mod_legops.f90:1244-1255)
+    double lnv = 0.0;
+    const bool logfix = !TR && p.ln_rhs && c00 && comp == 0;
+    if (logfix) lnv = *p.ln_rhs * p.ln_scale;
+    // IDEL2 (m = 0, k = 0): right-hand side shifted down one row, row 0 <- the LN condition (929-936)
+    const bool shift = !TR && HB == 3 && kind == 1 && c00;
+    double carry = shift && !comp && fo.has_ln ? fo.ln_in / g.norm0[0] : 0.0;
+    // recurrence state: v1, v2, v3 the last values; in the transposed passes the
+    // factors of the last rows too (column entries of U, of L)
+    double v1 = 0.0, v2 = 0.0, v3 = 0.0, a1 = 0.0, a2 = 0.0, a2p = 0.0, a3 = 0.0, a3p = 0.0, a3q = 0.0;
+    for (int c = 0; c < nch; ++c) {
+        if (!warp_wait(sh.full + c % SNST, c / SNST, sh.stop)) return give_up();
+        const double* S = sh.ring + (c % SNST) * (SCH * 64);
+        const int lo = c * SCH, rows = min(SCH, size - lo);
+        double rb[SCH], f[SCH][HB + 1];
+#pragma unroll
+        for (int q = 0; q < SCH; ++q) {  // rows past the end read stale values that are not used
+            rb[q] = XG && !staged ? (live && q < rows ? sc[(size_t)(lo + q) * st] : 0.0)
+                                  : (XG ? (q < rows ? xget(lo + q) : 0.0) : X[(lo + q) * 32]);
+            if constexpr (TR) row_u(S + q * WU, f[q]);
+            else row_l(S + q * WL, f[q]);
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(sh.empty + c % SNST);
+        if (logfix && c == 0) {
+            const double cf[3] = {4.0 / 3, -2.0, 2.0 / 3};
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                if (q < rows) rb[q] -= lnv * (cf[q] / g.ELL2) / g.norm0[q];
+        }
+        if (shift) {
+            const double last = rb[SCH - 1];
+#pragma unroll
+            for (int q = SCH - 1; q >= 1; --q) rb[q] = rb[q - 1];
+            rb[0] = carry;
+            carry = last;
+        }
+#pragma unroll
+        for (int q = 0; q < SCH; ++q) {
+            if (q >= rows) break;
+            double v = rb[q];
+            if constexpr (!TR) {
+                if constexpr (HB == 3) v = __fma_rn(-f[q][3], v3, v);
+                v = __fma_rn(-f[q][1], v1, __fma_rn(-f[q][2], v2, v));
+                xput(lo + q, v);
+            } else {
+                // w(r) = y(r) - u1(r-1) w(r-1) - u2(r-2) w(r-2) - ..., z(r) = w(r) / U(r, r)
+                if constexpr (HB == 3) v = __fma_rn(-a3q, v3, v);
+                v = __fma_rn(-a1, v1, __fma_rn(-a2p, v2, v));
+                xput(lo + q, __dmul_rn(v, f[q][0]));
+                a3q = a3p;
+                a3p = a3;
+                if constexpr (HB == 3) a3 = f[q][3];
+                a2p = a2;
+                a2 = f[q][2];
+                a1 = f[q][1];
+            }
+            v3 = v2;
+            v2 = v1;
+            v1 = v;
+        }
+    }
+    v1 = v2 = v3 = a1 = a2 = a2p = a3 = a3p = a3q = 0.0;
+    for (int c = nch; c < 2 * nch; ++c) {
+        if (!warp_wait(sh.full + c % SNST, c / SNST, sh.stop)) return give_up();
+        int lo, rows;
+        solve_chunk(c, nch, size, lo, rows);
+        const int hi = lo + rows - 1;
+        const double* S = sh.ring + (c % SNST) * (SCH * 64);
+        double vb[SCH], f[SCH][HB + 1];
+#pragma unroll
+        for (int q = 0; q < SCH; ++q) {  // rows past the end repeat row lo and are not used
+            const int r = max(lo, hi - q);
+            vb[q] = xget(r);
+            if constexpr (TR) row_l(S + (r - lo) * WL, f[q]);
+            else row_u(S + (r - lo) * WU, f[q]);
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(sh.empty + c % SNST);
+        if constexpr (!TR) {
+#pragma unroll
+            for (int q = 0; q < SCH; ++q) vb[q] = __dmul_rn(vb[q], f[q][0]);
+        }
+#pragma unroll
+        for (int q = 0; q < SCH; ++q) {
+            if (q >= rows) break;
+            double v = vb[q];
+            if constexpr (!TR) {
+                if constexpr (HB == 3) v = __fma_rn(-f[q][3], v3, v);
+                v = __fma_rn(-f[q][1], v1, __fma_rn(-f[q][2], v2, v));
+            } else {
+                // x(r) = z(r) - L(r+1, r) x(r+1) - L(r+2, r) x(r+2) - ...
+                if constexpr (HB == 3) v = __fma_rn(-a3q, v3, v);
+                v = __fma_rn(-a1, v1, __fma_rn(-a2p, v2, v));
+                a3q = a3p;
+                a3p = a3;
+                if constexpr (HB == 3) a3 = f[q][3];
+                a2p = a2;
+                a2 = f[q][2];
+                a1 = f[q][1];
+            }
+            xput(hi - q, v);
+            v3 = v2;
+            v2 = v1;
+            v1 = v;
+        }
+    }
+    if constexpr (TR) {
+        if (HB == 3 && nn > 0) {  // row NN - 1 zeroed
+            xput(size, 0.0);
+            return nn;
+        }
+        return size;
+    } else {
+        int rows_out = size;
+        if (HB == 3 && kind == 2 && nn > 0) {
+            // A(NN) = 0; A(:NN) = XM(:NN) y  (mod_legops.f90:1310-1316)
+            xput(nn - 1, 0.0);
+            rows_out = nn;
+            xm_pass(false);
+        }
+        if (c00 && size > 0) {
+            if (kind == 0) {
+                if (!comp) *p.ln_out = __dmul_rn(xget(0), g.norm0[0]);
+                xput(0, 0.0);
+            } else if (kind == 1 && !comp && p.ln_out) {
+                *p.ln_out = fo.has_ln ? __dmul_rn(xget(0), g.norm0[0]) : 0.0;
+            }
+        }
+        if (logfix && p.ln_out) *p.ln_out = lnv;
+        if (fo.farfield && m == 0 && size > 0) {
+            // a(n=0, m=0, k) -= sum_{n < NRCHOP+pad} AT1(n) a(n, 0, k) / AT1(0); the rows
+            // past the system are zero, four partial sums break the chain
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int r0 = 0; r0 < size; r0 += SCH) {
+#pragma unroll
+                for (int q = 0; q < SCH; ++q)
+                    if (r0 + q < size) s[q & 3] = __fma_rn(sh.at1[r0 + q], xget(r0 + q), s[q & 3]);
+            }
+            const double sum = __dadd_rn(__dadd_rn(s[0], s[1]), __dadd_rn(s[2], s[3]));
+            xput(0, __dsub_rn(xget(0), __ddiv_rn(sum, sh.at1[0])));
+        }
+        return rows_out;
+    }
+}
+
+template <int HB, bool TR, bool XG>
+__device__ __forceinline__ void band_solve(const DevGrid& g, const SolveItem& p, const SolveForm& fo, const double* FL,
+                                           const double* FU, int m, int k0, const SolveShared& sh) {
+    __shared__ int rows_sh;
+    const size_t NK = g.NXCHOPDIM, base = (size_t)m * g.NRCHOPDIM * NK + k0;
+    const int nsb = min(16, g.NXCHOPDIM - k0);
+    const int nn = max(0, g.NRCHOP + fo.pad - m);
+    const int size = max(0, (m == 0 && fo.kind == 2) ? nn - 1 : nn);
+    if (threadIdx.x >= 32) {
+        solve_producer<HB, TR, XG>(g, p.src + base, nsb, FL, FU, size, nn, sh);
+    } else {
+        const int rows = solve_consumer<HB, TR, XG>(g, p, fo, m, k0, nsb, size, nn, sh);
+        if (threadIdx.x == 0) rows_sh = rows;
+    }
+    __syncthreads();
+    const int rows_out = rows_sh;
+    if (rows_out < 0) return;
+    const int end = TR ? rows_out : g.NRCHOPDIM, q = threadIdx.x & 15;
+    double2* dst = p.dst + base + q;
+    if (q >= nsb) return;
+#pragma unroll 4
+    for (int r = (XG ? rows_out : 0) + (int)(threadIdx.x >> 4); r < end; r += 4)
+        dst[(size_t)r * NK] = !XG && r < rows_out ? sh.Xs[r * 16 + q] : make_double2(0.0, 0.0);
+}
+
+// doubles of a block's shared memory for columns of `rows` rows (at least SCH, whole chunks)
+__host__ __device__ inline size_t solve_doubles(int rows, bool xg) {
+    const int r = (rows + SCH - 1) / SCH * SCH;
+    return SRING + (size_t)(r + 2 * r) + (xg ? 0 : (size_t)r * 32);
+}
+
+template <bool TR, bool XG>
+__device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p, const SolveForm& fo, int b) {
+    extern __shared__ __align__(128) double sms[];
+    __shared__ uint64_t bars[2 * SNST + 1];
+    __shared__ int stop;
+    const FactorTable ft(g);
+    const int m = b / ft.nkb, kb = b - m * ft.nkb;
+    const int R = (max(g.NRCHOP + fo.pad, 0) + 1 + SCH - 1) / SCH * SCH;
+    SolveShared sh;
+    sh.ring = sms;
+    sh.at1 = sms + SRING;
+    sh.xm = sh.at1 + R;
+    sh.Xs = (double2*)(sh.xm + 2 * R);
+    sh.full = bars;
+    sh.empty = bars + SNST;
+    sh.whole = bars + 2 * SNST;
+    sh.stop = &stop;
+    if (threadIdx.x == 0) {
+        stop = 0;
+        for (int q = 0; q < SNST; ++q) {
+            bar_init(sh.full + q, 33);
+            bar_init(sh.empty + q, 1);
+        }
+        bar_init(sh.whole, 32);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (b == 0)
+            for (int j = 0; j < 2; ++j)
+                if (p.ln_dst[j]) *p.ln_dst[j] = *p.ln_src[j];
+    }
+    if (m == 0) {  // the tables of the m = 0 tails
+        const int nr = min(R, g.NRCHOPDIM);
+        if (fo.farfield)
+            for (int r = threadIdx.x; r < nr; r += 64) sh.at1[r] = g.at1[r];
+        if (fo.kind == 2)
+            for (int r = threadIdx.x; r < 2 * nr; r += 64) sh.xm[r] = g.xm[r];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    const bool wide = m == 0 && (TR ? fo.kind == 2 : fo.kind != 0);
+    if (wide) {
+        const double* FL = p.F + ft.l7 + (size_t)kb * ft.R * 48;
+        const double* FU = p.F + ft.u7 + (size_t)kb * ft.R * 64;
+        band_solve<3, TR, XG>(g, p, fo, FL, FU, m, kb * 16, sh);
+    } else {
+        const size_t blk = (size_t)m * ft.nkb + kb;
+        band_solve<2, TR, XG>(g, p, fo, p.F + blk * ft.R * 32, p.F + ft.u5 + blk * ft.R * 48, m, kb * 16, sh);
+    }
+}
+
+// blockIdx.y: the problem (a step's three viscous solves go in one launch)
+template <bool TR, bool XG>
+__global__ void __launch_bounds__(64) solve_factored_kernel(DevGrid g, const __grid_constant__ SolveBatch b,
+                                                            SolveForm fo) {
+    solve_block<TR, XG>(g, b.p[blockIdx.y], fo, blockIdx.x);
+}
+
+// Grouped form over the instances of an ensemble: a block's problem by binary
+// search over `first`.
+__global__ void __launch_bounds__(64) grouped_solve_kernel(const GroupSolve* __restrict__ pr,
+                                                           const int* __restrict__ first, int np) {
+    const int b = blockIdx.x;
+    int lo = 0, hi = np - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (first[mid] <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    const GroupSolve& P = pr[lo];
+    solve_block<false, false>(P.g, P.it, SolveForm{P.kind, P.has_ln, P.ln_in, P.pad, P.farfield}, b - P.first);
+}
+
+constexpr size_t SOLVE_SMEM_MAX = 220 * 1024;
+// g's columns at `pad` with one row to spare (IHELM's row NN at m = 0)
+size_t solve_smem(const DevGrid& g, int pad, bool xg) {
+    return solve_doubles(std::max(g.NRCHOP + pad, 0) + 1, xg) * sizeof(double);
+}
+
+template <class K>
+void allow_smem(K kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_SMEM_MAX);
+}
+
+template <bool TR>
+void launch_solve(const DevGrid& g, const SolveBatch& b, const SolveForm& fo, cudaStream_t s) {
+    static const bool attr = [] {
+        allow_smem(solve_factored_kernel<TR, false>);
+        allow_smem(solve_factored_kernel<TR, true>);
+        return true;
+    }();
+    (void)attr;
+    const dim3 grid(FactorTable(g).nkb * g.NTCHOPDIM, b.n);
+    const size_t smem = solve_smem(g, fo.pad, false);
+    if (smem <= SOLVE_SMEM_MAX) solve_factored_kernel<TR, false><<<grid, 64, smem, s>>>(g, b, fo);
+    else solve_factored_kernel<TR, true><<<grid, 64, solve_smem(g, fo.pad, true), s>>>(g, b, fo);
     count_launch();
 }
+}  // namespace
 
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
                             int farfield, cudaStream_t s) {
-    if (solve_small_ok(g, pad)) {  // the whole system fits in shared memory
-        k_solve_small(g, b, kind, has_ln, ln_in, pad, farfield, s);
-        return;
-    }
-    const int wpad = kind == 0 ? 0 : (32 - (2 * g.NXCHOPDIM) % 32) % 32;
-    const int n = 2 * g.NTCHOPDIM * g.NXCHOPDIM + wpad;
-    solve_factored_kernel<<<dim3((n + 127) / 128, b.n), 128, 0, s>>>(g, b, kind, has_ln, ln_in, pad, farfield, wpad);
-    count_launch();
+    launch_solve<false>(g, b, SolveForm{kind, has_ln, ln_in, pad, farfield}, s);
 }
 
-void k_solve_factored(const DevGrid& g, const double* F5, const double* F7, const double2* src, double2* dst,
-                      double* ln_out, int kind, int has_ln, double ln_in, int pad, int farfield, cudaStream_t s) {
+void k_solve_factored(const DevGrid& g, const double* F, const double2* src, double2* dst, double* ln_out, int kind,
+                      int has_ln, double ln_in, int pad, int farfield, cudaStream_t s, const double* ln_rhs,
+                      double ln_scale) {
     SolveBatch b{};
     b.n = 1;
-    b.p[0].F5 = F5;
-    b.p[0].F7 = F7;
+    b.p[0].F = F;
     b.p[0].src = src;
     b.p[0].dst = dst;
     b.p[0].ln_out = ln_out;
+    b.p[0].ln_rhs = ln_rhs;
+    b.p[0].ln_scale = ln_scale;
     k_solve_factored_batch(g, b, kind, has_ln, ln_in, pad, farfield, s);
+}
+
+void k_solve_T(const DevGrid& g, const double* F, double2* y, int kind, int pad, cudaStream_t s) {
+    SolveBatch b{};
+    b.n = 1;
+    b.p[0].F = F;
+    b.p[0].src = y;
+    b.p[0].dst = y;
+    launch_solve<true>(g, b, SolveForm{kind, 0, 0.0, pad, 0}, s);
+}
+
+int group_solve_blocks(const GroupSolve& p) { return FactorTable(p.g).nkb * p.g.NTCHOPDIM; }
+size_t group_solve_smem(const GroupSolve& p) { return solve_smem(p.g, p.pad, false); }
+
+void k_grouped_solve(const GroupSolve* d, const int* first, int np, int total_blocks, size_t smem, cudaStream_t s) {
+    static const bool attr = [] {
+        allow_smem(grouped_solve_kernel);
+        return true;
+    }();
+    (void)attr;
+    grouped_solve_kernel<<<total_blocks, 64, smem, s>>>(d, first, np);
+    count_launch();
 }
 
 void k_solve_del2(const DevGrid& g, double2* a, double* ln_out, int kind, double alp, int has_ln, double ln_in,
@@ -855,37 +981,6 @@ void k_ihelmp(const DevGrid& g, int P, const double* dq, int rows, double2* a, c
         case 12: ihelmp_kernel<6><<<nb, bs, 0, s>>>(g, dq, rows, a, ln, alp, nu, scratch, pad); break;
         default: ihelmp_kernel<7><<<nb, bs, 0, s>>>(g, dq, rows, a, ln, alp, nu, scratch, pad); break;
     }
-    count_launch();
-}
-
-// Grouped factored substitutions over the instances of an ensemble: each
-// block belongs to one problem (found by binary search over `first`), 64
-// systems per block.
-__global__ void __launch_bounds__(128) grouped_solve_kernel(const GroupSolve* __restrict__ pr,
-                                                            const int* __restrict__ first, int np) {
-    const int b = blockIdx.x;
-    int lo = 0, hi = np - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (first[mid] <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    const GroupSolve P = pr[lo];
-    // the 7-band m = 0 systems in whole warps, as in solve_factored_kernel
-    int u = (b - P.first) * 128 + threadIdx.x;
-    const int nw = 2 * P.g.NXCHOPDIM, wpad = P.kind == 0 ? 0 : (32 - nw % 32) % 32;
-    if (u >= nw && u < nw + wpad) return;
-    if (u >= nw) u -= wpad;
-    solve_factored_sys<8>(P.g, P.F5, P.F7, P.src, P.dst, P.ln_out, P.kind, P.has_ln, P.ln_in, P.pad, P.farfield, u);
-}
-
-int group_solve_blocks(const GroupSolve& p) {
-    const int nw = 2 * p.g.NXCHOPDIM, wpad = p.kind == 0 ? 0 : (32 - nw % 32) % 32;
-    return (2 * p.g.NTCHOPDIM * p.g.NXCHOPDIM + wpad + 127) / 128;
-}
-
-void k_grouped_solve(const GroupSolve* d, const int* first, int np, int total_blocks, cudaStream_t s) {
-    grouped_solve_kernel<<<total_blocks, 128, 0, s>>>(d, first, np);
     count_launch();
 }
 
