@@ -1685,36 +1685,48 @@ int mlegs_chopdo(mlegs_ctx* ctx, mlegs_field* f, int pad) {
     });
 }
 
-// In-place transforms on user fields swap with the context's scratch buffer
-// and then copy back so that the handle keeps its own buffer.
-static void user_inplace(mlegs_ctx* ctx, Field* f, const std::function<void(Field*)>& fn);
+// In-place transforms of a user field, which keeps its own buffer (captured
+// steps hold its address): two stages go through a scratch buffer and back,
+// three through two of them; a single stage is copied back.  (Copying in and out
+// around the chain cost 200 of the 742 us of a 256^3 TOFP + TOFF.)
+enum Stage { RTRAN_P, RTRAN_M, VERFFT_P, VERFFT_M, HORFFT_P, HORFFT_M };
+static void user_transform(mlegs_ctx* ctx, Field* f, std::initializer_list<Stage> stages, int pad = 0);
 
 int mlegs_rtran(mlegs_ctx* ctx, mlegs_field* f, int is, int pad) {
     return guard(ctx, [&] {
         check_pad(ctx, pad);
         if (is != 1 && is != -1) throw ApiError(MLEGS_ERR_ARG, "RTRAN: IS must be +1 or -1");
-        user_inplace(ctx, F(f), [&](Field* x) { ctx->rtran(x, is, pad); });
+        user_transform(ctx, F(f), {is == 1 ? RTRAN_P : RTRAN_M}, pad);
     });
 }
 int mlegs_horfft(mlegs_ctx* ctx, mlegs_field* f, int is) {
-    return guard(ctx, [&] { user_inplace(ctx, F(f), [&](Field* x) { ctx->horfft(x, is); }); });
+    return guard(ctx, [&] { user_transform(ctx, F(f), {is == -1 ? HORFFT_M : HORFFT_P}); });
 }
 int mlegs_verfft(mlegs_ctx* ctx, mlegs_field* f, int is) {
-    return guard(ctx, [&] { user_inplace(ctx, F(f), [&](Field* x) { ctx->verfft(x, is); }); });
+    return guard(ctx, [&] { user_transform(ctx, F(f), {is == -1 ? VERFFT_M : VERFFT_P}); });
 }
 int mlegs_plnfft(mlegs_ctx* ctx, mlegs_field* f, int is) {
-    return guard(ctx, [&] { user_inplace(ctx, F(f), [&](Field* x) { ctx->plnfft(x, is); }); });
+    return guard(ctx, [&] {
+        if (is == -1) user_transform(ctx, F(f), {HORFFT_M, VERFFT_M});
+        else user_transform(ctx, F(f), {VERFFT_P, HORFFT_P});
+    });
 }
 int mlegs_toff(mlegs_ctx* ctx, mlegs_field* f, int pad) {
     return guard(ctx, [&] {
         check_pad(ctx, pad);
-        user_inplace(ctx, F(f), [&](Field* x) { ctx->toff(x, pad); });
+        Field* x = F(f);
+        if (x->space == MLEGS_PPP) user_transform(ctx, x, {HORFFT_M, VERFFT_M, RTRAN_M}, pad);
+        else if (x->space == MLEGS_PFP) user_transform(ctx, x, {VERFFT_M, RTRAN_M}, pad);
+        else if (x->space == MLEGS_PFF) user_transform(ctx, x, {RTRAN_M}, pad);
     });
 }
 int mlegs_tofp(mlegs_ctx* ctx, mlegs_field* f, int pad) {
     return guard(ctx, [&] {
         check_pad(ctx, pad);
-        user_inplace(ctx, F(f), [&](Field* x) { ctx->tofp(x, pad); });
+        Field* x = F(f);
+        if (x->space == MLEGS_FFF) user_transform(ctx, x, {RTRAN_P, VERFFT_P, HORFFT_P}, pad);
+        else if (x->space == MLEGS_PFF) user_transform(ctx, x, {VERFFT_P, HORFFT_P}, pad);
+        else if (x->space == MLEGS_PFP) user_transform(ctx, x, {HORFFT_P}, pad);
     });
 }
 
@@ -1796,6 +1808,29 @@ int mlegs_project(mlegs_ctx* ctx, mlegs_field* rur, mlegs_field* rup, mlegs_fiel
     return guard(ctx, [&] {
         if (ln_mode < 0 || ln_mode > 2) throw ApiError(MLEGS_ERR_ARG, "PROJECT: bad ln_mode");
         Field *a = F(rur), *b2 = F(rup), *c = F(uz);
+        Field* const in[3] = {a, b2, c};
+        bool alias = a == b2 || a == c || b2 == c;
+        for (Field* q : in) alias = alias || q == F(psi) || q == F(chi);
+        if (!alias && a->space == b2->space && b2->space == c->space &&
+            (a->space == MLEGS_PPP || a->space == MLEGS_PFF)) {
+            // PLNFFT(-1) through temporaries into the fields' own buffers; PFF fields as they are
+            if (a->space == MLEGS_PPP) {
+                VerBatch h{}, v{};
+                h.n = v.n = 3;
+                Field* t[3] = {ctx->tmp(), ctx->tmp(), ctx->tmp()};
+                for (int q = 0; q < 3; ++q) {
+                    h.src[q] = v.dst[q] = in[q]->data;
+                    h.dst[q] = t[q]->data;
+                    v.src[q] = t[q]->data;
+                    in[q]->space = MLEGS_PFF;
+                }
+                k_horfft_batch(ctx->g, ctx->fft, h, -1, ctx->s);
+                ctx->verfft_batch(v, -1, ctx->s);
+                for (Field* q : t) ctx->rel(q);
+            }
+            ctx->project(a, b2, c, F(psi), F(chi), ln_mode, ln);
+            return;
+        }
         // work on temporaries so the user fields keep their buffers
         Field *ta = ctx->tmp(), *tb = ctx->tmp(), *tc = ctx->tmp();
         ctx->copy0(ta, a, 0);
@@ -2294,16 +2329,50 @@ void* mlegs_stream(mlegs_ctx* ctx) { return ctx ? (void*)ctx->s : nullptr; }
 
 }  // extern "C"
 
-static void user_inplace(mlegs_ctx* ctx, Field* f, const std::function<void(Field*)>& fn) {
+static void user_transform(mlegs_ctx* ctx, Field* f, std::initializer_list<Stage> stages, int pad) {
+    static const int from[] = {MLEGS_FFF, MLEGS_PFF, MLEGS_PFF, MLEGS_PFP, MLEGS_PFP, MLEGS_PPP};
+    static const int to[] = {MLEGS_PFF, MLEGS_FFF, MLEGS_PFP, MLEGS_PFF, MLEGS_PPP, MLEGS_PFP};
+    static const char* const who[] = {"RTRAN", "RTRAN", "VERFFT", "VERFFT", "HORFFT", "HORFFT"};
+    const int n = (int)stages.size();
+    ctx->require(f, from[*stages.begin()], who[*stages.begin()]);
     Field* t = ctx->tmp(f->space);
-    ctx->mark();
-    k_copy(t->data, f->data, ctx->d.elems(f->space), ctx->s);
-    cudaMemcpyAsync(t->ln, f->ln, sizeof(double), cudaMemcpyDeviceToDevice, ctx->s);
-    t->space = f->space;
-    fn(t);
-    k_copy(f->data, t->data, ctx->d.elems(t->space), ctx->s);
-    cudaMemcpyAsync(f->ln, t->ln, sizeof(double), cudaMemcpyDeviceToDevice, ctx->s);
-    f->space = t->space;
+    // buffer of the result of stage i: the last one is the field's own
+    double2* const mid[2] = {t->data, ctx->scratch};
+    const double2* src = f->data;
+    int i = 0;
+    bool zero_ln = false;  // RTRAN zeroes LN, in both directions
+    for (Stage st : stages) {
+        double2* dst = (i == n - 1 && n > 1) ? f->data : mid[i];
+        VerBatch v{};
+        v.n = 1;
+        v.src[0] = src;
+        v.dst[0] = dst;
+        switch (st) {
+            case RTRAN_P: {
+                B2PBatch b{};
+                b.n = 1;
+                b.in[0] = src;
+                b.out[0] = dst;
+                b.ln[0] = f->ln;
+                b.pad[0] = pad;
+                ctx->rtran_batch(b, ctx->s);
+                zero_ln = true;
+                break;
+            }
+            case RTRAN_M:
+                ctx->fold(0, ctx->pf, ctx->d.NRCHOPDIM + 1, src, dst, 0 | 2, 0, 0, pad);
+                zero_ln = true;
+                break;
+            case VERFFT_P: ctx->verfft_batch(v, +1, ctx->s); break;
+            case VERFFT_M: ctx->verfft_batch(v, -1, ctx->s); break;
+            case HORFFT_P: k_horfft_batch(ctx->g, ctx->fft, v, +1, ctx->s); break;
+            case HORFFT_M: k_horfft_batch(ctx->g, ctx->fft, v, -1, ctx->s); break;
+        }
+        src = dst;
+        f->space = to[st];
+        ++i;
+    }
+    if (n == 1) k_copy(f->data, src, ctx->d.elems(f->space), ctx->s);
+    if (zero_ln) ctx->ln_zero(f);
     ctx->rel(t);
-    ctx->restore();
 }

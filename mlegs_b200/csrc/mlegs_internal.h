@@ -266,6 +266,8 @@ struct VerBatch {
     int n;
 };
 bool k_verfft4_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s);
+// HORFFT of several fields (zln is not read).
+void k_horfft_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s);
 
 // Spectral operators on FFF.
 void k_delsqh(const DevGrid& g, const double2* a, const double* ln_a, double2* b, int pad, cudaStream_t s);

@@ -700,9 +700,8 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
 //   dir +1: PFP -> PPP (samples written from their slot positions),
 //   dir -1: PPP -> PFP (the row copied straight to its slot positions).
 template <int N1, int N2>
-__global__ void __launch_bounds__(256) horfft5_kernel(DevGrid g, const double2* __restrict__ src,
-                                                      double2* __restrict__ dst, const double2* tw_g,
-                                                      const double2* twh_g, int dir) {
+__global__ void __launch_bounds__(256) horfft5_kernel(DevGrid g, const __grid_constant__ VerBatch f,
+                                                      const double2* tw_g, const double2* twh_g, int dir) {
     constexpr int N = N1 * N2, G = 32 / N2;
     extern __shared__ double2 sm[];
     double2* tw = sm;
@@ -716,16 +715,17 @@ __global__ void __launch_bounds__(256) horfft5_kernel(DevGrid g, const double2* 
     const int gid = lane / N2, t = lane % N2;
     double2* L0 = twh + (N + 1) + (size_t)(warp * G + gid) * 2 * N;
     const int md = g.NTCHOPDIM, mlim = md < g.NTCHOP ? md : g.NTCHOP;
-    const int nlines = g.NR * g.NX;
+    const int flines = g.NR * g.NX, nlines = f.n * flines;  // the fields' lines one after another
     const int stride = gridDim.x * nw * G;
     // the warp's groups step through their lines together (the transforms
     // synchronise the warp); a group past the last line works on zeros
     auto fetch = [&](int line, double2* L) {
         if (line < nlines) {
+            const int fi = line / flines, l = line - fi * flines;
             if (dir > 0) {
-                row_async<N2>(src + (size_t)line * md, mlim, L, t);
+                row_async<N2>(f.src[fi] + (size_t)l * md, mlim, L, t);
             } else {
-                const double2* row = src + (size_t)line * N;
+                const double2* row = f.src[fi] + (size_t)l * N;
                 for (int j = t; j < N; j += N2)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                                      (uint32_t)__cvta_generic_to_shared(L + phys_pos<N1, N2>(j))),
@@ -745,15 +745,15 @@ __global__ void __launch_bounds__(256) horfft5_kernel(DevGrid g, const double2* 
         fetch(line + stride, L0 + (slot ^ 1) * N);
         async_wait<1>();
         __syncwarp();
+        const int fi = ok ? line / flines : 0;
+        double2* dst = f.dst[fi] + (size_t)(line - fi * flines) * (dir > 0 ? N : md);
         if (dir > 0) {
             grp_inverse5<N1, N2>(nullptr, ok, md, g.NTCHOP, tw, twh, L, t, true);
             __syncwarp();
-            if (ok) {
-                double2* out = dst + (size_t)line * N;
-                for (int j = t; j < N; j += N2) out[j] = L[phys_pos<N1, N2>(j)];
-            }
+            if (ok)
+                for (int j = t; j < N; j += N2) dst[j] = L[phys_pos<N1, N2>(j)];
         } else {
-            grp_forward5<N1, N2>(L, ok, ok ? dst + (size_t)line * md : nullptr, md, g.NTCHOP, tw, twh, t);
+            grp_forward5<N1, N2>(L, ok, ok ? dst : nullptr, md, g.NTCHOP, tw, twh, t);
         }
         __syncwarp();  // the slot is refilled two lines on
     }
@@ -988,8 +988,7 @@ void k_theta_fused(const DevGrid& g, const FFTPlan& p, const double2* const in[1
 }
 
 template <int N1, int N2>
-static void launch_horfft5(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir,
-                           cudaStream_t s) {
+static void launch_horfft5(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
     constexpr int N = N1 * N2, G = 32 / N2;
     const size_t per_warp = (size_t)G * 2 * N * sizeof(double2);
     const size_t fixed = 2 * (size_t)(N + 1) * sizeof(double2);
@@ -1003,35 +1002,47 @@ static void launch_horfft5(const DevGrid& g, const FFTPlan& p, const double2* sr
         cudaFuncSetAttribute(horfft5_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr = true;
     }
-    const int nlines = g.NR * g.NX;
+    const int nlines = g.NR * g.NX * f.n;
     const int per_cta = warps * G;
     const int blocks = std::min((nlines + per_cta - 1) / per_cta, sm_count() * 2);
-    horfft5_kernel<N1, N2><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, dir);
+    horfft5_kernel<N1, N2><<<blocks, warps * 32, sm, s>>>(g, f, p.tw_t, p.tw_h, dir);
     count_launch();
 }
 
-void k_horfft_warp(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s) {
+void k_horfft_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
     switch (g.NTH) {
-        case 16: launch_horfft5<4, 4>(g, p, src, dst, dir, s); return;
-        case 32: launch_horfft5<8, 4>(g, p, src, dst, dir, s); return;
-        case 64: launch_horfft5<8, 8>(g, p, src, dst, dir, s); return;
-        case 128: launch_horfft5<16, 8>(g, p, src, dst, dir, s); return;
-        case 256: launch_horfft5<16, 16>(g, p, src, dst, dir, s); return;
-        case 512: launch_horfft5<32, 16>(g, p, src, dst, dir, s); return;
+        case 16: launch_horfft5<4, 4>(g, p, f, dir, s); return;
+        case 32: launch_horfft5<8, 4>(g, p, f, dir, s); return;
+        case 64: launch_horfft5<8, 8>(g, p, f, dir, s); return;
+        case 128: launch_horfft5<16, 8>(g, p, f, dir, s); return;
+        case 256: launch_horfft5<16, 16>(g, p, f, dir, s); return;
+        case 512: launch_horfft5<32, 16>(g, p, f, dir, s); return;
         default: break;
     }
     const int warps = 8;
     size_t sm = (size_t)warps * (3 * g.NTH + 1) * sizeof(double2);
     int nlines = g.NR * g.NX;
     int blocks = std::min((nlines + warps - 1) / warps, sm_count() * 8);
-    switch (pp_of(g.NTH)) {
-        case 1: horfft_warp_kernel<1><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
-        case 2: horfft_warp_kernel<2><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
-        case 4: horfft_warp_kernel<4><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
-        case 8: horfft_warp_kernel<8><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
-        default: horfft_warp_kernel<16><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+    for (int q = 0; q < f.n; ++q) {
+        const double2* src = f.src[q];
+        double2* dst = f.dst[q];
+        switch (pp_of(g.NTH)) {
+            case 1: horfft_warp_kernel<1><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+            case 2: horfft_warp_kernel<2><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+            case 4: horfft_warp_kernel<4><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+            case 8: horfft_warp_kernel<8><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+            default: horfft_warp_kernel<16><<<blocks, warps * 32, sm, s>>>(g, src, dst, p.tw_t, p.tw_h, p.lt, dir); break;
+        }
+        count_launch();
     }
-    count_launch();
+}
+
+void k_horfft_warp(const DevGrid& g, const FFTPlan& p, const double2* src, double2* dst, int dir, cudaStream_t s) {
+    VerBatch f{};
+    f.n = 1;
+    f.src[0] = src;
+    f.dst[0] = dst;
+    k_horfft_batch(g, p, f, dir, s);
 }
 
 }  // namespace mlegs
