@@ -433,9 +433,8 @@ __device__ __forceinline__ void grp_inverse5(const double2* __restrict__ src, bo
         for (int m = t; m < mlim; m += N2) L[m] = src[m];
     __syncwarp();
     double2 v[N1], o[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-        const int m = t + N2 * n1, mc = N - m;
+    auto pack = [&](int m, double2 w) {  // w = e^{+i pi m/N}
+        const int mc = N - m;
         double2 xm = make_double2(0.0, 0.0), xc = make_double2(0.0, 0.0);
         if (valid) {
             if (m < mlim) xm = L[m];
@@ -443,9 +442,16 @@ __device__ __forceinline__ void grp_inverse5(const double2* __restrict__ src, bo
         }
         if (m == 0) xm.y = 0.0;
         xc = fft4::conj(xc);
-        double2 sm = make_double2(xm.x + xc.x, xm.y + xc.y), d = make_double2(xm.x - xc.x, xm.y - xc.y);
-        double2 ed = fft4::cmul(fft4::conj(twh[m]), d);  // e^{+i pi m/N} d
-        v[n1] = make_double2(sm.x - ed.y, sm.y + ed.x);
+        const double2 sm = make_double2(xm.x + xc.x, xm.y + xc.y), d = make_double2(xm.x - xc.x, xm.y - xc.y);
+        const double2 ed = fft4::cmul(w, d);
+        return make_double2(sm.x - ed.y, sm.y + ed.x);
+    };
+#pragma unroll
+    for (int n1 = 0; n1 < N1 / 2; ++n1) {  // m and m + N/2, whose twiddle is i times m's: one table read for both
+        const int m = t + N2 * n1;
+        const double2 w = fft4::conj(twh[m]);
+        v[n1] = pack(m, w);
+        v[n1 + N1 / 2] = pack(m + N / 2, make_double2(-w.y, w.x));
     }
     __syncwarp();
     fft4::line_fft_inplace<N1, N2, +1>(v, L, tw, t, o);
@@ -480,14 +486,23 @@ __device__ __forceinline__ void grp_forward5(double2* L, bool valid, double2* __
     for (int q = 0; q < N1; ++q) L[fft4::out_index<N1, N2>(t, q)] = o[q];  // Z_k, natural order
     __syncwarp();
     const double sc = 1.0 / (2.0 * N);
-    for (int m = t; m < md; m += N2) {
-        double2 zm = L[m % N], zc = fft4::conj(L[(N - m) % N]);
-        double2 sm = make_double2(zm.x + zc.x, zm.y + zc.y), d = make_double2(zm.x - zc.x, zm.y - zc.y);
-        double2 ed = fft4::cmul(twh[m], d);  // e^{-i pi m/N} d
+    const int mlim = md < ntchop ? md : ntchop;
+    auto put = [&](int m, double2 w) {  // w = e^{-i pi m/N}
+        const double2 zm = L[m], zc = fft4::conj(L[(N - m) & (N - 1)]);
+        const double2 sm = make_double2(zm.x + zc.x, zm.y + zc.y), d = make_double2(zm.x - zc.x, zm.y - zc.y);
+        const double2 ed = fft4::cmul(w, d);
         double2 x = make_double2(0.5 * (sm.x + ed.y) * sc, 0.5 * (sm.y - ed.x) * sc);
-        if (m >= ntchop) x = make_double2(0.0, 0.0);
+        if (m >= mlim) x = make_double2(0.0, 0.0);
         if (m == 0) x.y = 0.0;
         if (valid) dst[m] = x;
+    };
+#pragma unroll
+    for (int n1 = 0; n1 < N1 / 2; ++n1) {
+        const int m = t + N2 * n1;
+        if (m >= md) break;
+        const double2 w = twh[m];  // and -i times that for m + N/2
+        put(m, w);
+        if (m + N / 2 < md) put(m + N / 2, make_double2(w.y, -w.x));
     }
 }
 
@@ -510,9 +525,9 @@ __device__ __forceinline__ double2* pick_out(const PhysArgs& A, int i) {
 
 // After phase 2 (slots: 0-2 velocity, 3 B, 4-6 vorticity, 7 RBR): slots 4-6 <-
 // N_r, N_theta, N_z of VPRODSUB (+ the linear terms), slot 7 <- a1 c1.
-template <int N>
+template <int N, int TL>
 __device__ __forceinline__ void theta_products_r2(double2* L, int lane, double ir2, double o2, int linear) {
-    for (int j = lane; j < N; j += 32) {
+    for (int j = lane; j < N; j += TL) {
         const double2 a1 = L[j], a2 = L[N + j], a3 = L[2 * N + j];
         const double2 b1 = L[4 * N + j], b2 = L[5 * N + j], b3 = L[6 * N + j], c1 = L[7 * N + j];
         double2 nr_ = make_double2(a2.x * b3.x - a3.x * b2.x, a2.y * b3.y - a3.y * b2.y);
@@ -535,9 +550,9 @@ __device__ __forceinline__ void theta_products_r2(double2* L, int lane, double i
 }
 
 // After phase 3 (slot 3 RBP, slot 8 BZ): slot 7 <- N_b of VDOTPSUB (+ N^2 u_z).
-template <int N>
+template <int N, int TL>
 __device__ __forceinline__ void theta_products_r3(double2* L, int lane, double ir2, double n2, int linear) {
-    for (int j = lane; j < N; j += 32) {
+    for (int j = lane; j < N; j += TL) {
         const double2 a2 = L[N + j], a3 = L[2 * N + j], c2 = L[3 * N + j], c3 = L[8 * N + j];
         const double2 bp = L[7 * N + j];
         double2 bn_ = make_double2(-((bp.x + a2.x * c2.x) * ir2 + a3.x * c3.x),
@@ -552,9 +567,18 @@ __device__ __forceinline__ void theta_products_r3(double2* L, int lane, double i
 
 }  // namespace
 
+// Warps per CTA (one CTA per SM): at NTH = 128 the nine line slots of 12 warps
+// fill shared memory; shorter lines leave room for more warps than 168 registers
+// a thread would (12 warps), so the kernel is compiled for 24 there: it is bound
+// by the latency of its FP64 and shared-memory instructions.
+template <int N>
+constexpr int theta_warps() {
+    return N <= 64 ? 24 : 12;
+}
+
 template <int N1, int N2>
-__global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, const double2* tw_g,
-                                                     const double2* twh_g) {
+__global__ void __launch_bounds__(32 * theta_warps<N1 * N2>(), 1)
+    theta5_kernel(DevGrid g, PhysArgs A, const double2* tw_g, const double2* twh_g) {
     constexpr int N = N1 * N2, G = 32 / N2;
     static_assert(G == 4 || G == 2 || G == 8, "4 lines per round need G in {2, 4, 8}");
     extern __shared__ double2 sm[];
@@ -566,12 +590,16 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int gid = lane / N2, t = lane % N2;
-    double2* L = twh + (N + 1) + (size_t)warp * 9 * N;
+    const int t = lane % N2;
     const int md = g.NTCHOPDIM;
     const int nlines = g.NR * g.NX;
     const double o2 = 2 * A.omega, n2 = A.bv0 * A.bv0;
-    if constexpr (G == 4) {
+    if constexpr (G >= 4) {
+        // A team of four lane groups owns a line: one team per warp at N2 = 8, two
+        // (two lines side by side) at N2 = 4.
+        constexpr int TL = 4 * N2, TEAMS = 32 / TL;
+        const int gid = (lane / N2) % 4, team = lane / TL, tl = lane % TL;
+        double2* L = twh + (N + 1) + (size_t)(warp * TEAMS + team) * 9 * N;
         // Rows arrive by cp.async one round ahead: the three (four) round-1
         // rows of the next line while this line's forward transforms run, the
         // round-2 rows (and, without the linear terms, the round-3 rows into
@@ -588,13 +616,16 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
             if (gid < 2) row_async<N2>(pick_in(A, 7 + gid) + o, mlim, L + (size_t)(gid ? 8 : 3) * N, t);
             async_commit();
         };
-        const int line0 = blockIdx.x * nw + warp;
-        if (line0 < nlines) issue_r1(line0);
-        for (int line = line0; line < nlines; line += gridDim.x * nw) {
+        const int stride = gridDim.x * nw * TEAMS, base0 = (blockIdx.x * nw + warp) * TEAMS;
+        // a team past the last line repeats it without storing
+        auto mine = [&](int base) { return min(base + team, nlines - 1); };
+        if (base0 < nlines) issue_r1(mine(base0));
+        for (int base = base0; base < nlines; base += stride) {
+            const int line = mine(base), nxt = base + stride;
+            const bool live = base + team < nlines;
             const size_t off = (size_t)line * md;
-            const int nxt = line + gridDim.x * nw;
-            if (lane < 10 && nxt < nlines && (lane < 9 || A.linear))
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pick_in(A, lane) + (size_t)nxt * md),
+            if (tl < 10 && nxt < nlines && (tl < 9 || A.linear))
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pick_in(A, tl) + (size_t)mine(nxt) * md),
                              "r"((unsigned)(md * sizeof(double2)))
                              : "memory");
             const double rr = g.r[line / g.NX];
@@ -617,7 +648,7 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
             __syncwarp();
             grp_inverse5<N1, N2>(nullptr, true, md, g.NTCHOP, tw, twh, L + (size_t)(4 + gid) * N, t, true);
             __syncwarp();
-            theta_products_r2<N>(L, lane, ir2, o2, A.linear);
+            theta_products_r2<N, TL>(L, tl, ir2, o2, A.linear);
             __syncwarp();
             // phase 3: RBP -> slot 3, BZ -> slot 8
             if (A.linear) issue_r3(line);
@@ -628,13 +659,15 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
             else
                 idle_group_syncs();
             __syncwarp();
-            theta_products_r3<N>(L, lane, ir2, n2, A.linear);
+            theta_products_r3<N, TL>(L, tl, ir2, n2, A.linear);
             __syncwarp();
-            if (nxt < nlines) issue_r1(nxt);  // slots 0-3 are free from here on
-            grp_forward5<N1, N2>(L + (size_t)(4 + gid) * N, true, pick_out(A, gid) + off, md, g.NTCHOP, tw, twh, t);
+            if (nxt < nlines) issue_r1(mine(nxt));  // slots 0-3 are free from here on
+            grp_forward5<N1, N2>(L + (size_t)(4 + gid) * N, live, pick_out(A, gid) + off, md, g.NTCHOP, tw, twh, t);
             __syncwarp();
         }
     } else {
+    const int gid = lane / N2;
+    double2* L = twh + (N + 1) + (size_t)warp * 9 * N;
     for (int line = blockIdx.x * nw + warp; line < nlines; line += gridDim.x * nw) {
         const size_t off = (size_t)line * md;
         // the warp's next line: lanes 0..9 ask L2 for its ten input rows (md complex each)
@@ -650,7 +683,7 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
         }
         const double rr = g.r[line / g.NX];
         const double ir2 = 1.0 / (rr * rr);
-        // phase 1 and 2 (G = 4: one field per group; G = 2: two passes; G = 8: half the groups idle)
+        // phase 1 and 2, two fields at a time
         // phase 1: field q (q < 3) or B (q = 3, linear terms only) -> slot q;
         // phase 2: field 3 + q -> slot 4 + q
         for (int rd = 0; rd < 2; ++rd) {
@@ -668,7 +701,7 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
             __syncwarp();
         }
         // round-2 products
-        theta_products_r2<N>(L, lane, ir2, o2, A.linear);
+        theta_products_r2<N, 32>(L, lane, ir2, o2, A.linear);
         __syncwarp();
         // phase 3
         for (int f0 = 0; f0 < 4; f0 += G) {
@@ -679,7 +712,7 @@ __global__ void __launch_bounds__(384, 1) theta5_kernel(DevGrid g, PhysArgs A, c
                 idle_group_syncs();
         }
         __syncwarp();
-        theta_products_r3<N>(L, lane, ir2, n2, A.linear);
+        theta_products_r3<N, 32>(L, lane, ir2, n2, A.linear);
         __syncwarp();
         // forward transforms of the four results
         for (int f0 = 0; f0 < 4; f0 += G) {
@@ -937,21 +970,23 @@ static void launch_theta4(const DevGrid& g, const FFTPlan& p, const PhysArgs& A,
 
 template <int N1, int N2>
 static bool launch_theta5(const DevGrid& g, const FFTPlan& p, const PhysArgs& A, cudaStream_t s) {
-    constexpr int N = N1 * N2;
-    const size_t per_warp = (size_t)9 * N * sizeof(double2);
+    constexpr int N = N1 * N2, TEAMS = N2 <= 8 ? 8 / N2 : 1;  // lines a warp holds at a time
+    const size_t per_warp = (size_t)9 * N * TEAMS * sizeof(double2);
     const size_t fixed = 2 * (size_t)(N + 1) * sizeof(double2);
-    int warps = (int)((227 * 1024 - fixed) / per_warp);
-    if (warps > 12) warps = 12;
+    int warps = std::min((int)((227 * 1024 - fixed) / per_warp), theta_warps<N>());
     if (warps < 1) return false;
-    const size_t sm = fixed + warps * per_warp;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(theta5_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         attr = true;
     }
-    const int nlines = g.NR * g.NX;
-    const int blocks = std::min((nlines + warps - 1) / warps, sm_count());
-    theta5_kernel<N1, N2><<<blocks, warps * 32, sm, s>>>(g, A, p.tw_t, p.tw_h);
+    // the fewest rounds over the lines that the full CTAs need, then no more warps
+    // than those rounds take: every SM gets its share of a small grid
+    const int items = (g.NR * g.NX + TEAMS - 1) / TEAMS, sms = sm_count();
+    const int rounds = (items + sms * warps - 1) / (sms * warps);
+    warps = std::max(1, (items + sms * rounds - 1) / (sms * rounds));
+    const int blocks = std::min((items + warps - 1) / warps, sms);
+    theta5_kernel<N1, N2><<<blocks, warps * 32, fixed + warps * per_warp, s>>>(g, A, p.tw_t, p.tw_h);
     count_launch();
     return true;
 }
