@@ -47,6 +47,7 @@ struct EnsInst {
     Field* WK[3] = {};
     Field* VA[3] = {};  // fields solved by IHELM in phase 3
     int nvisc = 0;
+    bool fused = false;  // phase 3 as one pass (viscosity on every field)
     cudaEvent_t ev = nullptr;
 };
 
@@ -171,8 +172,15 @@ namespace {
 
 constexpr int P3 = 3;  // CHOPSET(3) of CALC_BOUSSI_FORCE
 
+// The phases' own passes are the single-context step's joint ones (one launch for
+// the nine derivative fields, one for the ten VERFFT(+1), one for the four
+// VERFFT(-1), one for the AB2 update with the viscous right-hand sides); as
+// separate copies, AXPBYs, chops and log-term rows they were a third of the
+// serialised step.
+
 // Phase 0: the derivative fields of CALC_BOUSSI_FORCE (GRAD, PC2VEL, PC2VOR at
-// CHOPSET(3); W = B at CHOPSET(0)) and their RTRAN(+1) problems.
+// CHOPSET(3)) and their RTRAN(+1) problems, and that of W = B at CHOPSET(0), read
+// from B itself (the GEMM uses only the rows that COPY0 keeps).
 void phase0(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
     I.pool0 = c->pool;
@@ -185,14 +193,13 @@ void phase0(mlegs_ensemble& E, EnsInst& I) {
     for (Field*& f : I.f) f = c->tmp();
     Field **f = I.f;
     c->derivatives(c->psi, c->chi, c->b, f, P3);
-    c->copy0(f[9], c->b, 0);
     for (int q = 0; q < 10; ++q) {
         I.T[q] = c->tmp(MLEGS_PFF);
         GroupB2P p{};
         p.g = c->g;
-        p.in = (const double*)f[q]->data;
+        p.in = (const double*)(q < 9 ? f[q] : c->b)->data;
         p.out = (double*)I.T[q]->data;
-        p.ln = f[q]->ln;
+        p.ln = q < 9 ? nullptr : c->b->ln;  // the derivative fields carry no log term
         p.pad = q < 9 ? P3 : 0;
         p.nj = E.nj_for(0, c->g);
         E.gb2p.h.push_back(p);
@@ -222,25 +229,27 @@ void phase1(mlegs_ensemble& E, EnsInst& I) {
     for (int q = 0; q < 10; ++q) in[q] = I.f[q]->data;
     double2* out[4] = {I.NR->data, I.NP->data, I.NZ->data, I.BNp->data};
     k_theta_fused(g, c->fft, in, out, c->p.omega, c->p.bv0, 1, c->s);
-    for (Field* x : {I.NR, I.NP, I.NZ, I.BNp}) {
-        x->space = MLEGS_PFP;
-        c->ln_zero(x);
+    // VERFFT(-1) of the four results, into buffers of the inputs that are done with
+    VerBatch w{};
+    w.n = 4;
+    Field* const res[4] = {I.NR, I.NP, I.NZ, I.BNp};
+    for (int q = 0; q < 4; ++q) {
+        w.src[q] = res[q]->data;
+        w.dst[q] = I.f[q]->data;
     }
-    for (Field* x : I.f) c->rel(x);
-    I.Wf = c->tmp();
-    // PROJECT(NR, NP, NZ, PSI_N, W, 0) of PFP input (mod_legops.f90:2397-2545)
-    c->verfft(I.NR, -1);
-    c->verfft(I.NP, -1);
-    c->verfft(I.NZ, -1);
-    I.PN->space = I.Wf->space = MLEGS_FFF;
-    launch_vel2pln(g, I.NP->data, I.PN->ln, 1, 0.0, c->v2p_pff, c->s, I.Wf->ln);
+    c->verfft_batch(w, -1, c->s);
+    I.Wf = I.f[9];
+    // PROJECT(NR, NP, NZ, PSI_N, W, 0) (mod_legops.f90:2397-2545)
+    I.PN->space = I.Wf->space = I.BN->space = MLEGS_FFF;
+    launch_vel2pln(g, I.f[1]->data, I.PN->ln, 1, 0.0, c->v2p_pff, c->s, I.Wf->ln, I.BN->ln);
     GroupFold pj{};
     pj.g = g;
-    const double* w[5] = {c->V, c->D, c->D, c->V, c->T};
-    const double2* x[5] = {I.NR->data, I.NP->data, I.NR->data, I.NP->data, I.NZ->data};
+    const double* wt[5] = {c->V, c->D, c->D, c->V, c->T};
+    Field** f = I.f;
+    const double2* x[5] = {f[0]->data, f[1]->data, f[0]->data, f[1]->data, f[2]->data};
     const int mode[5] = {0, 1, 1, 0, 0}, scale[5] = {2, 1, 3, 4, 1};
     for (int q = 0; q < 5; ++q) {
-        pj.fa.w[q] = w[q];
+        pj.fa.w[q] = wt[q];
         pj.fa.x[q] = (const double*)x[q];
         pj.fa.mode[q] = mode[q];
         pj.fa.scale[q] = scale[q];
@@ -252,29 +261,23 @@ void phase1(mlegs_ensemble& E, EnsInst& I) {
     pj.fa.wt_rows = g.NRCHOPDIM;
     pj.nj = E.nj_for(1, g);
     E.gfold.h.push_back(pj);
-    // TOFF(B_N): VERFFT(-1), then RTRAN(-1) into the context's scratch buffer
-    c->verfft(I.BNp, -1);
+    // TOFF(B_N): RTRAN(-1) of its VERFFT(-1) image
     GroupFold rt{};
     rt.g = g;
     rt.fa.w[0] = c->pf;
-    rt.fa.x[0] = (const double*)I.BNp->data;
+    rt.fa.x[0] = (const double*)f[3]->data;
     rt.fa.nseg = rt.fa.split = 1;
-    rt.fa.out0 = rt.fa.out1 = (double*)c->scratch;
+    rt.fa.out0 = rt.fa.out1 = (double*)I.BN->data;
     rt.fa.wt_rows = g.NRCHOPDIM + 1;
     rt.fa.use_w = 1;
     rt.nj = E.nj_for(1, g);
     E.gfold.h.push_back(rt);
 }
 
-// Phase 2: PROJECT's far-field fix, B_N = TOFF(...), IDEL2LN(W -> CHI_N) problem.
+// Phase 2: PROJECT's far-field fix, the IDEL2LN(W -> CHI_N) problem.
 void phase2(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
     k_farfield_fix(c->g, I.PN->data, c->d.NRCHOP, c->s);
-    c->swap_scratch_any(I.BNp);
-    I.BNp->space = MLEGS_FFF;
-    c->ln_zero(I.BNp);
-    c->copy0(I.BN, I.BNp, 0);
-    for (Field* x : {I.BNp, I.NR, I.NP, I.NZ}) c->rel(x);
     const auto* fc = c->factors(0, 0, 0.0);
     if (!fc) throw ApiError(MLEGS_ERR_STATE, "ensemble: IDEL2LN factors missing");
     GroupSolve p{};
@@ -295,7 +298,46 @@ void phase3(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
     const DevGrid& g = c->g;
     const double dt = c->p.dt;
-    c->rel(I.Wf);
+    for (Field* x : {I.BNp, I.NR, I.NP, I.NZ}) c->rel(x);
+    for (Field* x : I.f) c->rel(x);
+    I.nvisc = 0;
+    I.fused = c->p.visc_sw == 1 && c->p.nu != 0.0 && c->p.kappa != 0.0;
+    if (I.fused) {
+        Field* A[3] = {c->psi, c->chi, c->b};
+        Field* N1[3] = {I.PN, I.CN, I.BN};
+        const double nu[3] = {c->p.nu, c->p.nu, c->p.kappa};
+        Ab2Args a{};
+        a.n = 3;
+        a.c1 = 1.5 * dt;
+        a.c0 = -0.5 * dt;
+        for (int q = 0; q < 3; ++q) {
+            Field* WK = I.WK[q] = c->tmp();
+            a.a[q] = A[q]->data;
+            a.n1[q] = N1[q]->data;
+            a.n0[q] = c->hist[q]->data;
+            a.rhs[q] = WK->data;
+            a.a_ln[q] = A[q]->ln;
+            a.n1_ln[q] = q < 2 ? N1[q]->ln : nullptr;
+            a.n0_ln[q] = c->hist[q]->ln;
+            a.rhs_ln[q] = WK->ln;
+            a.alp[q] = 2 / nu[q] / dt;
+            const auto* fh = c->factors(2, 0, a.alp[q]);
+            if (!fh) throw ApiError(MLEGS_ERR_STATE, "ensemble: IHELM factors missing");
+            GroupSolve p{};
+            p.g = g;
+            p.kind = 2;
+            p.it.F = fh->F;
+            p.it.src = WK->data;
+            p.it.dst = A[q]->data;
+            p.it.ln_src[0] = WK->ln;
+            p.it.ln_dst[0] = A[q]->ln;
+            p.it.ln_src[1] = N1[q]->ln;
+            p.it.ln_dst[1] = c->hist[q]->ln;
+            E.gs2.h.push_back(p);
+        }
+        k_ab2_visc_rhs(g, a, c->s);
+        return;
+    }
     I.P0 = c->tmp();
     I.C0 = c->tmp();
     I.B0 = c->tmp();
@@ -315,7 +357,6 @@ void phase3(mlegs_ensemble& E, EnsInst& I) {
     c->rel(I.PN);
     c->rel(I.CN);
     c->rel(I.BN);
-    I.nvisc = 0;
     if (c->p.visc_sw != 1) return;
     Field* A[3] = {c->psi, c->chi, c->b};
     Field* AO[3] = {I.P0, I.C0, I.B0};
@@ -351,13 +392,18 @@ void phase3(mlegs_ensemble& E, EnsInst& I) {
 // Phase 4: IHELM's CHOPDO, CALC_BOUSSI_HYPERV, and the step's temporaries back.
 void phase4(mlegs_ensemble&, EnsInst& I) {
     mlegs_ctx* c = I.c;
-    for (int q = 0; q < I.nvisc; ++q) {
-        c->chopdo(I.VA[q], 0);
-        c->rel(I.WK[q]);
+    if (I.fused) {  // the solves wrote chopped fields
+        for (Field* x : I.WK) c->rel(x);
+        for (Field* x : {I.PN, I.CN, I.BN}) c->rel(x);
+    } else {
+        for (int q = 0; q < I.nvisc; ++q) {
+            c->chopdo(I.VA[q], 0);
+            c->rel(I.WK[q]);
+        }
+        c->rel(I.P0);
+        c->rel(I.C0);
+        c->rel(I.B0);
     }
-    c->rel(I.P0);
-    c->rel(I.C0);
-    c->rel(I.B0);
     c->hyperv3(c->psi, c->chi, c->b, 1.0);
     c->restore();
     c->pool = I.pool0;
