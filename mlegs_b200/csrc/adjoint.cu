@@ -203,6 +203,173 @@ __global__ void vdotp_T_kernel(const DevGrid g, P3 A, P3 B, const double2* y, Q3
     }
 }
 
+// The products' adjoints of a whole right-hand side in one pass, in place on the
+// operands (ROR = N_r + 2 OMEGA RUP, ROP = N_t - 2 OMEGA RUR, OZ = N_z - W,
+// BN = -VDOTP(U, G) + N^2 UZ): f[0..2] the velocity, f[3..5] the vorticity, f[6..8]
+// grad b in, their cotangents out; nb[0..2] the cotangents of N, nb[3] of BN in,
+// nb[2] out: W's cotangent.
+struct ProductsT {
+    double2* f[9];
+    double2* nb[4];
+    double o2, n2;
+};
+__global__ void __launch_bounds__(256) products_T_kernel(const DevGrid g, const __grid_constant__ ProductsT A) {
+    const int plane = g.NX * g.NTH;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+    if (e >= plane) return;
+    const size_t t = (size_t)r * plane + e;
+    const double ir2 = 1.0 / (g.r[r] * g.r[r]);
+    double2 f[9], b[4];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) f[q] = A.f[q][t];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = A.nb[q][t];
+    auto part = [&](double (&v)[9], double n1, double n2_, double n3, double nbv, double& w) {
+        const double b3r = n3 * ir2, y = -nbv;
+        const double u1 = v[0], u2 = v[1], u3 = v[2], w1 = v[3], w2 = v[4], w3 = v[5], g1 = v[6], g2 = v[7], g3 = v[8];
+        v[0] = -n2_ * w3 + b3r * w2 + ir2 * g1 * y - A.o2 * n2_;
+        v[1] = n1 * w3 - b3r * w1 + ir2 * g2 * y + A.o2 * n1;
+        v[2] = -n1 * w2 + n2_ * w1 + g3 * y + A.n2 * nbv;
+        v[3] = n2_ * u3 - b3r * u2;
+        v[4] = -n1 * u3 + b3r * u1;
+        v[5] = n1 * u2 - n2_ * u1;
+        v[6] = ir2 * u1 * y;
+        v[7] = ir2 * u2 * y;
+        v[8] = u3 * y;
+        w = -n3;
+    };
+    double re[9], im[9], wr, wi;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        re[q] = f[q].x;
+        im[q] = f[q].y;
+    }
+    part(re, b[0].x, b[1].x, b[2].x, b[3].x, wr);
+    part(im, b[0].y, b[1].y, b[2].y, b[3].y, wi);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) A.f[q][t] = make_double2(re[q], im[q]);
+    A.nb[2][t] = make_double2(wr, wi);
+}
+
+// (m, n, k) of a launch over tiles of 32 k by 8 rows n.
+__device__ __forceinline__ bool tile_of(const DevGrid& g, size_t& t, int& m, int& n, int& k) {
+    k = blockIdx.x * 32 + threadIdx.x;
+    n = blockIdx.y * 8 + threadIdx.y;
+    m = blockIdx.z;
+    t = ((size_t)m * g.NRCHOPDIM + n) * g.NXCHOPDIM + k;
+    return k < g.NXCHOPDIM && n < g.NRCHOPDIM;
+}
+inline dim3 tiles_of(const DevGrid& g) {
+    return dim3((g.NXCHOPDIM + 31) / 32, (g.NRCHOPDIM + 7) / 8, g.NTCHOPDIM);
+}
+// The far-field fix (CALCAT1 over n < NRCHOP) and the chop transposed, at (m, n, k).
+__device__ __forceinline__ double2 farfield_T_at(const DevGrid& g, const double2* y, size_t t, int m, int n, int k) {
+    if (n >= nrc(g, m, 0)) return make_double2(0.0, 0.0);
+    double2 v = y[t];
+    if (m == 0) {
+        if (n == 0) return make_double2(0.0, 0.0);
+        const double f = g.at1[n] / g.at1[0];
+        const double2 y0 = y[k];
+        v = make_double2(v.x - f * y0.x, v.y - f * y0.y);
+    }
+    return v;
+}
+// IDEL2LN^T up to its solve: the cotangent of A through the far-field fix, A%LN's
+// (ln / NORM(1,1)) in A(1,1,1)'s place.
+__global__ void __launch_bounds__(256) idel2ln_T_prep_kernel(const DevGrid g, const double2* a, const double* ln,
+                                                             double2* out) {
+    size_t t;
+    int m, n, k;
+    if (!tile_of(g, t, m, n, k)) return;
+    out[t] = (m == 0 && n == 0 && k == 0) ? make_double2(*ln * g.norm0[0], 0.0) : farfield_T_at(g, a, t, m, n, k);
+}
+// The inputs of PROJECT^T's products and of RTRAN(-1)^T, times s0 (m = 0) or s1:
+// -i k W, i m PSI, -PSI, m k W, -W and B_N, PSI's cotangent through the far-field fix.
+struct ProjectPrepT {
+    const double2 *psi, *w, *bn;
+    double2* z[6];
+    double s0, s1;
+};
+__global__ void __launch_bounds__(256) project_T_prep_kernel(const DevGrid g, const __grid_constant__ ProjectPrepT A) {
+    size_t t;
+    int m, n, k;
+    if (!tile_of(g, t, m, n, k) || n >= nrc(g, m, 0)) return;  // the GEMM reads the kept rows only
+    const double s = m == 0 ? A.s0 : A.s1, mv = m * s, kv = g.ak[k] * s;
+    const double2 p = farfield_T_at(g, A.psi, t, m, n, k), w = A.w[t], b = A.bn[t];
+    A.z[0][t] = make_double2(w.y * kv, -w.x * kv);
+    A.z[1][t] = make_double2(-p.y * mv, p.x * mv);
+    A.z[2][t] = make_double2(-s * p.x, -s * p.y);
+    A.z[3][t] = make_double2(mv * g.ak[k] * w.x, mv * g.ak[k] * w.y);
+    A.z[4][t] = make_double2(-s * w.x, -s * w.y);
+    A.z[5][t] = make_double2(s * b.x, s * b.y);
+}
+// Around the right-hand side's VJP in one AB2-CN step's: wk = IHELM^T of the state's
+// cotangents (blockIdx.z: field and m).  First the cotangents of the nonlinear terms
+// and of the history, wk's LN slot <- that of -ALP wk; then the state's:
+//   first:  fbar = n_bar chopped + 1.5 dt a, out_n = -0.5 dt a,   a = -ALP wk
+//   second: out = a - DEL2^T(wk) (chopped) + fo.
+struct StepT {
+    const double2* wk[3];
+    double* wk_ln[3];
+    const double* y_ln[3];   // LN of the state's cotangents
+    const double2* x[3];     // first: n_bar; second: fo
+    const double* x_ln[3];
+    double2* o1[3];          // first: fbar; second: out
+    double* o1_ln[3];
+    double2* o2[3];          // first: out_n
+    double* o2_ln[3];
+    double alp[3];
+    double dt;
+};
+template <bool FIRST>
+__global__ void __launch_bounds__(256) step_T_kernel(const DevGrid g, const __grid_constant__ StepT A) {
+    const int f = blockIdx.z / g.NTCHOPDIM, m = blockIdx.z - f * g.NTCHOPDIM;
+    const int k = blockIdx.x * 32 + threadIdx.x, n = blockIdx.y * 8 + threadIdx.y;
+    if (k >= g.NXCHOPDIM || n >= g.NRCHOPDIM) return;
+    const size_t st = g.NXCHOPDIM, t = ((size_t)m * g.NRCHOPDIM + n) * st + k;
+    const int nn = nrc(g, m, 0);
+    const double alp = A.alp[f], dt = A.dt;
+    const double2* wk = A.wk[f];
+    const double2 w = wk[t];
+    const double2 a = make_double2(-alp * w.x, -alp * w.y);
+    const double cf[3] = {4.0 / 3 / g.ELL2 / g.norm0[0], -2.0 / g.norm0[1] / g.ELL2, 2.0 / 3 / g.norm0[2] / g.ELL2};
+    const bool lnt = m == 0 && n == 0 && k == 0;
+    double lnrow = 0.0;
+    if (lnt)
+        for (int j = 0; j < 3; ++j) lnrow += cf[j] * wk[j * st].x;
+    if constexpr (FIRST) {
+        const double2 x = n < nn ? A.x[f][t] : make_double2(0.0, 0.0);
+        A.o1[f][t] = make_double2(x.x + 1.5 * dt * a.x, x.y + 1.5 * dt * a.y);
+        A.o2[f][t] = make_double2(-0.5 * dt * a.x, -0.5 * dt * a.y);
+        if (lnt) {  // b carries no log term
+            const double aln = f == 2 ? 0.0 : -alp * (-*A.y_ln[f] / alp + lnrow / alp);
+            const double fl = f == 2 ? 0.0 : *A.x_ln[f] + 1.5 * dt * aln;
+            *A.wk_ln[f] = aln;
+            *A.o1_ln[f] = fl;
+            *A.o2_ln[f] = -0.5 * dt * aln;
+        }
+    } else {
+        double2 d = make_double2(0.0, 0.0);
+        if (n < nn) {
+            const double* tb = g.del2h + ((size_t)m * g.NB + n) * 5;
+#pragma unroll
+            for (int e = 0; e < 5; ++e) {
+                const int j = n + e - 2;
+                if (j < 0 || j >= nn) continue;
+                const double2 v = wk[t + ((ptrdiff_t)e - 2) * (ptrdiff_t)st];
+                d.x += tb[e] * v.x;
+                d.y += tb[e] * v.y;
+            }
+            const double k2 = g.ak[k] * g.ak[k];
+            d.x -= k2 * w.x;
+            d.y -= k2 * w.y;
+        }
+        const double2 x = A.x[f][t];
+        A.o1[f][t] = make_double2(a.x - d.x + x.x, a.y - d.y + x.y);
+        if (lnt) *A.o1_ln[f] = f == 2 ? 0.0 : *A.wk_ln[f] - lnrow + *A.x_ln[f];
+    }
+}
+
 // y = s W_r R(m, r, k) on PFF with W_r = w_r [/ (1 - x_r)^2] and m = 0 halved:
 // the per-entry weights of the PRODCT_MK / L2NORM_MK quadratures of
 // CALC_BOUSSI_ENERGY and CALC_BOUSSI_PE (mod_boussinesq.f90:112-206).
@@ -235,6 +402,13 @@ __global__ void fff_dot_kernel(const DevGrid g, const double2* a, const double2*
 __global__ void zero_col00_kernel(const DevGrid g, double2* y) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n < g.NRCHOPDIM) y[(size_t)n * g.NXCHOPDIM] = make_double2(0.0, 0.0);
+}
+
+// PF times the Gauss weights (RTRAN(-1)^T as a RTRAN(+1) GEMM).
+__global__ void pf_w_kernel(const DevGrid g, double* Wp) {
+    const size_t n = (size_t)g.NTCHOPDIM * (g.NRCHOPDIM + 1) * g.NRH;
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (t < n) Wp[t] = g.pf[t] * g.w[t % g.NRH];
 }
 
 // V, D or T [m][NRCHOPDIM][NRH] copied into PF's row stride [m][NRCHOPDIM + 1][NRH]
@@ -311,9 +485,24 @@ struct Adj {
             pad_rows_kernel<<<nb(np, 256), 256, 0, c->s>>>(c->g, W[q], c->adj_w[q]);
             count_launch();
         }
+        if (joint()) {
+            c->adj_w[3] = dalloc<double>(np);
+            pf_w_kernel<<<nb(np, 256), 256, 0, c->s>>>(c->g, c->adj_w[3]);
+            count_launch();
+            c->adj_fc = dalloc<double>(fold_table_doubles(c->g, d.NRCHOPDIM));
+            k_fold_table(c->g, c->pf, d.NRCHOPDIM + 1, d.NRCHOPDIM, 0, c->adj_fc, c->s);
+        }
         c->adj_dot = dalloc<double>(1);
         CK(cudaStreamSynchronize(c->s));
         c->adj_ready = true;
+    }
+
+    // The VJP's joint launches: grids whose GEMMs have the bulk-copy forms and whose
+    // FFT lengths have the batched kernels.
+    bool joint() const {
+        const DevGrid& g = c->g;
+        auto fft = [](int v) { return v >= 16 && v <= 512; };
+        return b2p_bulk_supported(g) && fold_bulk_supported(g, g.NRCHOPDIM) && fft(g.NX) && fft(g.NTH);
     }
 
     // Temporaries; the pool grows on demand (outside capture), recorded in the
@@ -634,6 +823,10 @@ struct Adj {
     // CALC_BOUSSI_FORCE at (PSI, CHI, B): (PSIN_bar, CHIN_bar, BN_bar) -> (PSI_bar, CHI_bar, B_bar)
     void force_vjp(const Field* PSI, const Field* CHI, const Field* B, const Field* pnb, const Field* cnb,
                    const Field* bnb, Field* pb, Field* cb, Field* bb) {
+        if (c->adj_fc) {
+            force_vjp_joint(PSI, CHI, B, pnb, cnb, bnb, pb, cb, bb);
+            return;
+        }
         const int P3v = 3;  // CHOPSET(3)
         const size_t np = c->d.ppp();
         // the products' operands in PPP (TOFP of PC2VEL, PC2VOR and GRAD(B) at CHOPSET(3))
@@ -701,9 +894,193 @@ struct Adj {
         for (Field* f : {pb, cb, bb}) f->space = MLEGS_FFF;
     }
 
+    // force_vjp with each stage's fields in one launch: 16 launches where the
+    // operators one by one take about 220, most of them a few us at 96x64x64 (the
+    // whole step's VJP: 1390 us, of which the transforms and solves were 550).
+    // Linear factors of the FFT transposes (per mode m) ride on the passes next
+    // to them.
+    void force_vjp_joint(const Field* PSI, const Field* CHI, const Field* B, const Field* pnb, const Field* cnb,
+                         const Field* bnb, Field* pb, Field* cb, Field* bb) {
+        const DevGrid& gr = g();
+        const double nx = c->d.NX, n2t = 2.0 * c->d.NTH;
+        Field *f[9], *T[9], *h[4];
+        for (Field*& q : f) q = tmp();
+        for (Field*& q : T) q = tmp();
+        for (Field*& q : h) q = tmp();
+        auto ver = [&](Field* const* src, Field* const* dst, int n, int dir) {
+            VerBatch v{};
+            v.n = n;
+            for (int q = 0; q < n; ++q) {
+                v.src[q] = src[q]->data;
+                v.dst[q] = dst[q]->data;
+            }
+            c->verfft_batch(v, dir, s());
+        };
+        auto hor = [&](Field* const* src, Field* const* dst, int n, int dir) {
+            VerBatch v{};
+            v.n = n;
+            for (int q = 0; q < n; ++q) {
+                v.src[q] = src[q]->data;
+                v.dst[q] = dst[q]->data;
+            }
+            k_horfft_batch(gr, c->fft, v, dir, s());
+        };
+        // the products' operands in PPP: TOFP of PC2VEL, PC2VOR and GRAD(B) at CHOPSET(3), in T
+        c->derivatives(PSI, CHI, B, f, 3);
+        {
+            B2PBatch b{};
+            b.n = 9;
+            for (int q = 0; q < 9; ++q) {
+                b.in[q] = f[q]->data;
+                b.out[q] = T[q]->data;
+                b.pad[q] = 3;
+            }
+            k_rtran_b2p_batch(gr, b, s());
+        }
+        ver(T, f, 9, +1);
+        hor(f, T, 9, +1);
+        // cotangents of W = DEL2(CHI_N) (IDEL2LN^T, in f[0])
+        idel2ln_T_prep_kernel<<<tiles_of(gr), dim3(32, 8), 0, s()>>>(gr, cnb->data, cnb->ln, f[0]->data);
+        count_launch();
+        k_solve_T(gr, factors(0, 0.0)->F, f[0]->data, 0, 0, s());
+        // PROJECT^T and TOFF^T up to PPP: h[0..2] the cotangents of N, h[3] of B_N;
+        // VERFFT(-1)^T and HORFFT(-1)^T carry 1/NX and 1/(2 NTH) (m = 0), 1/(4 NTH)
+        {
+            ProjectPrepT a{};
+            a.psi = pnb->data;
+            a.w = f[0]->data;
+            a.bn = bnb->data;
+            for (int q = 0; q < 6; ++q) a.z[q] = f[1 + q]->data;
+            a.s0 = 1.0 / (nx * n2t);
+            a.s1 = 0.5 / (nx * n2t);
+            project_T_prep_kernel<<<tiles_of(gr), dim3(32, 8), 0, s()>>>(gr, a);
+            count_launch();
+            B2PBatch b{};
+            b.n = 4;
+            const int first[5] = {0, 2, 4, 5, 6}, mode[6] = {1, 0, 1, 0, 0, 0};
+            const int w[6] = {1, 0, 1, 0, 2, 3};  // D, V, D, V, T, PF w
+            for (int q = 0; q < 6; ++q) {
+                b.in[q] = f[1 + q]->data;
+                b.pf[q] = c->adj_w[w[q]];
+                b.mode[q] = mode[q];
+            }
+            for (int o = 0; o < 4; ++o) b.out[o] = h[o]->data;
+            for (int o = 0; o < 5; ++o) b.first[o] = first[o];
+            k_rtran_b2p_batch(gr, b, s());
+        }
+        vel2pln_T_kernel<<<1, 256, 0, s()>>>(gr, h[1]->data, c->v2p_pff);
+        count_launch();
+        ver(h, f, 4, +1);
+        hor(f, h, 4, +1);
+        {
+            ProductsT a{};
+            for (int q = 0; q < 9; ++q) a.f[q] = T[q]->data;
+            for (int q = 0; q < 4; ++q) a.nb[q] = h[q]->data;
+            a.o2 = 2 * c->p.omega;
+            a.n2 = c->p.bv0 * c->p.bv0;
+            const int plane = gr.NX * gr.NTH;
+            products_T_kernel<<<dim3(nb(plane, 256), gr.NR), 256, 0, s()>>>(gr, a);
+            count_launch();
+        }
+        // TOFP^T of the nine cotangents at CHOPSET(3) and of W's at CHOPSET(0):
+        // VERFFT(+1)^T and HORFFT(+1)^T carry NX and 2 NTH (m = 0), 4 NTH
+        Field *a10[10], *b10[10];
+        for (int q = 0; q < 9; ++q) {
+            a10[q] = T[q];
+            b10[q] = f[q];
+        }
+        a10[9] = h[2];
+        b10[9] = h[0];
+        hor(a10, b10, 10, -1);
+        a10[9] = h[1];
+        ver(b10, a10, 10, -1);
+        ln_lnx_kernel<<<1, 256, 0, s()>>>(gr, h[1]->data, h[2]->ln);
+        count_launch();
+        {
+            FoldSeg seg[10];
+            int first[11], pads[10];
+            double2* outs[10];
+            for (int q = 0; q < 10; ++q) {
+                seg[q] = FoldSeg{c->adj_fc, a10[q]->data, 0, 0};
+                first[q] = q;
+                pads[q] = q < 9 ? 3 : 0;
+                outs[q] = b10[q]->data;
+            }
+            first[10] = 10;
+            k_fold_bulk(gr, seg, first, 10, outs, c->d.NRCHOPDIM, pads, 0, s());
+        }
+        DerivTArgs d{};
+        for (int q = 0; q < 10; ++q) d.y[q] = b10[q]->data;
+        d.lnw = h[2]->ln;
+        d.psi = pb->data;
+        d.chi = cb->data;
+        d.b = bb->data;
+        d.psi_ln = pb->ln;
+        d.chi_ln = cb->ln;
+        d.b_ln = bb->ln;
+        d.f0 = nx * n2t;
+        d.f1 = 2.0 * nx * n2t;
+        d.pad = 3;
+        k_deriv_T(c->gT, d, s());
+        for (Field* q : f) rel(q);
+        for (Field* q : T) rel(q);
+        for (Field* q : h) rel(q);
+        for (Field* q : {pb, cb, bb}) q->space = MLEGS_FFF;
+    }
+
+    // ab2_step_vjp with the three fields' viscous transposes and updates together
+    void ab2_step_vjp_joint(Field* const st[3], Field* const bar[6], Field* const out[6]) {
+        const double nu[3] = {c->p.nu, c->p.nu, c->p.kappa};
+        Field *wk[3], *fbar[3], *fo[3];
+        for (int q = 0; q < 3; ++q) {
+            wk[q] = tmp();
+            fbar[q] = tmp();
+            fo[q] = tmp();
+        }
+        SolveBatch sb{};
+        sb.n = 3;
+        StepT a{};
+        a.dt = c->p.dt;
+        for (int q = 0; q < 3; ++q) {
+            a.alp[q] = 2 / nu[q] / a.dt;
+            sb.p[q].F = factors(2, a.alp[q])->F;
+            sb.p[q].src = bar[q]->data;
+            sb.p[q].dst = wk[q]->data;
+            a.wk[q] = wk[q]->data;
+            a.wk_ln[q] = wk[q]->ln;
+            a.y_ln[q] = bar[q]->ln;
+            a.x[q] = bar[3 + q]->data;
+            a.x_ln[q] = bar[3 + q]->ln;
+            a.o1[q] = fbar[q]->data;
+            a.o1_ln[q] = fbar[q]->ln;
+            a.o2[q] = out[3 + q]->data;
+            a.o2_ln[q] = out[3 + q]->ln;
+        }
+        k_solve_T_batch(g(), sb, 2, 0, s());
+        dim3 grid = tiles_of(g());
+        grid.z *= 3;
+        step_T_kernel<true><<<grid, dim3(32, 8), 0, s()>>>(g(), a);
+        count_launch();
+        force_vjp(st[0], st[1], st[2], fbar[0], fbar[1], fbar[2], fo[0], fo[1], fo[2]);
+        for (int q = 0; q < 3; ++q) {
+            a.x[q] = fo[q]->data;
+            a.x_ln[q] = fo[q]->ln;
+            a.o1[q] = out[q]->data;
+            a.o1_ln[q] = out[q]->ln;
+        }
+        step_T_kernel<false><<<grid, dim3(32, 8), 0, s()>>>(c->gT, a);
+        count_launch();
+        for (int q = 0; q < 3; ++q) rel({wk[q], fbar[q], fo[q]});
+        for (int q = 0; q < 6; ++q) out[q]->space = MLEGS_FFF;
+    }
+
     // One steady STEP_BOUSSI_AB_CN (VISC%SW = 1) as the map of (psi, chi, b,
     // n_psi, n_chi, n_b) at st (psi, chi, b): cotangents bar[6] -> out[6]
     void ab2_step_vjp(Field* const st[3], Field* const bar[6], Field* const out[6]) {
+        if (c->p.nu != 0.0 && c->p.kappa != 0.0) {
+            ab2_step_vjp_joint(st, bar, out);
+            return;
+        }
         const double dt = c->p.dt;
         const double nu[3] = {c->p.nu, c->p.nu, c->p.kappa};
         Field* abar[3] = {tmp(), tmp(), tmp()};

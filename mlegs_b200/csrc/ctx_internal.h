@@ -129,7 +129,7 @@ struct mlegs_ctx {
             const FoldSeg seg[1] = {{fc_pf, in, mode & 1, scale}};
             const int first[2] = {0, 1};
             double2* const outs[1] = {out};
-            k_fold_bulk(g, seg, first, 1, outs, d.NRCHOPDIM, pad, accumulate, st);
+            k_fold_bulk(g, seg, first, 1, outs, d.NRCHOPDIM, &pad, accumulate, st);
             return;
         }
         k_fold_gemm(g, Wt, wt_rows, in, out, mode, scale, accumulate, pad, st);
@@ -156,7 +156,8 @@ struct mlegs_ctx {
     // on the host and the scratch state of the step and start-up maps
     bool adj_ready = false;
     DevGrid gT{};
-    double* adj_w[3] = {};
+    double* adj_w[4] = {};             // V, D, T; PF times the Gauss weights
+    double* adj_fc = nullptr;          // PF without the weights, chunked for the fold GEMM (RTRAN(+1)^T)
     double* adj_dot = nullptr;
     double adj_n0[3] = {};
     Field* adj_state[6] = {};
@@ -657,7 +658,8 @@ struct mlegs_ctx {
                                 {fc_V, rur, 0, 2}, {fc_D, rup, 1, 1}, {fc_pf, bn, 0, 0}};
         const int first[4] = {0, 3, 5, 6};
         double2* const outs[3] = {chi_, psi_, bn_out};
-        k_fold_bulk(g, seg, first, bn ? 3 : 2, outs, d.NRCHOPDIM, 0, 0, st);
+        const int pads[3] = {0, 0, 0};
+        k_fold_bulk(g, seg, first, bn ? 3 : 2, outs, d.NRCHOPDIM, pads, 0, st);
     }
     // PROJECT(NR, NP, NZ, PSI, W, 0.0) and BN = TOFF(BN) (pad 0) of PFP results of
     // the theta stage, whose PFF images go to pff[0..3]; PSI, W, BNout in FFF.

@@ -83,7 +83,7 @@ __device__ __forceinline__ void chunk_mma(double (&acc)[MTW][4][2], const double
 // stage's data (written before the stage's arrive, read after its wait).
 struct StageInfo {
     int tile;    // tile index ((m * fields + field) * ntx + column tile), -1: no more work
-    int p;       // parity of the K rows
+    int p;       // parity of the K rows (swapped for a segment of mode 1): the accumulators they go to
     int kvalid;  // valid K rows in this chunk (0: a tile without K rows)
     int last;    // 1: the tile's last chunk (the consumers write the tile out)
 };
@@ -135,19 +135,21 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
             int nn = g.NRCHOP + fb_.pad[fi] - m;
             if (nn < 0) nn = 0;
             const int kp0 = (nn + 1) / 2, kp1 = nn / 2;
-            const int nc0 = (kp0 + BK - 1) / BK, nc1 = (kp1 + BK - 1) / BK;
-            const int total = max(1, nc0 + nc1);  // a tile without K rows still hands over one empty chunk
-            const double* pf = g.pf + (size_t)m * ne * g.NRH;
-            const double* a = (const double*)fb_.in[fi] + (size_t)m * g.NRCHOPDIM * ncol;
+            const int nc0 = (kp0 + BK - 1) / BK, nc1 = (kp1 + BK - 1) / BK, ncs = nc0 + nc1;
+            const int s0 = fb_.first[fi], nseg = fb_.first[fi + 1] - s0;
+            const int total = max(1, nseg * ncs);  // a tile without K rows still hands over one empty chunk
             const uint32_t bbytes = (uint32_t)min(BCT, ncol - c0) * 8u;
-            for (int c = 0; c < total; ++c) {
+            for (int cc = 0; cc < total; ++cc) {
                 const int st = seq % NST;
                 if (!acquire(st)) {
                     ok = false;
                     break;
                 }
                 int p = 0, t0 = 0, rows = 0;
-                if (nc0 + nc1 > 0) {
+                const int sl = ncs > 0 ? cc / ncs : 0, sg = s0 + sl, c = cc - sl * ncs;
+                const double* pf = (fb_.pf[sg] ? fb_.pf[sg] : g.pf) + (size_t)m * ne * g.NRH;
+                const double* a = (const double*)fb_.in[sg] + (size_t)m * g.NRCHOPDIM * ncol;
+                if (ncs > 0) {
                     p = c < nc0 ? 0 : 1;
                     t0 = (c - (p ? nc0 : 0)) * BK;
                     rows = min(BK, (p ? kp1 : kp0) - t0);
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
                 double* As = smd + (size_t)st * STG;
                 double* Bs = As + BK * SA;
                 if (lane == 0) {
-                    info[st] = StageInfo{tile, p, rows, c == total - 1 ? 1 : 0};
+                    info[st] = StageInfo{tile, p ^ fb_.mode[sg], rows, cc == total - 1 ? 1 : 0};
                     bar_expect_tx(full + st, (uint32_t)rows * (abytes + bbytes));
                 }
                 __syncwarp();
@@ -253,8 +255,9 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
 // products, mod_legops.f90:2497-2535, 2548-2648) with the same pipeline:
 //   out(n, c) (+)= sum_seg sum_{i < NRH} W_seg(n, i) s_seg(c) F_seg(i, c),
 //   F = x(i) +/- x(NR-1-i), the sign by output-row parity xor the segment's mode.
-// A launch has up to three outputs, each the sum of its own segments: PROJECT's
-// PSI and CHI and the RTRAN(-1) of a fourth field go together, as separate tiles.
+// A launch has up to ten outputs, each the sum of its own segments at its own
+// CHOPSET(pad): PROJECT's PSI and CHI and the RTRAN(-1) of a fourth field, or the
+// ten transposed RTRAN(+1) of a VJP, go together as separate tiles.
 // One CTA tile = (m, output, output parity pr, 64 columns): each of four consumer
 // warps folds its own 16 columns once per chunk and multiplies them by every
 // valid output-row tile (8 rows) of the weights, so the fold work is not
@@ -276,7 +279,8 @@ struct FoldBulkArgs {
     int scale[FOLD_SEGS];           // 0 none, 1 -v, 2 -i m v, 3 i k v, 4 m k v
     int first[FOLD_OUTS + 1];       // output o sums the segments [first[o], first[o + 1])
     double* out[FOLD_OUTS];
-    int nout, wt_rows, pad, accumulate, RB;  // RB: rows per (m, pr) block of the tables
+    int pad[FOLD_OUTS];
+    int nout, wt_rows, accumulate, RB;  // RB: rows per (m, pr) block of the tables
 };
 // The segments' input fields as 2-D tensor maps: columns (2 NXCHOPDIM) x rows (NTCHOPDIM NR).
 struct alignas(64) FoldMaps {
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
         rem -= ou * 2 * ntx;
         pr = rem / ntx;
         c0 = (rem - pr * ntx) * FCT;
-        nn = g.NRCHOP + fa.pad - m;
+        nn = g.NRCHOP + fa.pad[ou] - m;
         if (nn < 0) nn = 0;
         const int nw = min(nn, fa.wt_rows);
         const int rows = (g.NRCHOPDIM - pr + 1) / 2;
@@ -658,7 +662,10 @@ bool b2p_bulk_supported(const DevGrid& g) {
     return (g.NRH % 2) == 0 && RT <= 4 * BNW;
 }
 
-void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
+void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& fin, cudaStream_t s) {
+    B2PBatch f = fin;
+    if (f.first[f.n] == 0)
+        for (int o = 0; o <= f.n; ++o) f.first[o] = o;
     const int RT = (g.NRH + 7) / 8;
     switch ((RT + BNW - 1) / BNW) {
         case 1: launch_b2p_bulk<1>(g, f, s); break;
@@ -705,7 +712,7 @@ bool fold_bulk_supported(const DevGrid& g, int wt_rows) {
 // outs[o] (+)= sum over the segments [first[o], first[o + 1]); the segments' tables
 // come from k_fold_table with the same wt_rows.
 void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nout, double2* const* outs, int wt_rows,
-                 int pad, int accumulate, cudaStream_t s) {
+                 const int* pads, int accumulate, cudaStream_t s) {
     FoldBulkArgs fa{};
     FoldMaps tm;
     memset(&tm, 0, sizeof(tm));
@@ -719,10 +726,12 @@ void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nou
     }
     for (int q = nseg; q < FOLD_SEGS; ++q) tm.x[q] = tm.x[0];
     for (int o = 0; o <= FOLD_OUTS; ++o) fa.first[o] = first[std::min(o, nout)];
-    for (int o = 0; o < nout; ++o) fa.out[o] = (double*)outs[o];
+    for (int o = 0; o < nout; ++o) {
+        fa.out[o] = (double*)outs[o];
+        fa.pad[o] = pads[o];
+    }
     fa.nout = nout;
     fa.wt_rows = wt_rows;
-    fa.pad = pad;
     fa.accumulate = accumulate;
     fa.RB = fold_table_rows(g, wt_rows);
     const int RT = fa.RB / 8;  // output-row tiles of a block

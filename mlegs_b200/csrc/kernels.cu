@@ -948,6 +948,95 @@ void k_deriv(const DevGrid& g, const DerivArgs& a, int which, cudaStream_t s) {
     count_launch();
 }
 
+// PC2VEL^T, PC2VOR^T and GRAD^T of the nine cotangents of a right-hand side's
+// derivative fields, with the transposes' band tables in gT (mod_legops.f90:
+// 1727-1919): rows n < NRCHOPS(m) at pad,
+//   psi = -i m rur - XX^T rup + XX^T(-i k ror) - m k rop + DELSQH (XM^T)^2 (-oz),
+//   chi = XX^T(-i k rur) - m k rup + DELSQH (XM^T)^2 (-uz) + DEL2^T(i m ror + XX^T rop),
+//   b   = XX^T rr - i m rp - i k gz, and W's cotangent at CHOPSET(0) added,
+// with the log-term rows of XXDX, DELSQH and DEL2 folded into the LN outputs.  As
+// separate operators this was 27 launches of a few us each at 96x64x64.
+__device__ __forceinline__ double2 xm2_T_row(const DevGrid& g, int m, const Col& c, int n) {
+    // (XM^T)^2 at row n: the middle of XM^T applied to rows n-1, n, n+1 of XM^T c
+    const double* xm = g.xm + (size_t)m * g.NB * 2;
+    double2 w[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int j = n - 1 + q;
+        w[q] = make_double2(0.0, 0.0);
+        if (j < 0 || j >= c.nn) continue;
+        const double2 a = c.at(j - 1), b = c.at(j + 1);
+        double2 v = c.at(j);
+        if (j >= 1) v = cadd(v, cscale(a, xm[j * 2]));
+        if (j + 1 < c.nn) v = cadd(v, cscale(b, xm[j * 2 + 1]));
+        w[q] = v;
+    }
+    double2 v = w[1];
+    if (n >= 1) v = cadd(v, cscale(w[0], xm[n * 2]));
+    if (n + 1 < c.nn) v = cadd(v, cscale(w[2], xm[n * 2 + 1]));
+    return v;
+}
+__global__ void __launch_bounds__(256) deriv_T_kernel(DevGrid g, const __grid_constant__ DerivTArgs A) {
+    size_t t;
+    int m, n, k;
+    if (!tile_index(g, t, m, n, k)) return;
+    const double f = m == 0 ? A.f0 : A.f1, mv = (double)m, kv = g.ak[k];
+    const int nn = nrchops(g, m, A.pad);
+    double2 ps = make_double2(0.0, 0.0), ch = ps, bb = ps;
+    if (n < nn) {
+        Col c[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) c[q] = column(g, A.y[q], m, k, A.pad);
+        const double lap = (m == 0 && n == 0 && k == 0) ? 0.0 : g.lap[m + n];
+        const double2 xrur = xxdx_row(g, m, k, c[0], n, 0.0), xrup = xxdx_row(g, m, k, c[1], n, 0.0),
+                      xror = xxdx_row(g, m, k, c[3], n, 0.0);
+        ps = csub(cmuli(c[0].at(n), -mv), xrup);
+        ps = cadd(ps, cmuli(xror, -kv));
+        ps = csub(ps, cscale(c[4].at(n), mv * kv));
+        ps = csub(ps, cscale(xm2_T_row(g, m, c[5], n), lap));
+        // w = i m ror + XX^T rop at rows n-2 .. n+2, DEL2^T of it
+        const double* tb = g.del2h + ((size_t)m * g.NB + n) * 5;
+        double2 d = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int e = 0; e < 5; ++e) {
+            const int j = n + e - 2;
+            if (j < 0 || j >= nn) continue;
+            const double2 w = cadd(cmuli(c[3].at(j), mv), xxdx_row(g, m, k, c[4], j, 0.0));
+            d = cadd(d, cscale(w, e == 2 ? tb[e] - kv * kv : tb[e]));
+        }
+        ch = csub(cmuli(xrur, -kv), cscale(c[1].at(n), mv * kv));
+        ch = csub(ch, cscale(xm2_T_row(g, m, c[2], n), lap));
+        ch = cadd(ch, d);
+        bb = cadd(xxdx_row(g, m, k, c[6], n, 0.0), cadd(cmuli(c[7].at(n), -mv), cmuli(c[8].at(n), -kv)));
+    }
+    if (n < nrchops(g, m, 0)) bb = cadd(bb, A.y[9][t]);
+    A.psi[t] = cscale(ps, f);
+    A.chi[t] = cscale(ch, f);
+    A.b[t] = cscale(bb, f);
+    if (m == 0 && n == 0 && k == 0) {
+        // the LN cotangents: log-term rows of XXDX (rup, rr), DELSQH (of (XM^T)^2 oz and
+        // uz at row 0) and DEL2 (rows 0..2 of w)
+        Col c[9];
+        for (int q = 0; q < 9; ++q) c[q] = column(g, A.y[q], 0, 0, A.pad);
+        const double i0 = 1.0 / g.norm0[0], i1 = 1.0 / g.norm0[1], i2 = 1.0 / g.norm0[2], ie = 1.0 / g.ELL2;
+        double lp = -(c[1].at(0).x * i0 + c[1].at(1).x * i1);
+        double lc = 0.0;
+        if (nn > 0) {
+            lp -= xm2_T_row(g, 0, c[5], 0).x * ie * i0;
+            lc -= xm2_T_row(g, 0, c[2], 0).x * ie * i0;
+        }
+        const double cf[3] = {4.0 / 3 * i0 * ie, -2.0 * i1 * ie, 2.0 / 3 * i2 * ie};
+        for (int j = 0; j < 3 && j < nn; ++j) lc += cf[j] * xxdx_row(g, 0, 0, c[4], j, 0.0).x;
+        *A.psi_ln = f * lp;
+        *A.chi_ln = f * lc;
+        *A.b_ln = f * (c[6].at(0).x * i0 + c[6].at(1).x * i1 + *A.lnw);
+    }
+}
+void k_deriv_T(const DevGrid& gT, const DerivTArgs& a, cudaStream_t s) {
+    deriv_T_kernel<<<fff_tiles(gT), dim3(32, 8), 0, s>>>(gT, a);
+    count_launch();
+}
+
 // The coefficient update of STEP_BOUSSI_ETDAB_CN (mod_march.f90:811-901) from
 // the projected nonlinear terms to the new state, in one pass per FFF entry:
 //   HYPERV of the nonlinear terms (1352-1416, at TF = 1, chopped at pad 0;

@@ -110,14 +110,19 @@ void k_split_fold(const DevGrid& g, int S, const uint8_t* img, const int* eA, in
 void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
 // RTRAN(+1) of up to ten fields, each at its own CHOPSET(pad), in one launch when
 // the bulk-copy form runs (one launch per field otherwise).  ln: the fields' LN
-// slots (null: no log term).
+// slots (null: no log term).  The adjoint's form: output o sums the segments
+// [first[o], first[o + 1]) with weights pf[s] (rows as PF's) in PF's place; mode 1
+// negates a segment's mirror half (the transpose of an OE fold).  Bulk-copy form only.
 constexpr int BATCH = 10;
 struct B2PBatch {
     const double2* in[BATCH];
+    const double* pf[BATCH];   // null: PF
+    int mode[BATCH];
+    int first[BATCH + 1];      // all zero: segment o is output o
     double2* out[BATCH];
     const double* ln[BATCH];
     int pad[BATCH];
-    int n;
+    int n;                     // outputs
 };
 void k_rtran_b2p_batch(const DevGrid& g, const B2PBatch& f, cudaStream_t s);
 // Fold GEMM arguments (gemm_dmma.cu): RTRAN(-1) and PROJECT's five EOMUL/OEMUL
@@ -200,7 +205,7 @@ int bulk_gemm_error(bool reset);
 // tables re-laid per (m, parity, 16-row chunk) by k_fold_table (rows n < wt_rows of
 // W[m][src_rows][NRH], times w_i when use_w), then k_fold_bulk: output o sums the
 // segments [first[o], first[o + 1]) (mode / scale as in FoldArgs).
-constexpr int FOLD_SEGS = 6, FOLD_OUTS = 3;
+constexpr int FOLD_SEGS = 10, FOLD_OUTS = 10;
 struct FoldSeg {
     const double* wc;
     const double2* x;
@@ -212,7 +217,7 @@ void k_fold_table(const DevGrid& g, const double* W, int src_rows, int wt_rows, 
                   cudaStream_t s);
 bool fold_bulk_supported(const DevGrid& g, int wt_rows);
 void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nout, double2* const* outs, int wt_rows,
-                 int pad, int accumulate, cudaStream_t s);
+                 const int* pads, int accumulate, cudaStream_t s);
 // FP64 tensor-path (mma.sync m8n8k4.f64) forms used by k_rtran_b2p / k_fold_gemm when supported.
 bool dmma_supported(const DevGrid& g);
 void k_rtran_b2p_dmma(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
@@ -313,8 +318,10 @@ void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F, 
 void k_solve_factored(const DevGrid& g, const double* F, const double2* src, double2* dst, double* ln_out, int kind,
                       int has_ln, double ln_in, int pad, int farfield, cudaStream_t s, const double* ln_rhs = nullptr,
                       double ln_scale = 0.0);
-// The transposed systems (adjoint), in place: kind 0 IDEL2LN, 2 IHELM.
+// The transposed systems (adjoint): kind 0 IDEL2LN, 2 IHELM.  In place, rows from
+// the system size on left as they are; the batch form writes them as zero.
 void k_solve_T(const DevGrid& g, const double* F, double2* y, int kind, int pad, cudaStream_t s);
+void k_solve_T_batch(const DevGrid& g, const SolveBatch& b, int kind, int pad, cudaStream_t s);
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
                             int farfield, cudaStream_t s);
 // The AB2 update with VISC2's right-hand side for up to three fields (kernels.cu).
@@ -338,6 +345,20 @@ void k_ab2_visc_rhs(const DevGrid& g, const Ab2Args& a, cudaStream_t s);
 // `msg` receives the reason.
 extern const size_t kStaticSolveBytes;
 int static_solve_scratch(int device, size_t need_doubles, double** out, char* msg, size_t msg_len);
+
+// The VJP's passes (kernels.cu, adjoint.cu).
+// PC2VEL^T + PC2VOR^T of cotangents y[0..5] and GRAD^T of y[6..8] at CHOPSET(pad) plus
+// y[9] (at CHOPSET(0)) -> psi, chi, b cotangents; every input is times f0 (m = 0) or
+// f1 (m > 0); lnw: LN of y[9] before that factor.  gT: the grid with transposed band tables.
+struct DerivTArgs {
+    const double2* y[10];
+    const double* lnw;
+    double2 *psi, *chi, *b;
+    double *psi_ln, *chi_ln, *b_ln;
+    double f0, f1;
+    int pad;
+};
+void k_deriv_T(const DevGrid& gT, const DerivTArgs& a, cudaStream_t s);
 
 // Pointwise physics in PPP.
 void k_force_pointwise(const DevGrid& g, double2* rur, double2* rup, double2* uz, double2* ror,

@@ -353,6 +353,7 @@ struct SolveForm {
     int kind, has_ln;
     double ln_in;
     int pad, farfield;
+    int keep_tail;  // transposed systems: rows from the system size on are not written
 };
 // A block's shared memory: the ring, the tables of the m = 0 tails (at1 [R],
 // xm [R][2]), the column Xs [R][16].
@@ -440,8 +441,8 @@ __device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, co
     }
 }
 
-// HB: half-bandwidth; TR: the transposed system U^T z = y, L^T x = z (rows from
-// the system size on left as they are), else L y = b, U x = y with the tails.
+// HB: half-bandwidth; TR: the transposed system U^T z = y, L^T x = z, else
+// L y = b, U x = y with the tails.
 // Returns the rows to write, -1 when a wait ran out.
 template <int HB, bool TR, bool XG>
 __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveForm& fo, int m, int k0, int nsb,
@@ -683,7 +684,7 @@ __device__ __forceinline__ void band_solve(const DevGrid& g, const SolveItem& p,
     __syncthreads();
     const int rows_out = rows_sh;
     if (rows_out < 0) return;
-    const int end = TR ? rows_out : g.NRCHOPDIM, q = threadIdx.x & 15;
+    const int end = fo.keep_tail ? rows_out : g.NRCHOPDIM, q = threadIdx.x & 15;
     double2* dst = p.dst + base + q;
     if (q >= nsb) return;
 #pragma unroll 4
@@ -765,7 +766,7 @@ __global__ void __launch_bounds__(64) grouped_solve_kernel(const GroupSolve* __r
         else hi = mid - 1;
     }
     const GroupSolve& P = pr[lo];
-    solve_block<false, false>(P.g, P.it, SolveForm{P.kind, P.has_ln, P.ln_in, P.pad, P.farfield}, b - P.first);
+    solve_block<false, false>(P.g, P.it, SolveForm{P.kind, P.has_ln, P.ln_in, P.pad, P.farfield, 0}, b - P.first);
 }
 
 constexpr size_t SOLVE_SMEM_MAX = 220 * 1024;
@@ -797,7 +798,7 @@ void launch_solve(const DevGrid& g, const SolveBatch& b, const SolveForm& fo, cu
 
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
                             int farfield, cudaStream_t s) {
-    launch_solve<false>(g, b, SolveForm{kind, has_ln, ln_in, pad, farfield}, s);
+    launch_solve<false>(g, b, SolveForm{kind, has_ln, ln_in, pad, farfield, 0}, s);
 }
 
 void k_solve_factored(const DevGrid& g, const double* F, const double2* src, double2* dst, double* ln_out, int kind,
@@ -820,7 +821,11 @@ void k_solve_T(const DevGrid& g, const double* F, double2* y, int kind, int pad,
     b.p[0].F = F;
     b.p[0].src = y;
     b.p[0].dst = y;
-    launch_solve<true>(g, b, SolveForm{kind, 0, 0.0, pad, 0}, s);
+    launch_solve<true>(g, b, SolveForm{kind, 0, 0.0, pad, 0, 1}, s);
+}
+
+void k_solve_T_batch(const DevGrid& g, const SolveBatch& b, int kind, int pad, cudaStream_t s) {
+    launch_solve<true>(g, b, SolveForm{kind, 0, 0.0, pad, 0, 0}, s);
 }
 
 int group_solve_blocks(const GroupSolve& p) { return FactorTable(p.g).nkb * p.g.NTCHOPDIM; }
