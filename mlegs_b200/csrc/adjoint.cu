@@ -1578,8 +1578,31 @@ int mlegs_field_device_copy(mlegs_ctx* ctx, mlegs_field* f, int to_field, int sp
     return guard(ctx, [&] {
         if (!dev) throw ApiError(MLEGS_ERR_ARG, "mlegs_field_device_copy: null device buffer");
         Field* fd = F(f);
+        if (to_field && (space < 0 || space > 3))
+            throw ApiError(MLEGS_ERR_TRANSFORM, "mlegs_field_device_copy: bad space");
+        // this device's memory: data and LN in one launch (two copies cost twice the
+        // gaps around them); anything else (unaligned, host or another device's) by
+        // the runtime's copies
+        auto local = [&](const void* q, size_t align) {
+            if (!q) return true;
+            cudaPointerAttributes a{};
+            if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            return a.type == cudaMemoryTypeDevice && a.device == ctx->dev && ((uintptr_t)q & (align - 1)) == 0;
+        };
+        if (local(dev, 16) && local(ln_dev, 8)) {
+            double2* d = (double2*)dev;
+            if (to_field) {
+                k_copy_ln(fd->data, d, ctx->d.elems(space), fd->ln, ln_dev, ctx->s);
+                fd->space = space;
+            } else {
+                k_copy_ln(d, fd->data, ctx->d.elems(fd->space), ln_dev, fd->ln, ctx->s);
+            }
+            return;
+        }
         if (to_field) {
-            if (space < 0 || space > 3) throw ApiError(MLEGS_ERR_TRANSFORM, "mlegs_field_device_copy: bad space");
             CK(cudaMemcpyAsync(fd->data, dev, ctx->d.elems(space) * sizeof(double2), cudaMemcpyDeviceToDevice,
                                ctx->s));
             fd->space = space;

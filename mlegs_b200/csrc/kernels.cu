@@ -45,10 +45,11 @@ void k_copy(double2* dst, const double2* src, size_t n, cudaStream_t s) {
     count_launch();
 }
 
-// dst = src over n entries and the field's LN slot (thread 0), in one launch.
+// dst = src over n entries and the field's LN slot (thread 0), in one launch; a null
+// source LN is 0, a null destination LN is left out.
 __global__ void copy_ln_kernel(double2* d, const double2* a, size_t n, double* dln, const double* aln) {
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t == 0) *dln = *aln;
+    if (t == 0 && dln) *dln = aln ? *aln : 0.0;
     if (t < n) d[t] = a[t];
 }
 void k_copy_ln(double2* dst, const double2* src, size_t n, double* dln, const double* sln, cudaStream_t s) {
