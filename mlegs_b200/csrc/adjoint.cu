@@ -485,10 +485,16 @@ struct Adj {
             pad_rows_kernel<<<nb(np, 256), 256, 0, c->s>>>(c->g, W[q], c->adj_w[q]);
             count_launch();
         }
-        if (joint()) {
-            c->adj_w[3] = dalloc<double>(np);
-            pf_w_kernel<<<nb(np, 256), 256, 0, c->s>>>(c->g, c->adj_w[3]);
+        if (c->g.pft) {
+            double* pfw = dalloc<double>(np);
+            pf_w_kernel<<<nb(np, 256), 256, 0, c->s>>>(c->g, pfw);
             count_launch();
+            for (int q = 0; q < 4; ++q) {
+                c->adj_wt[q] = dalloc<double>(b2p_table_doubles(c->g));
+                k_b2p_table(c->g, q < 3 ? c->adj_w[q] : pfw, c->adj_wt[q], c->s);
+            }
+        }
+        if (joint()) {
             c->adj_fc = dalloc<double>(fold_table_doubles(c->g, d.NRCHOPDIM));
             k_fold_table(c->g, c->pf, d.NRCHOPDIM + 1, d.NRCHOPDIM, 0, c->adj_fc, c->s);
         }
@@ -502,7 +508,7 @@ struct Adj {
     bool joint() const {
         const DevGrid& g = c->g;
         auto fft = [](int v) { return v >= 16 && v <= 512; };
-        return b2p_bulk_supported(g) && fold_bulk_supported(g, g.NRCHOPDIM) && fft(g.NX) && fft(g.NTH);
+        return g.pft && fold_bulk_supported(g, g.NRCHOPDIM) && fft(g.NX) && fft(g.NTH);
     }
 
     // Temporaries; the pool grows on demand (outside capture), recorded in the
@@ -772,6 +778,7 @@ struct Adj {
     void fold_T(int w, const Field* z, Field* out, int mode, bool first, Field* work) {
         DevGrid gw = g();
         gw.pf = c->adj_w[w];
+        gw.pft = c->adj_wt[w];
         const size_t n = c->d.pff();
         if (mode == 0 && first) {
             k_rtran_b2p(gw, z->data, out->data, nullptr, 0, s());
@@ -961,7 +968,7 @@ struct Adj {
             const int w[6] = {1, 0, 1, 0, 2, 3};  // D, V, D, V, T, PF w
             for (int q = 0; q < 6; ++q) {
                 b.in[q] = f[1 + q]->data;
-                b.pf[q] = c->adj_w[w[q]];
+                b.pf[q] = c->adj_wt[w[q]];
                 b.mode[q] = mode[q];
             }
             for (int o = 0; o < 4; ++o) b.out[o] = h[o]->data;

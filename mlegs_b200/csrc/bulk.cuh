@@ -50,5 +50,13 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
         : "memory");
 }
 
+// 16-byte copies of the calling thread, and its arrival once those so far have landed.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa_of(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy16_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sa_of(bar)) : "memory");
+}
+
 }  // namespace bulk
 }  // namespace mlegs

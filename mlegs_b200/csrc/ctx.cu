@@ -256,6 +256,11 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     g.del2h = tb_del2h;
     g.NB = NB;
     g.lap = lap;
+    if (b2p_bulk_supported(g)) {
+        double* tab = dalloc<double>(b2p_table_doubles(g));
+        k_b2p_table(g, pf, tab, s);
+        g.pft = tab;
+    }
 
     // --- PROJECT weights (device, from PF)
     size_t vsz = (size_t)d.NTCHOPDIM * d.NRCHOPDIM * d.NRH;

@@ -156,7 +156,8 @@ struct mlegs_ctx {
     // on the host and the scratch state of the step and start-up maps
     bool adj_ready = false;
     DevGrid gT{};
-    double* adj_w[4] = {};             // V, D, T; PF times the Gauss weights
+    double* adj_w[3] = {};             // V, D, T
+    double* adj_wt[4] = {};            // weight tables of V, D, T and PF times the Gauss weights
     double* adj_fc = nullptr;          // PF without the weights, chunked for the fold GEMM (RTRAN(+1)^T)
     double* adj_dot = nullptr;
     double adj_n0[3] = {};

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(128) rtran_b2p_kernel(DevGrid g, const double*
 }
 
 void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
-    if (b2p_bulk_supported(g)) {
+    if (g.pft) {
         B2PBatch f{};
         f.n = 1;
         f.in[0] = a;
@@ -123,7 +123,7 @@ void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* l
 }
 
 void k_rtran_b2p_batch(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
-    if (b2p_bulk_supported(g)) {
+    if (g.pft) {
         k_rtran_b2p_bulk(g, f, s);
         return;
     }

@@ -10,17 +10,21 @@
 // computes a 32-column tile of one m of one field for all NRH output rows:
 //   warps 0..3   consumers: m8n8k4 FP64 MMAs over their MTW m-tiles x four
 //                n-tiles, both parities' accumulators in registers;
-//   warp 4       producer: per 16-row K chunk, one 1-D bulk copy
-//                (cp.async.bulk) per PF row and per field row into a ring of
-//                NST shared-memory stages, completing on the stage's
+//   warp 4       producer: per 16-row K chunk, one bulk copy (cp.async.bulk) of
+//                the weights and 16-byte cp.async copies of the field rows into
+//                a ring of NST shared-memory stages, completing on the stage's
 //                mbarrier.
+// The weights come from a table with PF's rows laid out per (m, parity, chunk)
+// at the stage's row stride, zero past NRH (any NRH), so a chunk is one
+// contiguous piece.  A bulk copy costs its warp some 80 cycles to issue: with one
+// per weight row and field row (32 a chunk) the producer took as long as the
+// three CTAs' MMAs of a chunk and the tensor pipe stood at 57%.
 // The consumers' fragment loads are shared-memory loads at fixed offsets from
 // a per-thread base (row strides = 8 mod 16 doubles: the minimum two
-// wavefronts per load); no address arithmetic runs per MMA.  K rows past the
-// parity's extent are not copied; their B fragments are zeroed in registers
-// (the stale A rows there are finite: the ring starts zeroed).  Every
-// mbarrier wait is bounded (about a second); on a timeout the CTA raises the
-// module's error word and its roles stop, the producer first waiting (again
+// wavefronts per load); no address arithmetic runs per MMA.  Field rows past the
+// parity's extent are not copied; their B fragments are zeroed in registers.
+// Every mbarrier wait is bounded (about a second); on a timeout the CTA raises
+// the module's error word and its roles stop, the producer first waiting (again
 // bounded) for the copies it issued.
 #include "bulk.cuh"
 #include "mlegs_internal.h"
@@ -88,10 +92,15 @@ struct StageInfo {
     int last;    // 1: the tile's last chunk (the consumers write the tile out)
 };
 
+// 16-row chunks of a parity's weight rows in the table.
+__host__ __device__ inline int b2p_chunks(const DevGrid& g) { return ((g.NRCHOPDIM + 1) / 2 + BK - 1) / BK; }
+// Weight row stride (doubles) for m-tiles per warp MTW, = 8 mod 16.
+__host__ __device__ constexpr int b2p_stride(int mtw) { return BNW * mtw * 8 + (((BNW * mtw) & 1) ? 0 : 8); }
+
 template <int MTW, int NST>
 __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
     b2p_bulk_kernel(DevGrid g, const __grid_constant__ B2PBatch fb_) {
-    constexpr int SA = BNW * MTW * 8 + (((BNW * MTW) & 1) ? 0 : 8);  // PF row stride, = 8 mod 16
+    constexpr int SA = b2p_stride(MTW);
     constexpr int STG = BK * SA + BK * BSB;                          // doubles per stage
     extern __shared__ __align__(128) double smd[];
     uint64_t* full = (uint64_t*)(smd + NST * STG);
@@ -101,12 +110,10 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ncol = 2 * g.NXCHOPDIM;
     const int ntx = (ncol + BCT - 1) / BCT, ntf = ntx * fb_.n, ntiles = ntf * g.NTCHOPDIM;
-    // zeroed ring (rows that are never copied stay finite), barriers
-    for (int e = tid; e < NST * STG; e += blockDim.x) smd[e] = 0.0;
     if (tid == 0) {
         abort_f = 0;
         for (int st = 0; st < NST; ++st) {
-            bar_init(full + st, 1);
+            bar_init(full + st, 33);  // the bulk copy and the producer's 32 lanes
             bar_init(empty + st, BNW);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -119,8 +126,7 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
         // The CTA's tiles are blockIdx.x, + gridDim.x, ... (m ascending over all
         // fields: the largest K first); their chunks form one stream through the
         // ring, so the next tile's rows arrive while the current one is finishing.
-        const int ne = g.NRCHOPDIM + 1;
-        const uint32_t abytes = (uint32_t)g.NRH * 8u;
+        const int nchp = b2p_chunks(g);
         int seq = 0;  // chunks handed over so far
         bool ok = true;
         auto acquire = [&](int st) -> bool {  // the stage's previous contents consumed
@@ -138,36 +144,42 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
             const int nc0 = (kp0 + BK - 1) / BK, nc1 = (kp1 + BK - 1) / BK, ncs = nc0 + nc1;
             const int s0 = fb_.first[fi], nseg = fb_.first[fi + 1] - s0;
             const int total = max(1, nseg * ncs);  // a tile without K rows still hands over one empty chunk
-            const uint32_t bbytes = (uint32_t)min(BCT, ncol - c0) * 8u;
             for (int cc = 0; cc < total; ++cc) {
                 const int st = seq % NST;
                 if (!acquire(st)) {
                     ok = false;
                     break;
                 }
-                int p = 0, t0 = 0, rows = 0;
+                int p = 0, ch = 0, rows = 0;
                 const int sl = ncs > 0 ? cc / ncs : 0, sg = s0 + sl, c = cc - sl * ncs;
-                const double* pf = (fb_.pf[sg] ? fb_.pf[sg] : g.pf) + (size_t)m * ne * g.NRH;
-                const double* a = (const double*)fb_.in[sg] + (size_t)m * g.NRCHOPDIM * ncol;
                 if (ncs > 0) {
                     p = c < nc0 ? 0 : 1;
-                    t0 = (c - (p ? nc0 : 0)) * BK;
-                    rows = min(BK, (p ? kp1 : kp0) - t0);
+                    ch = c - (p ? nc0 : 0);
+                    rows = min(BK, (p ? kp1 : kp0) - ch * BK);
                 }
                 double* As = smd + (size_t)st * STG;
                 double* Bs = As + BK * SA;
                 if (lane == 0) {
                     info[st] = StageInfo{tile, p ^ fb_.mode[sg], rows, cc == total - 1 ? 1 : 0};
-                    bar_expect_tx(full + st, (uint32_t)rows * (abytes + bbytes));
+                    // the weight rows of the k-steps in use
+                    const uint32_t abytes = (uint32_t)((rows + 3) / 4 * 4) * SA * 8u;
+                    bar_expect_tx(full + st, abytes);
+                    if (abytes)
+                        bulk_copy(As, (fb_.pf[sg] ? fb_.pf[sg] : g.pft) + (((size_t)m * 2 + p) * nchp + ch) * BK * SA,
+                                  abytes, full + st);
                 }
-                __syncwarp();
-                if (lane < rows) {
-                    const int n = 2 * (t0 + lane) + p;
-                    bulk_copy(As + lane * SA, pf + (size_t)n * g.NRH, abytes, full + st);
-                } else if (lane >= 16 && lane - 16 < rows) {
-                    const int n = 2 * (t0 + lane - 16) + p;
-                    bulk_copy(Bs + (lane - 16) * BSB, a + (size_t)n * ncol + c0, bbytes, full + st);
+                // field rows n = 2 (16 ch + r) + p: 16 lanes a row
+                const int col = c0 + 2 * (lane & 15);
+                if (col < ncol) {
+                    const double* a = (const double*)fb_.in[sg] + (size_t)m * g.NRCHOPDIM * ncol + col;
+#pragma unroll
+                    for (int r = 0; r < BK; r += 2) {
+                        const int rr = r + (lane >> 4);
+                        if (rr < rows)
+                            copy16_async(Bs + rr * BSB + 2 * (lane & 15), a + (size_t)(2 * (ch * BK + rr) + p) * ncol);
+                    }
                 }
+                copy16_arrive(full + st);
                 ++seq;
             }
         }
@@ -178,6 +190,7 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
                     info[st] = StageInfo{-1, 0, 0, 0};
                     bar_expect_tx(full + st, 0u);
                 }
+                copy16_arrive(full + st);
                 ++seq;
             } else {
                 ok = false;
@@ -560,7 +573,7 @@ int bulk_sm_count() {
 
 template <int MTW, int NST>
 void launch_b2p_bulk_n(const DevGrid& g, const B2PBatch& f, int per_sm, cudaStream_t s) {
-    constexpr int SA = BNW * MTW * 8 + (((BNW * MTW) & 1) ? 0 : 8);
+    constexpr int SA = b2p_stride(MTW);
     constexpr size_t smem = (size_t)NST * (BK * SA + BK * BSB) * sizeof(double) + 2 * NST * sizeof(uint64_t);
     static bool attr = false;
     if (!attr) {
@@ -657,17 +670,36 @@ double k_dmma_peak(double* out, cudaStream_t s) {
     return dmma_peak_flops();
 }
 
-bool b2p_bulk_supported(const DevGrid& g) {
-    const int RT = (g.NRH + 7) / 8;
-    return (g.NRH % 2) == 0 && RT <= 4 * BNW;
+bool b2p_bulk_supported(const DevGrid& g) { return (g.NRH + 7) / 8 <= 4 * BNW; }
+
+// The RTRAN(+1) weight table: W's rows n = 2 (16 ch + kk) + p of parity p, chunk ch
+// at [m][p][ch][kk][SA], zero past NRH and NRCHOPDIM.
+__global__ void b2p_table_kernel(DevGrid g, const double* __restrict__ W, int SA, double* __restrict__ T) {
+    const int nchp = b2p_chunks(g);
+    const size_t total = (size_t)g.NTCHOPDIM * 2 * nchp * BK * SA;
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    const int i = (int)(t % SA);
+    const size_t q = t / SA;
+    const int kk = (int)(q % (nchp * BK)), p = (int)(q / (nchp * BK) % 2), m = (int)(q / (nchp * BK) / 2);
+    const int n = 2 * kk + p;
+    T[t] = i < g.NRH && n < g.NRCHOPDIM ? W[((size_t)m * (g.NRCHOPDIM + 1) + n) * g.NRH + i] : 0.0;
+}
+static int b2p_mtw(const DevGrid& g) { return std::max(1, ((g.NRH + 7) / 8 + BNW - 1) / BNW); }
+size_t b2p_table_doubles(const DevGrid& g) {
+    return (size_t)g.NTCHOPDIM * 2 * b2p_chunks(g) * BK * b2p_stride(b2p_mtw(g));
+}
+void k_b2p_table(const DevGrid& g, const double* W, double* T, cudaStream_t s) {
+    const size_t n = b2p_table_doubles(g);
+    b2p_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, W, b2p_stride(b2p_mtw(g)), T);
+    count_launch();
 }
 
 void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& fin, cudaStream_t s) {
     B2PBatch f = fin;
     if (f.first[f.n] == 0)
         for (int o = 0; o <= f.n; ++o) f.first[o] = o;
-    const int RT = (g.NRH + 7) / 8;
-    switch ((RT + BNW - 1) / BNW) {
+    switch (b2p_mtw(g)) {
         case 1: launch_b2p_bulk<1>(g, f, s); break;
         case 2: launch_b2p_bulk<2>(g, f, s); break;
         case 3: launch_b2p_bulk<3>(g, f, s); break;

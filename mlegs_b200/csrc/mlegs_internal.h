@@ -64,6 +64,7 @@ struct DevGrid {
     const double* xm;       // [NTCHOPDIM][NB][2]  (sub, super)     diag = 1
     const double* del2h;    // [NTCHOPDIM][NB][5]
     int NB;                 // NRCHOPDIM + 2
+    const double* pft;      // PF as the bulk-copy RTRAN(+1)'s weight table (null when that form is not used)
     const double* lap;      // -N (N + 1) / ELL2 by degree N = m + n (DELSQH's diagonal)
     int* err;               // the context's error word: set to 1 when a bounded wait runs out
 };
@@ -111,7 +112,7 @@ void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* l
 // RTRAN(+1) of up to ten fields, each at its own CHOPSET(pad), in one launch when
 // the bulk-copy form runs (one launch per field otherwise).  ln: the fields' LN
 // slots (null: no log term).  The adjoint's form: output o sums the segments
-// [first[o], first[o + 1]) with weights pf[s] (rows as PF's) in PF's place; mode 1
+// [first[o], first[o + 1]) with weight tables pf[s] (k_b2p_table) in PF's place; mode 1
 // negates a segment's mirror half (the transpose of an OE fold).  Bulk-copy form only.
 constexpr int BATCH = 10;
 struct B2PBatch {
@@ -200,6 +201,9 @@ bool b2p_bulk_supported(const DevGrid& g);
 double k_dmma_peak(double* out, cudaStream_t s);
 double dmma_peak_flops();
 void k_rtran_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s);
+// Its weight table from W[m][NRCHOPDIM + 1][NRH].
+size_t b2p_table_doubles(const DevGrid& g);
+void k_b2p_table(const DevGrid& g, const double* W, double* T, cudaStream_t s);
 int bulk_gemm_error(bool reset);
 // Fold GEMMs (RTRAN(-1), PROJECT's products) on the same pipeline: weight
 // tables re-laid per (m, parity, 16-row chunk) by k_fold_table (rows n < wt_rows of

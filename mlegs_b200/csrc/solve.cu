@@ -368,14 +368,6 @@ struct SolveShared {
     int* stop;        // a wait ran out
 };
 
-__device__ __forceinline__ void cpa16(void* d, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src)
-                 : "memory");
-}
-// arrival once this thread's cp.async copies so far have landed
-__device__ __forceinline__ void cpa_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sa_of(bar)) : "memory");
-}
 // A whole warp's wait; false (for all lanes) when it runs out or the other warp stopped.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, int phase, int* stop) {
     return __all_sync(0xffffffffu, bar_wait(bar, (uint32_t)(phase & 1))) && !*(volatile int*)stop;
@@ -404,8 +396,8 @@ __device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, co
     const bool staged = TR && HB == 3;
     if (staged && !XG) {
         if (q < nsb)
-            for (int r = r0; r < nn; r += 2) cpa16(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
-        cpa_arrive(sh.whole);
+            for (int r = r0; r < nn; r += 2) copy16_async(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
+        copy16_arrive(sh.whole);
     }
     int c = 0;
     bool ok = true;
@@ -427,10 +419,10 @@ __device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, co
 #pragma unroll
             for (int i = 0; i < SCH / 2; ++i) {
                 const int r = lo + r0 + 2 * i;
-                if (r < lo + rows) cpa16(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
+                if (r < lo + rows) copy16_async(sh.Xs + r * 16 + q, src + (size_t)r * NK + q);
             }
         }
-        cpa_arrive(sh.full + st);
+        copy16_arrive(sh.full + st);
     }
     if (!ok) {  // the copies in flight land before the CTA ends
         if (lane == 0) {
