@@ -433,8 +433,9 @@ __device__ __forceinline__ void grp_inverse5(const double2* __restrict__ src, bo
         for (int m = t; m < mlim; m += N2) L[m] = src[m];
     __syncwarp();
     double2 v[N1], o[N1];
-    auto pack = [&](int m, double2 w) {  // w = e^{+i pi m/N}
-        const int mc = N - m;
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) {
+        const int m = t + N2 * n1, mc = N - m;
         double2 xm = make_double2(0.0, 0.0), xc = make_double2(0.0, 0.0);
         if (valid) {
             if (m < mlim) xm = L[m];
@@ -442,16 +443,9 @@ __device__ __forceinline__ void grp_inverse5(const double2* __restrict__ src, bo
         }
         if (m == 0) xm.y = 0.0;
         xc = fft4::conj(xc);
-        const double2 sm = make_double2(xm.x + xc.x, xm.y + xc.y), d = make_double2(xm.x - xc.x, xm.y - xc.y);
-        const double2 ed = fft4::cmul(w, d);
-        return make_double2(sm.x - ed.y, sm.y + ed.x);
-    };
-#pragma unroll
-    for (int n1 = 0; n1 < N1 / 2; ++n1) {  // m and m + N/2, whose twiddle is i times m's: one table read for both
-        const int m = t + N2 * n1;
-        const double2 w = fft4::conj(twh[m]);
-        v[n1] = pack(m, w);
-        v[n1 + N1 / 2] = pack(m + N / 2, make_double2(-w.y, w.x));
+        double2 sm = make_double2(xm.x + xc.x, xm.y + xc.y), d = make_double2(xm.x - xc.x, xm.y - xc.y);
+        double2 ed = fft4::cmul(fft4::conj(twh[m]), d);  // e^{+i pi m/N} d
+        v[n1] = make_double2(sm.x - ed.y, sm.y + ed.x);
     }
     __syncwarp();
     fft4::line_fft_inplace<N1, N2, +1>(v, L, tw, t, o);
@@ -486,23 +480,14 @@ __device__ __forceinline__ void grp_forward5(double2* L, bool valid, double2* __
     for (int q = 0; q < N1; ++q) L[fft4::out_index<N1, N2>(t, q)] = o[q];  // Z_k, natural order
     __syncwarp();
     const double sc = 1.0 / (2.0 * N);
-    const int mlim = md < ntchop ? md : ntchop;
-    auto put = [&](int m, double2 w) {  // w = e^{-i pi m/N}
-        const double2 zm = L[m], zc = fft4::conj(L[(N - m) & (N - 1)]);
-        const double2 sm = make_double2(zm.x + zc.x, zm.y + zc.y), d = make_double2(zm.x - zc.x, zm.y - zc.y);
-        const double2 ed = fft4::cmul(w, d);
+    for (int m = t; m < md; m += N2) {
+        double2 zm = L[m % N], zc = fft4::conj(L[(N - m) % N]);
+        double2 sm = make_double2(zm.x + zc.x, zm.y + zc.y), d = make_double2(zm.x - zc.x, zm.y - zc.y);
+        double2 ed = fft4::cmul(twh[m], d);  // e^{-i pi m/N} d
         double2 x = make_double2(0.5 * (sm.x + ed.y) * sc, 0.5 * (sm.y - ed.x) * sc);
-        if (m >= mlim) x = make_double2(0.0, 0.0);
+        if (m >= ntchop) x = make_double2(0.0, 0.0);
         if (m == 0) x.y = 0.0;
         if (valid) dst[m] = x;
-    };
-#pragma unroll
-    for (int n1 = 0; n1 < N1 / 2; ++n1) {
-        const int m = t + N2 * n1;
-        if (m >= md) break;
-        const double2 w = twh[m];  // and -i times that for m + N/2
-        put(m, w);
-        if (m + N / 2 < md) put(m + N / 2, make_double2(w.y, -w.x));
     }
 }
 
@@ -570,7 +555,9 @@ __device__ __forceinline__ void theta_products_r3(double2* L, int lane, double i
 // Warps per CTA (one CTA per SM): at NTH = 128 the nine line slots of 12 warps
 // fill shared memory; shorter lines leave room for more warps than 168 registers
 // a thread would (12 warps), so the kernel is compiled for 24 there: it is bound
-// by the latency of its FP64 and shared-memory instructions.
+// by the latency of its FP64 and shared-memory instructions (70.7 -> 61.7 us for
+// the 12,800 lines of 100x64x128; with two lines per warp at NTH = 32, 21.2 -> 11.1 us
+// for the 2,048 lines of 64x32x32).
 template <int N>
 constexpr int theta_warps() {
     return N <= 64 ? 24 : 12;
@@ -830,102 +817,123 @@ void phys_set_attributes() {
 // ------------------------------------------------------------------------
 // VERFFT with the four-step blocks.  CTA = (r, block of MB = W*G consecutive m);
 // group (warp w, gid) owns line m0 + w*G + gid.  PFP rows [r][z][m0..m0+MB)
-// move through a shared tile T[z][mloc] so global accesses stay contiguous.
-template <int N1, int N2>
-__global__ void __launch_bounds__(256) verfft4_kernel(DevGrid g, const __grid_constant__ VerBatch f,
-                                                      const double2* tw_g, int dir) {
-    constexpr int N = N1 * N2, G = 32 / N2;
+// move through a shared tile T[z][mloc] so global accesses stay contiguous: every
+// thread keeps one column of the tile and steps through z by N2, without the
+// division per element that a run-time tile width took.  A step's 14 fields at
+// 64x32x32 13.2 -> 9.9 us, at 100x64x128 59 -> 54 us; at 192x128x256 26.4 us a field
+// as before (the latency of load, FFT and store phases at five CTAs per SM).
+template <int N1, int N2, int W, int DIR>
+__global__ void __launch_bounds__(W * 32) verfft4_kernel(DevGrid g, const __grid_constant__ VerBatch f,
+                                                         const double2* tw_g) {
+    constexpr int N = N1 * N2, G = 32 / N2, MB = W * G, CS = MB + 1;
     extern __shared__ double2 sm[];
     const double2* src = f.src[blockIdx.z];
     double2* dst = f.dst[blockIdx.z];
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && f.zln[blockIdx.z]) *f.zln[blockIdx.z] = 0.0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane / N2, t = lane % N2;
-    const int MB = nw * G;
     double2* tw = sm;
     double2* tw2 = tw + (N + 1);                // step-2 twiddles, [k1][t]
-    double2* T = tw2 + N;                       // [N][MB + 1]; column mloc is line m0 + mloc
-    for (int q = threadIdx.x; q <= N; q += blockDim.x) tw[q] = tw_g[q];
-    for (int q = threadIdx.x; q < N; q += blockDim.x) tw2[q] = tw_g[(q % N2) * (q / N2)];
+    double2* T = tw2 + N;                       // [N][CS]; column mloc is line m0 + mloc
     const int r = blockIdx.y, m0 = blockIdx.x * MB;  // the m-blocks of one r run together
     const int mloc = warp * G + gid, m = m0 + mloc;
-    const bool ok = m < g.NTCHOPDIM;
     const int kd = g.NXCHOPDIM, kc = g.NXCHOP, md = g.NTCHOPDIM;
-    const int nmb = min(MB, md - m0);
-    double2* col = T + mloc;                    // this group's line, stride MB + 1
-    const int cs = MB + 1;
+    const bool ok = m < md;
+    double2* col = T + mloc;                    // this group's line, stride CS
+    const int ml = threadIdx.x % MB, z0 = threadIdx.x / MB;  // this thread's tile column and first row
+    const bool tok = m0 + ml < md;
+    double2* tile = T + z0 * CS + ml;
     double2 v[N1], o[N1];
-    if (dir > 0) {  // PFF [m][r][k] -> PFP [r][z][m]
-        __syncthreads();
-        const double2* line = src + ((size_t)m * g.NR + r) * kd;
+    if constexpr (DIR > 0) {  // PFF [m][r][k] -> PFP [r][z][m]
+        // k < kc as they are, the negative ones (q >= N - kd + kc) from the row's end
+        const double2* line = src + ((size_t)(ok ? m : 0) * g.NR + r) * kd;
+        const int hi = N - kd + kc, sh = N - kd;
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1) {
             const int q = t + N2 * n1;
-            int kk = -1;
-            if (q < kc) kk = q;
-            else if (q >= N - kd + kc) kk = q - (N - kd);
-            v[n1] = (ok && kk >= 0) ? line[kk] : make_double2(0.0, 0.0);
+            v[n1] = make_double2(0.0, 0.0);
+            if (ok && (q < kc || q >= hi)) v[n1] = line[q < kc ? q : q - sh];
         }
-        fft4::line_fft_inplace<N1, N2, +1>(v, col, tw, t, o, cs, tw2);
-#pragma unroll
-        for (int q = 0; q < N1; ++q) col[(size_t)fft4::out_index<N1, N2>(t, q) * cs] = o[q];
+        for (int q = threadIdx.x; q <= N; q += W * 32) tw[q] = tw_g[q];
+        for (int q = threadIdx.x; q < N; q += W * 32) tw2[q] = tw_g[(q % N2) * (q / N2)];
         __syncthreads();
-        for (int e = threadIdx.x; e < N * nmb; e += blockDim.x) {
-            const int z = e / nmb, ml = e - z * nmb;
-            dst[((size_t)r * N + z) * md + m0 + ml] = T[(size_t)z * cs + ml];
+        fft4::line_fft_inplace<N1, N2, +1>(v, col, tw, t, o, CS, tw2);
+#pragma unroll
+        for (int q = 0; q < N1; ++q) col[fft4::out_index<N1, N2>(t, q) * CS] = o[q];
+        __syncthreads();
+        double2* out = dst + ((size_t)r * N + z0) * md + m0 + ml;
+        if (tok) {
+#pragma unroll
+            for (int i = 0; i < N1; ++i) out[(size_t)(i * N2) * md] = tile[i * N2 * CS];
         }
     } else {  // PFP [r][z][m] -> PFF [m][r][k], scaled 1/NX, chopped
-        __syncthreads();
-        // the tile [z][m0 .. m0 + nmb) by cp.async: every thread keeps its column
-        // ml and issues all its rows before waiting (MB divides the block size)
-        {
-            const int ml = threadIdx.x % MB;
-            if (ml < nmb)
-                for (int z = threadIdx.x / MB; z < N; z += blockDim.x / MB)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
-                                     (uint32_t)__cvta_generic_to_shared(T + (size_t)z * cs + ml)),
-                                 "l"(src + ((size_t)r * N + z) * md + m0 + ml)
-                                 : "memory");
-            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        // the tile by cp.async: every thread issues all its rows before waiting
+        const double2* in = src + ((size_t)r * N + z0) * md + m0 + ml;
+        if (tok) {
+#pragma unroll
+            for (int i = 0; i < N1; ++i)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(tile + i * N2 * CS)),
+                             "l"(in + (size_t)(i * N2) * md)
+                             : "memory");
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int q = threadIdx.x; q <= N; q += W * 32) tw[q] = tw_g[q];
+        for (int q = threadIdx.x; q < N; q += W * 32) tw2[q] = tw_g[(q % N2) * (q / N2)];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
 #pragma unroll
-        for (int n1 = 0; n1 < N1; ++n1) v[n1] = ok ? col[(size_t)(t + N2 * n1) * cs] : make_double2(0.0, 0.0);
+        for (int n1 = 0; n1 < N1; ++n1) v[n1] = ok ? col[(t + N2 * n1) * CS] : make_double2(0.0, 0.0);
         __syncwarp();
-        fft4::line_fft_inplace<N1, N2, -1>(v, col, tw, t, o, cs, tw2);
+        fft4::line_fft_inplace<N1, N2, -1>(v, col, tw, t, o, CS, tw2);
 #pragma unroll
-        for (int q = 0; q < N1; ++q) col[(size_t)fft4::out_index<N1, N2>(t, q) * cs] = o[q];
+        for (int q = 0; q < N1; ++q) col[fft4::out_index<N1, N2>(t, q) * CS] = o[q];
         __syncwarp();
         const double sc = 1.0 / N;
-        double2* line = dst + ((size_t)m * g.NR + r) * kd;
-        for (int kk = t; kk < kd; kk += N2) {
-            const int q = (kk < kc) ? kk : (N - kd + kk);
-            double2 y = col[(size_t)q * cs];
-            if (ok) line[kk] = make_double2(y.x * sc, y.y * sc);
+        double2* line = dst + ((size_t)(ok ? m : 0) * g.NR + r) * kd;
+        if (ok) {
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) {
+                const int kk = t + N2 * n1;
+                if (kk < kd) {
+                    const double2 y = col[((kk < kc) ? kk : N - kd + kk) * CS];
+                    line[kk] = make_double2(y.x * sc, y.y * sc);
+                }
+            }
         }
     }
 }
 
-template <int N1, int N2>
-static void launch_verfft4(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
-    constexpr int N = N1 * N2, G = 32 / N2;
-    // (+1): MB = 4 G lines per CTA, more and smaller CTAs per SM overlapping their
-    // load, FFT and store phases; (-1): 8 warps, longer tile rows per cp.async pass
-    int warps = dir > 0 ? 4 : 8;
-    auto need = [&](int w) {
-        int MB = w * G;
-        return (size_t)((N + 1) + N + N * (MB + 1)) * sizeof(double2);
-    };
-    while (warps > 1 && need(warps) > 110 * 1024) --warps;
+template <int N1, int N2, int W, int DIR>
+static void launch_verfft4_w(const DevGrid& g, const FFTPlan& p, const VerBatch& f, cudaStream_t s) {
+    constexpr int N = N1 * N2, MB = W * (32 / N2);
+    constexpr size_t smem = (size_t)((N + 1) + N + N * (MB + 1)) * sizeof(double2);
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(verfft4_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(verfft4_kernel<N1, N2, W, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
-    const int MB = warps * G;
     dim3 grid((g.NTCHOPDIM + MB - 1) / MB, g.NR, f.n);
-    verfft4_kernel<N1, N2><<<grid, warps * 32, need(warps), s>>>(g, f, p.tw_x, dir);
+    verfft4_kernel<N1, N2, W, DIR><<<grid, W * 32, smem, s>>>(g, f, p.tw_x);
     count_launch();
+}
+
+// (+1): 4 G lines per CTA, more and smaller CTAs per SM overlapping their load, FFT
+// and store phases; (-1): 8 warps, longer tile rows per cp.async pass (4 at NX =
+// 512, whose tile would leave one CTA per SM).  Fewer warps where NTCHOP would leave
+// most of the lines idle (NX <= 32 has 8 lines a warp).
+template <int N1, int N2>
+static void launch_verfft4(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
+    constexpr int G = 32 / N2;
+    const int md = g.NTCHOPDIM;
+    if (dir > 0) {
+        if (md <= 2 * G) launch_verfft4_w<N1, N2, 2, +1>(g, p, f, s);
+        else launch_verfft4_w<N1, N2, 4, +1>(g, p, f, s);
+    } else {
+        if (md <= 2 * G) launch_verfft4_w<N1, N2, 2, -1>(g, p, f, s);
+        else if (md <= 4 * G || N1 * N2 > 256) launch_verfft4_w<N1, N2, 4, -1>(g, p, f, s);
+        else launch_verfft4_w<N1, N2, 8, -1>(g, p, f, s);
+    }
 }
 
 bool k_verfft4_batch(const DevGrid& g, const FFTPlan& p, const VerBatch& f, int dir, cudaStream_t s) {
