@@ -289,6 +289,8 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     v2p_pff = dalloc<double>(d.NR);
     v2p_fff = dalloc<double>(std::max(d.NRCHOP, 1));
     k_vel2pln_coef(g, explog0, d.NRCHOP, v2p_pff, v2p_fff, s);
+    v2p_d = dalloc<double>(d.NRCHOPDIM);
+    k_vel2pln_dvec(g, D, v2p_d, s);
     if (p.precision == MLEGS_PREC_FP64 && dmma_supported(g)) {
         const size_t nc = proj_comp_doubles(g);
         compV = dalloc<double>(nc);
@@ -539,8 +541,8 @@ void mlegs_ctx::force(const Field* PSI, const Field* CHI, const Field* B, Field*
     if (!split_S && fc_V) {
         for (Field* f : {NR, NP, NZ, BN}) f->space = MLEGS_PFP;
         double2* const pff[4] = {RUR->data, RUP->data, UZ->data, ROR->data};
-        project_toff(NR, NP, NZ, BN, pff, PSIN, Wf, BNout);
-        idel2ln(Wf, CHIN, 0);
+        const ProjectTail tail = project_toff(NR, NP, NZ, BN, pff, PSIN, Wf, BNout);
+        idel2ln(Wf, CHIN, 0, &tail);
         for (Field* f : {RUR, RUP, UZ, ROR, ROP, OZ, RBR, RBP, BZ, W, NR, NP, NZ, BN}) rel(f);
         return;
     }

@@ -95,7 +95,7 @@ struct mlegs_ctx {
     // chunked weight tables of the bulk fold GEMMs (FP64 contexts): PF times w_i
     // (RTRAN(-1)) and V, D, T (PROJECT of PFF inputs)
     double *fc_pf = nullptr, *fc_V = nullptr, *fc_D = nullptr, *fc_T = nullptr;
-    double *v2p_pff = nullptr, *v2p_fff = nullptr;                 // VEL2PLN coefficient vectors
+    double *v2p_pff = nullptr, *v2p_fff = nullptr, *v2p_d = nullptr;  // VEL2PLN coefficient vectors
     double* diag = nullptr;                                         // 4 x [m][k] quadratures (energy)
     double *sp_damp = nullptr, *sp_damp_h = nullptr;                // sponge factors for DT and DT/2 (RMV%SW = 2)
     double *etdE = nullptr, *etdN = nullptr, *hetdE = nullptr, *hetdN = nullptr;
@@ -457,13 +457,21 @@ struct mlegs_ctx {
         chopdo(a, pad);
         k_farfield_fix(g, a->data, d.NRCHOP + pad, s);
     }
-    void idel2ln(const Field* bb, Field* a, int pad) {  // 1013-1176
+    // tail (optional): PROJECT's closing passes, in the solve's launch
+    void idel2ln(const Field* bb, Field* a, int pad, const ProjectTail* tail = nullptr) {  // 1013-1176
         require(bb, MLEGS_FFF, "IDEL2LN");
         if (const SolveFactors* f = factors(0, pad, 0.0)) {
-            k_solve_factored(g, f->F, bb->data, a->data, a->ln, 0, 0, 0.0, pad, 1, s);
+            SolveBatch sb{};
+            sb.n = 1;
+            sb.p[0].F = f->F;
+            sb.p[0].src = bb->data;
+            sb.p[0].dst = a->data;
+            sb.p[0].ln_out = a->ln;
+            k_solve_factored_batch(g, sb, 0, 0, 0.0, pad, 1, s, tail);
             a->space = MLEGS_FFF;
             return;
         }
+        if (tail) k_project_tail(g, *tail, s);
         copy0(a, bb, pad);
         ln_zero(a);
         k_solve_del2(g, a->data, a->ln, 0, 0.0, 0, 0.0, nullptr, solve_scr, pad, s);
@@ -622,20 +630,16 @@ struct mlegs_ctx {
             throw ApiError(MLEGS_ERR_TRANSFORM, "PROJECT: bad input space");
         }
         psi_->space = chi_->space = MLEGS_FFF;
-        if (ln_mode == 1) launch_vel2pln(g, rup->data, psi_->ln, 1, ln, v2p_pff, s, chi_->ln);
-        else if (ln_mode == 2) launch_vel2pln(g, rup->data, psi_->ln, 0, 0.0, v2p_pff, s, chi_->ln);
-        else {
-            ln_zero(psi_);
-            ln_zero(chi_);
-        }
+        ProjectTail tail = project_tail(rup->data, psi_, ln_mode, ln, chi_->ln);
+        tail.keep = 1;
         if (!split_S && fc_V) {
             project_bulk(rur->data, rup->data, uz->data, psi_->data, chi_->data, s);
-            k_farfield_fix(g, psi_->data, d.NRCHOP, s);
+            k_project_tail(g, tail, s);
             return;
         }
         if (!split_S && dmma_supported(g)) {
             k_project_dmma(g, V, D, T, rur->data, rup->data, uz->data, psi_->data, chi_->data, s);
-            k_farfield_fix(g, psi_->data, d.NRCHOP, s);
+            k_project_tail(g, tail, s);
             return;
         }
         const int wr = d.NRCHOPDIM;
@@ -646,7 +650,23 @@ struct mlegs_ctx {
         fold(2, D, wr, rur->data, chi_->data, 1, 3, 0, 0);
         fold(1, V, wr, rup->data, chi_->data, 0, 4, 1, 0);
         fold(3, T, wr, uz->data, chi_->data, 0, 1, 1, 0);
-        k_farfield_fix(g, psi_->data, d.NRCHOP, s);
+        k_project_tail(g, tail, s);
+    }
+    // ln_mode as in project: 0 no LN argument, 1 its value, 2 PSI%LN by reference
+    ProjectTail project_tail(double2* rup_pff, Field* psi_, int ln_mode, double ln, double* zero_ln,
+                             double* zero_ln2 = nullptr) const {
+        ProjectTail t{};
+        t.psi = psi_->data;
+        t.line = ln_mode ? rup_pff : nullptr;
+        t.Lpff = v2p_pff;
+        t.dvec = v2p_d;
+        t.psi_ln = psi_->ln;
+        t.zero_ln[0] = zero_ln;
+        t.zero_ln[1] = zero_ln2;
+        t.mode = ln_mode == 2 ? 0 : 1;
+        t.ln = ln_mode == 1 ? ln : 0.0;
+        t.nr_sum = d.NRCHOP;
+        return t;
     }
 
     // PROJECT's five fold products of PFF inputs (mod_legops.f90:2497-2535) on
@@ -662,10 +682,11 @@ struct mlegs_ctx {
         const int pads[3] = {0, 0, 0};
         k_fold_bulk(g, seg, first, bn ? 3 : 2, outs, d.NRCHOPDIM, pads, 0, st);
     }
-    // PROJECT(NR, NP, NZ, PSI, W, 0.0) and BN = TOFF(BN) (pad 0) of PFP results of
-    // the theta stage, whose PFF images go to pff[0..3]; PSI, W, BNout in FFF.
-    void project_toff(Field* NR, Field* NP, Field* NZ, Field* BN, double2* const* pff, Field* PSI, Field* W,
-                      Field* BNout) {
+    // PROJECT(NR, NP, NZ, PSI, W, 0.0) up to its tail, which is returned for the solve
+    // that follows, and BN = TOFF(BN) (pad 0) of PFP results of the theta stage,
+    // whose PFF images go to pff[0..3]; PSI, W, BNout in FFF.
+    ProjectTail project_toff(Field* NR, Field* NP, Field* NZ, Field* BN, double2* const* pff, Field* PSI, Field* W,
+                             Field* BNout) {
         VerBatch v{};
         v.n = 4;
         Field* const f[4] = {NR, NP, NZ, BN};
@@ -674,10 +695,9 @@ struct mlegs_ctx {
             v.dst[q] = pff[q];
         }
         verfft_batch(v, -1, s);
-        launch_vel2pln(g, pff[1], PSI->ln, 1, 0.0, v2p_pff, s, W->ln, BNout->ln);
         project_bulk(pff[0], pff[1], pff[2], PSI->data, W->data, s, pff[3], BNout->data);
-        k_farfield_fix(g, PSI->data, d.NRCHOP, s);
         PSI->space = W->space = BNout->space = MLEGS_FFF;
+        return project_tail(pff[1], PSI, 1, 0.0, W->ln, BNout->ln);
     }
     // PROJECT(RUR, RUP, UZ, PSI, CHI) with PSI%LN by reference (ln_mode 2) for
     // FFF inputs whose LN terms are zero: one composite FFF -> FFF product per m

@@ -241,7 +241,6 @@ void phase1(mlegs_ensemble& E, EnsInst& I) {
     I.Wf = I.f[9];
     // PROJECT(NR, NP, NZ, PSI_N, W, 0) (mod_legops.f90:2397-2545)
     I.PN->space = I.Wf->space = I.BN->space = MLEGS_FFF;
-    launch_vel2pln(g, I.f[1]->data, I.PN->ln, 1, 0.0, c->v2p_pff, c->s, I.Wf->ln, I.BN->ln);
     GroupFold pj{};
     pj.g = g;
     const double* wt[5] = {c->V, c->D, c->D, c->V, c->T};
@@ -274,10 +273,10 @@ void phase1(mlegs_ensemble& E, EnsInst& I) {
     E.gfold.h.push_back(rt);
 }
 
-// Phase 2: PROJECT's far-field fix, the IDEL2LN(W -> CHI_N) problem.
+// Phase 2: PROJECT's VEL2PLN and far-field fix, the IDEL2LN(W -> CHI_N) problem.
 void phase2(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
-    k_farfield_fix(c->g, I.PN->data, c->d.NRCHOP, c->s);
+    k_project_tail(c->g, c->project_tail(I.f[1]->data, I.PN, 1, 0.0, I.Wf->ln, I.BN->ln), c->s);
     const auto* fc = c->factors(0, 0, 0.0);
     if (!fc) throw ApiError(MLEGS_ERR_STATE, "ensemble: IDEL2LN factors missing");
     GroupSolve p{};

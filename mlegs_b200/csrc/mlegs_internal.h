@@ -183,6 +183,24 @@ struct SolveBatch {
     SolveItem p[3];
     int n;
 };
+// What follows PROJECT's fold products: VEL2PLN with PSI%LN given or extracted
+// (mod_legops.f90:2277-2339; line: RUP's (m, k) = (0, 0) PFF line, stride NXCHOPDIM,
+// null: no LN argument) applied to PSI's (0, 0) column, and the far-field fix of PSI's
+// m = 0 columns over nr_sum rows.  VEL2PLN adds PLN u to the line before the products,
+// a fixed u: dvec is the change of PSI's column per unit of PLN.  keep: the line is the
+// caller's RUP and takes VEL2PLN's change too.
+struct ProjectTail {
+    double2* psi;
+    double2* line;
+    int keep;
+    const double *Lpff, *dvec;
+    double* psi_ln;       // <- ln (mode 1) or PLN (mode 0)
+    double* zero_ln[2];   // LN slots set to 0 (null: none)
+    int mode, nr_sum;
+    double ln;
+};
+void k_vel2pln_dvec(const DevGrid& g, const double* D, double* dvec, cudaStream_t s);
+void k_project_tail(const DevGrid& g, const ProjectTail& t, cudaStream_t s);
 struct GroupSolve {
     DevGrid g;
     SolveItem it;
@@ -305,9 +323,7 @@ void k_ihelmp(const DevGrid& g, int P, const double* dq, int rows, double2* a, c
 // on the PFF line of RUP (Lpff, NR entries), or on RUP's FFF (0, 0) column
 // (Lfff, NRCHOP entries; mode 0, applied to that column).
 void k_vel2pln_coef(const DevGrid& g, const double* explog0, int nn, double* Lpff, double* Lfff, cudaStream_t s);
-// zero_ln, zero_ln2 (optional): further LN slots set to 0 by the same launch.
-void launch_vel2pln(const DevGrid& g, double2* rup_pff, double* psi_ln, int mode, double ln, const double* Lpff,
-                    cudaStream_t s, double* zero_ln = nullptr, double* zero_ln2 = nullptr);
+// zero_ln (optional): one more LN slot set to 0 by the same launch.
 void launch_vel2pln_fff(const DevGrid& g, double2* rup_fff, double* psi_ln, const double* Lfff, cudaStream_t s,
                         double* zero_ln = nullptr);
 
@@ -326,8 +342,10 @@ void k_solve_factored(const DevGrid& g, const double* F, const double2* src, dou
 // the system size on left as they are; the batch form writes them as zero.
 void k_solve_T(const DevGrid& g, const double* F, double2* y, int kind, int pad, cudaStream_t s);
 void k_solve_T_batch(const DevGrid& g, const SolveBatch& b, int kind, int pad, cudaStream_t s);
+// tail (optional): PROJECT's, which depends on the same launch as the solve does, in
+// further blocks of this one.
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
-                            int farfield, cudaStream_t s);
+                            int farfield, cudaStream_t s, const ProjectTail* tail = nullptr);
 // The AB2 update with VISC2's right-hand side for up to three fields (kernels.cu).
 struct Ab2Args {
     const double2* a[3];     // state before the step

@@ -16,6 +16,7 @@
 //  kind 2  IHELM:   m = 0 solves (H XM) y = rhs on NN-1 rows, A = XM y
 #include "bulk.cuh"
 #include "mlegs_internal.h"
+#include "project_tail.cuh"
 
 #include <algorithm>
 
@@ -739,11 +740,21 @@ __device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p
     }
 }
 
-// blockIdx.y: the problem (a step's three viscous solves go in one launch)
+// blockIdx.y: the problem (a step's three viscous solves go in one launch); blocks
+// from nblocks on: PROJECT's tail, two axial modes each
 template <bool TR, bool XG>
 __global__ void __launch_bounds__(64) solve_factored_kernel(DevGrid g, const __grid_constant__ SolveBatch b,
-                                                            SolveForm fo) {
+                                                            SolveForm fo, const __grid_constant__ ProjectTail tail,
+                                                            int nblocks) {
+    if ((int)blockIdx.x >= nblocks) {
+        project_tail_warp(g, tail, 2 * (blockIdx.x - nblocks) + (threadIdx.x >> 5), threadIdx.x & 31);
+        return;
+    }
     solve_block<TR, XG>(g, b.p[blockIdx.y], fo, blockIdx.x);
+}
+
+__global__ void __launch_bounds__(64) project_tail_kernel(DevGrid g, const __grid_constant__ ProjectTail tail) {
+    project_tail_warp(g, tail, 2 * blockIdx.x + (threadIdx.x >> 5), threadIdx.x & 31);
 }
 
 // Grouped form over the instances of an ensemble: a block's problem by binary
@@ -773,24 +784,32 @@ void allow_smem(K kernel) {
 }
 
 template <bool TR>
-void launch_solve(const DevGrid& g, const SolveBatch& b, const SolveForm& fo, cudaStream_t s) {
+void launch_solve(const DevGrid& g, const SolveBatch& b, const SolveForm& fo, cudaStream_t s,
+                  const ProjectTail* tail = nullptr) {
     static const bool attr = [] {
         allow_smem(solve_factored_kernel<TR, false>);
         allow_smem(solve_factored_kernel<TR, true>);
         return true;
     }();
     (void)attr;
-    const dim3 grid(FactorTable(g).nkb * g.NTCHOPDIM, b.n);
+    const int nblocks = FactorTable(g).nkb * g.NTCHOPDIM;
+    const dim3 grid(nblocks + (tail ? (g.NXCHOPDIM + 1) / 2 : 0), b.n);
+    const ProjectTail tl = tail ? *tail : ProjectTail{};
     const size_t smem = solve_smem(g, fo.pad, false);
-    if (smem <= SOLVE_SMEM_MAX) solve_factored_kernel<TR, false><<<grid, 64, smem, s>>>(g, b, fo);
-    else solve_factored_kernel<TR, true><<<grid, 64, solve_smem(g, fo.pad, true), s>>>(g, b, fo);
+    if (smem <= SOLVE_SMEM_MAX) solve_factored_kernel<TR, false><<<grid, 64, smem, s>>>(g, b, fo, tl, nblocks);
+    else solve_factored_kernel<TR, true><<<grid, 64, solve_smem(g, fo.pad, true), s>>>(g, b, fo, tl, nblocks);
     count_launch();
 }
 }  // namespace
 
 void k_solve_factored_batch(const DevGrid& g, const SolveBatch& b, int kind, int has_ln, double ln_in, int pad,
-                            int farfield, cudaStream_t s) {
-    launch_solve<false>(g, b, SolveForm{kind, has_ln, ln_in, pad, farfield, 0}, s);
+                            int farfield, cudaStream_t s, const ProjectTail* tail) {
+    launch_solve<false>(g, b, SolveForm{kind, has_ln, ln_in, pad, farfield, 0}, s, tail);
+}
+
+void k_project_tail(const DevGrid& g, const ProjectTail& t, cudaStream_t s) {
+    project_tail_kernel<<<(g.NXCHOPDIM + 1) / 2, 64, 0, s>>>(g, t);
+    count_launch();
 }
 
 void k_solve_factored(const DevGrid& g, const double* F, const double2* src, double2* dst, double* ln_out, int kind,
