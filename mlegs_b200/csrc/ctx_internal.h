@@ -630,16 +630,20 @@ struct mlegs_ctx {
             throw ApiError(MLEGS_ERR_TRANSFORM, "PROJECT: bad input space");
         }
         psi_->space = chi_->space = MLEGS_FFF;
-        ProjectTail tail = project_tail(rup->data, psi_, ln_mode, ln, chi_->ln);
-        tail.keep = 1;
+        if (ln_mode == 1) launch_vel2pln(g, rup->data, psi_->ln, 1, ln, v2p_pff, s, chi_->ln);
+        else if (ln_mode == 2) launch_vel2pln(g, rup->data, psi_->ln, 0, 0.0, v2p_pff, s, chi_->ln);
+        else {
+            ln_zero(psi_);
+            ln_zero(chi_);
+        }
         if (!split_S && fc_V) {
             project_bulk(rur->data, rup->data, uz->data, psi_->data, chi_->data, s);
-            k_project_tail(g, tail, s);
+            k_farfield_fix(g, psi_->data, d.NRCHOP, s);
             return;
         }
         if (!split_S && dmma_supported(g)) {
             k_project_dmma(g, V, D, T, rur->data, rup->data, uz->data, psi_->data, chi_->data, s);
-            k_project_tail(g, tail, s);
+            k_farfield_fix(g, psi_->data, d.NRCHOP, s);
             return;
         }
         const int wr = d.NRCHOPDIM;
@@ -650,22 +654,17 @@ struct mlegs_ctx {
         fold(2, D, wr, rur->data, chi_->data, 1, 3, 0, 0);
         fold(1, V, wr, rup->data, chi_->data, 0, 4, 1, 0);
         fold(3, T, wr, uz->data, chi_->data, 0, 1, 1, 0);
-        k_project_tail(g, tail, s);
+        k_farfield_fix(g, psi_->data, d.NRCHOP, s);
     }
-    // ln_mode as in project: 0 no LN argument, 1 its value, 2 PSI%LN by reference
-    ProjectTail project_tail(double2* rup_pff, Field* psi_, int ln_mode, double ln, double* zero_ln,
-                             double* zero_ln2 = nullptr) const {
+    ProjectTail project_tail(const double2* rup_pff, Field* psi_, Field* w, Field* bn) const {
         ProjectTail t{};
         t.psi = psi_->data;
-        t.line = ln_mode ? rup_pff : nullptr;
+        t.line = rup_pff;
         t.Lpff = v2p_pff;
         t.dvec = v2p_d;
-        t.psi_ln = psi_->ln;
-        t.zero_ln[0] = zero_ln;
-        t.zero_ln[1] = zero_ln2;
-        t.mode = ln_mode == 2 ? 0 : 1;
-        t.ln = ln_mode == 1 ? ln : 0.0;
-        t.nr_sum = d.NRCHOP;
+        t.zero_ln[0] = psi_->ln;
+        t.zero_ln[1] = w->ln;
+        t.zero_ln[2] = bn->ln;
         return t;
     }
 
@@ -697,7 +696,7 @@ struct mlegs_ctx {
         verfft_batch(v, -1, s);
         project_bulk(pff[0], pff[1], pff[2], PSI->data, W->data, s, pff[3], BNout->data);
         PSI->space = W->space = BNout->space = MLEGS_FFF;
-        return project_tail(pff[1], PSI, 1, 0.0, W->ln, BNout->ln);
+        return project_tail(pff[1], PSI, W, BNout);
     }
     // PROJECT(RUR, RUP, UZ, PSI, CHI) with PSI%LN by reference (ln_mode 2) for
     // FFF inputs whose LN terms are zero: one composite FFF -> FFF product per m

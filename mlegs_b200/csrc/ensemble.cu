@@ -276,7 +276,7 @@ void phase1(mlegs_ensemble& E, EnsInst& I) {
 // Phase 2: PROJECT's VEL2PLN and far-field fix, the IDEL2LN(W -> CHI_N) problem.
 void phase2(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
-    k_project_tail(c->g, c->project_tail(I.f[1]->data, I.PN, 1, 0.0, I.Wf->ln, I.BN->ln), c->s);
+    k_project_tail(c->g, c->project_tail(I.f[1]->data, I.PN, I.Wf, I.BN), c->s);
     const auto* fc = c->factors(0, 0, 0.0);
     if (!fc) throw ApiError(MLEGS_ERR_STATE, "ensemble: IDEL2LN factors missing");
     GroupSolve p{};

@@ -342,6 +342,29 @@ __device__ double vel2pln_dot(const double* L, const double2* line, size_t st, i
     return tot;
 }
 
+__global__ void vel2pln_kernel(DevGrid g, double2* rup, double* psi_ln, int mode, double ln_in, const double* Lpff,
+                               double* zero_ln) {
+    __shared__ double part[8];
+    const size_t st = g.NXCHOPDIM;  // PFF row stride for m = 0 ([0][r][k])
+    const double pln = vel2pln_dot(Lpff, rup, st, g.NR, part);
+    const double* pf = g.pf;
+    for (int i = threadIdx.x; i < g.NRH; i += blockDim.x) {
+        double e2 = -pf[i] * pln / g.norm0[0];
+        double o2 = -pf[(size_t)g.NRH + i] * pln / g.norm0[1];
+        rup[(size_t)i * st].x -= (e2 + o2);
+        rup[(size_t)(g.NR - 1 - i) * st].x -= (e2 - o2);
+    }
+    if (threadIdx.x == 0) {
+        *psi_ln = (mode == 1) ? ln_in : pln;
+        if (zero_ln) *zero_ln = 0.0;
+    }
+}
+void launch_vel2pln(const DevGrid& g, double2* rup_pff, double* psi_ln, int mode, double ln, const double* Lpff,
+                    cudaStream_t s, double* zero_ln) {
+    vel2pln_kernel<<<1, 256, 0, s>>>(g, rup_pff, psi_ln, mode, ln, Lpff, zero_ln);
+    count_launch();
+}
+
 // dvec of ProjectTail: -D . (OE fold of u), u = PF_0 / NORM(1) +- PF_1 / NORM(2) (+ for
 // i < NRH, - on the mirror rows), at m = 0.
 __global__ void vel2pln_dvec_kernel(DevGrid g, const double* D, double* dvec) {

@@ -183,21 +183,19 @@ struct SolveBatch {
     SolveItem p[3];
     int n;
 };
-// What follows PROJECT's fold products: VEL2PLN with PSI%LN given or extracted
-// (mod_legops.f90:2277-2339; line: RUP's (m, k) = (0, 0) PFF line, stride NXCHOPDIM,
-// null: no LN argument) applied to PSI's (0, 0) column, and the far-field fix of PSI's
-// m = 0 columns over nr_sum rows.  VEL2PLN adds PLN u to the line before the products,
-// a fixed u: dvec is the change of PSI's column per unit of PLN.  keep: the line is the
-// caller's RUP and takes VEL2PLN's change too.
+// What follows the fold products of PROJECT(NR, NP, NZ, PSI, W, 0.0) in the right-hand
+// side: VEL2PLN with PSI%LN = 0 (mod_legops.f90:2277-2339; line: RUP's (m, k) = (0, 0)
+// PFF line, stride NXCHOPDIM) applied to PSI's (0, 0) column, and the far-field fix of
+// PSI's m = 0 columns over NRCHOP rows.  VEL2PLN adds PLN u to the line before the
+// products, a fixed u: dvec is the change of PSI's column per unit of PLN.
+// CALC_BOUSSI_FORCE returns PSI as it is.  Where PSI goes on through PC2VEL and IDEL2LN
+// (the ETD step, PROJECT itself) the line is changed before the products, as the formulas
+// stand: IDEL2LN magnifies a last-bit change some 1e5 times.
 struct ProjectTail {
     double2* psi;
-    double2* line;
-    int keep;
+    const double2* line;
     const double *Lpff, *dvec;
-    double* psi_ln;       // <- ln (mode 1) or PLN (mode 0)
-    double* zero_ln[2];   // LN slots set to 0 (null: none)
-    int mode, nr_sum;
-    double ln;
+    double* zero_ln[3];  // LN slots set to 0, PSI's among them
 };
 void k_vel2pln_dvec(const DevGrid& g, const double* D, double* dvec, cudaStream_t s);
 void k_project_tail(const DevGrid& g, const ProjectTail& t, cudaStream_t s);
@@ -324,6 +322,8 @@ void k_ihelmp(const DevGrid& g, int P, const double* dq, int rows, double2* a, c
 // (Lfff, NRCHOP entries; mode 0, applied to that column).
 void k_vel2pln_coef(const DevGrid& g, const double* explog0, int nn, double* Lpff, double* Lfff, cudaStream_t s);
 // zero_ln (optional): one more LN slot set to 0 by the same launch.
+void launch_vel2pln(const DevGrid& g, double2* rup_pff, double* psi_ln, int mode, double ln, const double* Lpff,
+                    cudaStream_t s, double* zero_ln = nullptr);
 void launch_vel2pln_fff(const DevGrid& g, double2* rup_fff, double* psi_ln, const double* Lfff, cudaStream_t s,
                         double* zero_ln = nullptr);
 
