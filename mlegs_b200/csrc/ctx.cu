@@ -10,9 +10,14 @@
 
 thread_local std::vector<void*>* mlegs_host::g_allocs = nullptr;
 
-// A PFF image up to this size: TOFP of several fields as one launch per stage
-// (tofp_pipe); above it, groups of three fields with the stages overlapped.
-static constexpr size_t PIPE_ALL_BYTES = (size_t)8 << 20;
+// TOFP of several fields (tofp_pipe) goes in one launch per stage while the PFF images
+// between the stages stay within PIPE_BYTES, 5% of the device's memory; larger grids run
+// groups of PIPE_MIN fields.  One launch was the faster form at every size measured
+// (CALC_BOUSSI_FORCE, against groups of three with the two stages on two streams, which
+// held as many images as PIPE_MIN): 61 against 81 us at 64x32x32, 218 against 236 us at
+// 100x64x128, 478 against 501 us at 128x128x128, 1447 against 1481 us at 192x128x256.
+static constexpr size_t PIPE_BYTES = (size_t)8 << 30;
+static constexpr int PIPE_MIN = 6;
 
 // ====================================================================== set-up
 namespace {
@@ -426,11 +431,10 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     lnslots = dalloc<double>(nslots);
     CK(cudaMemsetAsync(lnslots, 0, nslots * sizeof(double), s));
     scratch = dalloc<double2>(d.cap());
-    pipe_group = d.pff() * sizeof(double2) <= PIPE_ALL_BYTES ? BATCH : 3;
+    pipe_group = BATCH * d.pff() * sizeof(double2) <= PIPE_BYTES ? BATCH : PIPE_MIN;
     {
-        const int images = pipe_group == BATCH ? BATCH : 2 * pipe_group;
-        double2* slab = dalloc<double2>(images * d.pff());
-        for (int q = 0; q < images; ++q) pbuf[q] = slab + q * d.pff();
+        double2* slab = dalloc<double2>(pipe_group * d.pff());
+        for (int q = 0; q < pipe_group; ++q) pbuf[q] = slab + q * d.pff();
     }
     size_t nsys = (size_t)d.NTCHOPDIM * d.NXCHOPDIM;
     solve_scr = dalloc<double>((size_t)d.NRCHOPDIM * 4 * nsys);

@@ -66,12 +66,11 @@ struct mlegs_ctx {
     Dims d{};
     DevGrid g{};
     cudaStream_t s = nullptr;
-    cudaStream_t s2 = nullptr;         // second stream of the RTRAN(+1) -> VERFFT(+1) pipeline
+    cudaStream_t s2 = nullptr;         // second stream (nonlin, the ETD step's PC2VOR)
     cudaEvent_t evs[64] = {};          // fork/join events, used in rotation
     int ev_next = 0;
-    // TOFP of several fields (tofp_pipe): fields per launch, and the PFF images
-    // between RTRAN(+1) and VERFFT(+1) (pipe_group of them, twice that when the
-    // two stages overlap)
+    // TOFP of several fields (tofp_pipe): fields per launch, and as many PFF images
+    // between RTRAN(+1) and VERFFT(+1)
     int pipe_group = 1;
     double2* pbuf[BATCH] = {};
     int dev = 0;
@@ -312,15 +311,20 @@ struct mlegs_ctx {
     // TOFP of FFF fields up to PFP (RTRAN(+1) then VERFFT(+1), the reference's
     // order per field).  Each field ends in its own buffer, in PFP, LN 0; src and
     // ln, when given, are the FFF data and LN slots read instead of the fields' own
-    // (null ln entries: no log term).  Small grids (pipe_group = BATCH) run all
-    // fields in one launch per stage: one field alone leaves most of the chip idle
-    // and each launch costs a few us.  Large ones run groups of pipe_group fields
-    // as a two-stream pipeline, the GEMM of a group on s beside the VERFFT of the
-    // group before it on s2, through two sets of PFF images.
+    // (null ln entries: no log term).  Groups of pipe_group fields, one launch per stage
+    // and group: one field alone leaves much of the chip idle on small grids, and the
+    // last wave of a launch on large ones.  The split GEMMs, one launch per field, run
+    // beside the VERFFT of the three fields before them, which s2 takes (1% of
+    // CALC_BOUSSI_FORCE at 128x128x128).
     cudaEvent_t next_event() {
         cudaEvent_t e = evs[ev_next];
         ev_next = (ev_next + 1) % 64;
         return e;
+    }
+    void order(cudaStream_t first, cudaStream_t then) {  // what `then` gets next waits for `first`
+        cudaEvent_t e = next_event();
+        CK(cudaEventRecord(e, first));
+        CK(cudaStreamWaitEvent(then, e, 0));
     }
     void rtran_batch(const B2PBatch& f, cudaStream_t st) {
         if (!split_S) {
@@ -343,49 +347,34 @@ struct mlegs_ctx {
                    const double2* const* src = nullptr, const double* const* ln = nullptr) {
         if (!src)
             for (int i = 0; i < n; ++i) require(fs[i], MLEGS_FFF, "RTRAN");
-        const bool all = pipe_group >= BATCH;
-        if (!all) {
-            cudaEvent_t e0 = next_event();
-            CK(cudaEventRecord(e0, s));
-            CK(cudaStreamWaitEvent(s2, e0, 0));
-        }
-        cudaEvent_t done[2] = {nullptr, nullptr};  // last VERFFT reading image set j
-        for (int i0 = 0, set = 0; i0 < n; i0 += pipe_group, set ^= 1) {
-            const int cnt = std::min(pipe_group, n - i0);
+        const int step = split_S ? 3 : pipe_group;
+        if (split_S) order(s, s2);
+        for (int i0 = 0, img = 0; i0 < n; i0 += step, img += step) {
+            const int cnt = std::min(step, n - i0);
+            if (img + cnt > pipe_group) {  // every image taken: wait for their VERFFT
+                if (split_S) order(s2, s);
+                img = 0;
+            }
             B2PBatch b{};
             VerBatch v{};
             b.n = v.n = cnt;
             for (int q = 0; q < cnt; ++q) {
                 Field* f = fs[i0 + q];
-                double2* buf = pbuf[(all ? 0 : set * pipe_group) + q];
                 b.in[q] = src ? src[i0 + q] : f->data;
-                b.out[q] = buf;
+                b.out[q] = pbuf[img + q];
                 b.ln[q] = ln ? ln[i0 + q] : f->ln;
                 b.pad[q] = pads[i0 + q];
-                v.src[q] = buf;
+                v.src[q] = pbuf[img + q];
                 v.dst[q] = f->data;
                 v.zln[q] = f->ln;  // RTRAN zeroes LN
                 if (ready && ready[i0 + q]) CK(cudaStreamWaitEvent(s, ready[i0 + q], 0));  // field made on s2
             }
-            if (done[set]) CK(cudaStreamWaitEvent(s, done[set], 0));
             rtran_batch(b, s);
-            if (all) {
-                verfft_batch(v, +1, s);
-            } else {
-                cudaEvent_t eb = next_event();
-                CK(cudaEventRecord(eb, s));
-                CK(cudaStreamWaitEvent(s2, eb, 0));
-                verfft_batch(v, +1, s2);
-                cudaEvent_t ev = next_event();
-                CK(cudaEventRecord(ev, s2));
-                done[set] = ev;
-            }
+            if (split_S) order(s, s2);
+            verfft_batch(v, +1, split_S ? s2 : s);
             for (int q = 0; q < cnt; ++q) fs[i0 + q]->space = MLEGS_PFP;
         }
-        if (all) return;
-        cudaEvent_t ej = next_event();
-        CK(cudaEventRecord(ej, s2));
-        CK(cudaStreamWaitEvent(s, ej, 0));
+        if (split_S) order(s2, s);
     }
 
     // ------------------------------------------------------------------ operators
