@@ -112,10 +112,6 @@ void k_rtran_b2p(const DevGrid& g, const double2* a, double2* b, const double* l
         k_rtran_b2p_bulk(g, f, s);
         return;
     }
-    if (dmma_supported(g)) {
-        k_rtran_b2p_dmma(g, a, b, ln, pad, s);
-        return;
-    }
     int ncol = 2 * g.NXCHOPDIM;
     dim3 grid((ncol + TN - 1) / TN, (g.NRH + TM - 1) / TM, g.NTCHOPDIM);
     rtran_b2p_kernel<<<grid, 128, 0, s>>>(g, (const double*)a, (double*)b, ln, pad);

@@ -1,7 +1,7 @@
 // RTRAN(A, +1) on the FP64 tensor path with bulk-copy staging and a
 // warp-specialised pipeline (FP64 contexts).
 //
-// Same contract as b2p_dmma_kernel (gemm_dmma.cu, mod_fft.f90:1264-1336): per
+// The contract of rtran_b2p_kernel (gemm.cu, mod_fft.f90:1264-1336): per
 // m and parity p of n,
 //     C_p(i, c) = sum_t PF(i, 2t+p) A(2t+p, c),  B(i) = C_0 + C_1,
 //     B(NR-1-i) = C_0 - C_1,  plus the (m, k) = (0, 0) log term.

@@ -48,12 +48,12 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
 // B(i) = C_0 + C_1 and B(NR-1-i) = C_0 - C_1.  The output-row m-tiles go
 // round-robin over NW warps.
 constexpr int KCB = 16;
-constexpr int NST_B2P = 2;   // ring stages of b2p_dmma_kernel
+constexpr int NST_B2P = 2;   // ring stages of b2p_tile
 constexpr int NST_FOLD = 2;  // ring stages of legfold_dmma_kernel
 constexpr int NST_PFFF = 2;  // ring stages of projfff_dmma_kernel
 
-// One (m, 8 NJ-column) tile of RTRAN(+1): the body of b2p_dmma_kernel (NJ = 4),
-// also run per work item by the grouped ensemble kernel (ensemble.cu).
+// One (m, 8 NJ-column) tile of RTRAN(+1): a work item of the grouped ensemble kernel
+// (ensemble.cu); a context's own RTRAN(+1) is b2p_bulk_kernel (gemm_bulk.cu).
 template <int NW, int MTW, int NJ = 4>
 __device__ __forceinline__ void b2p_tile(const DevGrid& g, const double* __restrict__ A, double* __restrict__ out,
                                          const double* ln, int pad, int SA, int m, int c0, double* smd) {
@@ -169,14 +169,6 @@ __device__ __forceinline__ void b2p_tile(const DevGrid& g, const double* __restr
             *(double2*)(o + (size_t)rh * ncol + c) = hi;
         }
     }
-}
-
-template <int NW, int MTW>
-__global__ void __launch_bounds__(NW * 32) b2p_dmma_kernel(DevGrid g, const double* __restrict__ A,
-                                                           double* __restrict__ out, const double* ln, int pad,
-                                                           int SA) {
-    extern __shared__ double smd[];
-    b2p_tile<NW, MTW>(g, A, out, ln, pad, SA, blockIdx.y, blockIdx.x * CT, smd);
 }
 
 // Fold GEMMs: RTRAN(-1) and PROJECT's five EOMUL/OEMUL products.  One CTA
@@ -542,33 +534,6 @@ __global__ void __launch_bounds__(NW * 32, 5) projfff_dmma_kernel(DevGrid g, Pro
 static int pad16_8(int v) { return v + ((8 - v % 16) + 16) % 16; }  // smallest >= v that is 8 mod 16
 
 bool dmma_supported(const DevGrid& g) { return g.NRH <= 128 && g.NRH % 2 == 0 && g.NRCHOPDIM <= 256; }
-
-template <int NW, int MTW>
-static void b2p_launch(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
-    const int SA = pad16_8(((g.NRH + 7) / 8) * 8);
-    const size_t smem = NST_B2P * (size_t)KCB * (SA + SBS) * sizeof(double);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(b2p_dmma_kernel<NW, MTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        attr = true;
-    }
-    dim3 grid((2 * g.NXCHOPDIM + CT - 1) / CT, g.NTCHOPDIM);
-    b2p_dmma_kernel<NW, MTW><<<grid, NW * 32, smem, s>>>(g, (const double*)a, (double*)b, ln, pad, SA);
-    count_launch();
-}
-
-// The NRH / 8 output m-tiles go round-robin over 6 warps.
-void k_rtran_b2p_dmma(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s) {
-    // 4 warps per CTA: the small CTAs (about 140 registers a thread, 36 KB of
-    // shared memory) run three to an SM; the m-tiles go round-robin over the warps
-    const int RT = (g.NRH + 7) / 8;
-    switch ((RT + 3) / 4) {
-        case 1: b2p_launch<4, 1>(g, a, b, ln, pad, s); break;
-        case 2: b2p_launch<4, 2>(g, a, b, ln, pad, s); break;
-        case 3: b2p_launch<4, 3>(g, a, b, ln, pad, s); break;
-        default: b2p_launch<4, 4>(g, a, b, ln, pad, s); break;
-    }
-}
 
 template <int NW, int MTW>
 static void legfold_launch(const DevGrid& g, const FoldArgs& fa, cudaStream_t s) {

@@ -240,7 +240,6 @@ void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nou
                  const int* pads, int accumulate, cudaStream_t s);
 // FP64 tensor-path (mma.sync m8n8k4.f64) forms used by k_rtran_b2p / k_fold_gemm when supported.
 bool dmma_supported(const DevGrid& g);
-void k_rtran_b2p_dmma(const DevGrid& g, const double2* a, double2* b, const double* ln, int pad, cudaStream_t s);
 void k_fold_gemm_dmma(const DevGrid& g, const double* Wt, int wt_rows, const double2* in, double2* out, int mode,
                       int scale, int accumulate, int pad, cudaStream_t s);
 // PROJECT's five fold products in one launch (FP64 tensor path): PSI and CHI from
