@@ -341,8 +341,8 @@ void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F, 
 // at a time from global memory, 34 us with one warp doing both jobs.  A 58-row
 // solve at 64x32x32 takes 11.6 us, 17-19 us in the other forms (ncu, cold cache).
 // The blocks run m ascending: longest first.
-// XG: columns too long for shared memory (more than about 800 rows) stay in
-// global memory, read and written a chunk at a time.
+// XG: columns too long for shared memory (NRCHOP + pad > 727 rows at SOLVE_SMEM_MAX)
+// stay in global memory, read and written a chunk at a time.
 namespace {
 using namespace bulk;
 
@@ -481,16 +481,21 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
         }
         return -1;
     };
-    // column <- A column for a tri-diagonal A of unit diagonal over rows < nn (XM and XM^T)
+    // column <- A column for a tri-diagonal A of unit diagonal over rows < nn (XM and XM^T);
+    // XM^T comes first and takes the right-hand side, which XG reads from src (src may be
+    // dst: a row is read before its chunk is written)
     auto xm_pass = [&](bool transposed) {
-        double prev = 0.0, cur = nn > 0 ? xget(0) : 0.0;
+        auto get = [&](int r) -> double {
+            return XG && transposed ? (live ? sc[(size_t)r * st] : 0.0) : xget(r);
+        };
+        double prev = 0.0, cur = nn > 0 ? get(0) : 0.0;
         for (int r0 = 0; r0 < nn; r0 += SCH) {
             double nx[SCH], lo[SCH], hi[SCH];
 #pragma unroll
             for (int q = 0; q < SCH; ++q) {
                 const int r = r0 + q, rl = transposed ? r - 1 : r, rh = transposed ? r + 1 : r;
                 const bool a = r >= 1 && r < nn, b = r + 1 < nn;
-                nx[q] = b ? xget(r + 1) : 0.0;
+                nx[q] = b ? get(r + 1) : 0.0;
                 lo[q] = a ? sh.xm[2 * rl + (transposed ? 1 : 0)] : 0.0;
                 hi[q] = b ? sh.xm[2 * rh + (transposed ? 0 : 1)] : 0.0;
             }
@@ -508,7 +513,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
         }
     };
     // the transposed IHELM system at m = 0 takes w = XM^T y, which couples
-    // neighbouring rows: the column is staged (nn rows) before the passes
+    // neighbouring rows: the column is formed (nn rows, in dst for XG) before the passes
     constexpr bool staged = TR && HB == 3;
     if constexpr (staged) {
         if (!XG && !warp_wait(sh.whole, 0, sh.stop)) return give_up();
