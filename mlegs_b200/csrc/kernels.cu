@@ -921,12 +921,15 @@ template <int WHICH>
 __global__ void __launch_bounds__(256) deriv_kernel(DevGrid g, const __grid_constant__ DerivArgs A) {
     size_t t;
     int m, n, k;
-    if (!tile_index(g, t, m, n, k)) return;
-    // the outputs' LN slots (these fields carry no log term); read by no thread here
-    if (t < 9) {
-        double* z = A.zln[t];
+    const bool in = tile_index(g, t, m, n, k);
+    // the outputs' LN slots (these fields carry no log term), by thread number: a field
+    // can have fewer than nine entries.  Read by no thread here
+    const int th = threadIdx.y * 32 + threadIdx.x;
+    if (th < 9 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+        double* z = A.zln[th];
         if (z) *z = 0.0;
     }
+    if (!in) return;
     double2 u[3], w[3], d[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) u[q] = w[q] = d[q] = make_double2(0.0, 0.0);
