@@ -91,13 +91,14 @@ int mlegs_create(const mlegs_params* p, mlegs_ctx** out);
 int mlegs_destroy(mlegs_ctx* ctx);
 const char* mlegs_last_error(const mlegs_ctx* ctx);
 /* Waits for the context's stream; returns MLEGS_ERR_TIMEOUT (once) when a
- * bounded wait inside a tensor-core kernel ran out since the last sync (the
- * results of that launch are invalid; the context stays usable). */
+ * bounded wait inside a tensor-core kernel or a banded solve ran out since the
+ * last sync (the results of that launch are invalid; the context stays usable). */
 int mlegs_sync(mlegs_ctx* ctx);
-/* Limit of the pipeline waits inside the tensor-core kernels, in SM cycles
- * (0 restores the default, about one second).  No counterpart in the
- * reference.  A short limit makes a wait run out: the kernel then drains what
- * it has in flight, frees its tensor memory and returns, and the next
+/* Limit of the pipeline waits inside the split-BF16 tensor-core kernels and the
+ * banded solves, in SM cycles (0 restores the default, about one second), for
+ * the launches from here on (a captured graph keeps its own).  No counterpart
+ * in the reference.  A short limit makes a wait run out: the kernel then drains
+ * what it has in flight, frees its tensor memory and returns, and the next
  * mlegs_sync reports MLEGS_ERR_TIMEOUT; used to test that error path. */
 int mlegs_set_wait_limit(mlegs_ctx* ctx, int64_t cycles);
 /* Sizes (NDIMR, NDIMTH, NX, NRCHOPDIM, NTCHOPDIM, NXCHOPDIM, NRH, NR, NTH). */

@@ -43,6 +43,28 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
         if ((uint64_t)clock64() - t0 > WAIT_CYCLES) return false;
     return true;
 }
+__device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(sa_of(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// The same with the caller's limit (0: WAIT_CYCLES), which is polled: try_wait may suspend
+// the thread for longer than a limit of a few cycles.  The clock is read before the
+// barrier, so a limit of one cycle runs out in every wait.
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, uint64_t limit) {
+    if (limit == 0) return bar_wait(bar, parity);
+    const uint64_t t0 = (uint64_t)clock64();
+    do {
+        if ((uint64_t)clock64() - t0 > limit) return false;
+    } while (!bar_test(bar, parity));
+    return true;
+}
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sa_of(dst)),

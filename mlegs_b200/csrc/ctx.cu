@@ -1426,7 +1426,7 @@ const char* mlegs_last_error(const mlegs_ctx* ctx) { return ctx ? ctx->err.c_str
 
 int mlegs_set_wait_limit(mlegs_ctx* ctx, int64_t cycles) {
     if (!ctx || cycles < 0) return MLEGS_ERR_ARG;
-    ctx->split_wait = (uint64_t)cycles;
+    ctx->split_wait = ctx->g.wait = ctx->gT.wait = (uint64_t)cycles;
     return MLEGS_OK;
 }
 

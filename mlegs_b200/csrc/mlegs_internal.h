@@ -67,6 +67,7 @@ struct DevGrid {
     const double* pft;      // PF as the bulk-copy RTRAN(+1)'s weight table (null when that form is not used)
     const double* lap;      // -N (N + 1) / ELL2 by degree N = m + n (DELSQH's diagonal)
     int* err;               // the context's error word: set to 1 when a bounded wait runs out
+    uint64_t wait;          // limit of the banded solves' waits in SM cycles (0: about a second)
 };
 
 struct Field {

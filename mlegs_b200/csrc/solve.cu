@@ -366,12 +366,13 @@ struct SolveShared {
     uint64_t* full;   // a chunk has arrived: 32 producer lanes and the bulk copy
     uint64_t* empty;  // the consumer has read it
     uint64_t* whole;  // the staged column of the transposed m = 0 system
-    int* stop;        // a wait ran out
+    uint64_t limit;   // of the two warps' waits (0: WAIT_CYCLES)
 };
 
-// A whole warp's wait; false (for all lanes) when it runs out or the other warp stopped.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, int phase, int* stop) {
-    return __all_sync(0xffffffffu, bar_wait(bar, (uint32_t)(phase & 1))) && !*(volatile int*)stop;
+// A whole warp's wait; false for all lanes when it runs out.  The warp then stops; the
+// other one, which gets no more chunks or no more room, stops at its own next wait.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, int phase, const SolveShared& sh) {
+    return __all_sync(0xffffffffu, bar_wait(bar, (uint32_t)(phase & 1), sh.limit));
 }
 
 // Chunk c of 2 nch: rows [lo, lo + rows), ascending in the first pass, descending in the second.
@@ -386,8 +387,9 @@ __device__ __forceinline__ void solve_chunk(int c, int nch, int size, int& lo, i
     }
 }
 
+// Returns the chunks issued: fewer than 2 nch when a wait ran out.
 template <int HB, bool TR, bool XG>
-__device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, const double* FL, const double* FU,
+__device__ int solve_producer(const DevGrid& g, const double2* src, int nsb, const double* FL, const double* FU,
                                int size, int nn, const SolveShared& sh) {
     constexpr int WL = HB * 16, WU = (HB + 1) * 16, WA = TR ? WU : WL, WB = TR ? WL : WU;
     const int lane = threadIdx.x & 31;
@@ -401,13 +403,9 @@ __device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, co
         copy16_arrive(sh.whole);
     }
     int c = 0;
-    bool ok = true;
     for (; c < 2 * nch; ++c) {
         const int st = c % SNST;
-        if (c >= SNST && !warp_wait(sh.empty + st, c / SNST - 1, sh.stop)) {
-            ok = false;
-            break;
-        }
+        if (c >= SNST && !warp_wait(sh.empty + st, c / SNST - 1, sh)) break;
         int lo, rows;
         solve_chunk(c, nch, size, lo, rows);
         const bool up = c < nch;
@@ -425,13 +423,14 @@ __device__ void solve_producer(const DevGrid& g, const double2* src, int nsb, co
         }
         copy16_arrive(sh.full + st);
     }
-    if (!ok) {  // the copies in flight land before the CTA ends
-        if (lane == 0) {
-            *sh.stop = 1;
-            if (g.err) *g.err = 1;
-        }
-        for (int b = max(0, c - SNST); b < c; ++b) bar_wait(sh.full + b % SNST, (uint32_t)((b / SNST) & 1));
-    }
+    return c;
+}
+
+// After a wait ran out, in the producing warp: its copies in flight land (bounded waits
+// again, at the full limit) before the CTA ends and its shared memory is another's.
+__device__ void solve_drain(int issued, const SolveShared& sh) {
+    for (int b = max(0, issued - SNST); b < issued; ++b) bar_wait(sh.full + b % SNST, (uint32_t)((b / SNST) & 1));
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // HB: half-bandwidth; TR: the transposed system U^T z = y, L^T x = z, else
@@ -474,13 +473,6 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
         if (!XG) X[r * 32] = v;
         else if (live) dc[(size_t)r * st] = v;
     };
-    auto give_up = [&] {
-        if (lane == 0) {
-            *sh.stop = 1;
-            if (g.err) *g.err = 1;
-        }
-        return -1;
-    };
     // column <- A column for a tri-diagonal A of unit diagonal over rows < nn (XM and XM^T);
     // XM^T comes first and takes the right-hand side, which XG reads from src (src may be
     // dst: a row is read before its chunk is written)
@@ -516,7 +508,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
     // neighbouring rows: the column is formed (nn rows, in dst for XG) before the passes
     constexpr bool staged = TR && HB == 3;
     if constexpr (staged) {
-        if (!XG && !warp_wait(sh.whole, 0, sh.stop)) return give_up();
+        if (!XG && !warp_wait(sh.whole, 0, sh)) return -1;
         xm_pass(true);
     }
     // IHELM of a right-hand side with a log term (mod_legops.f90:1244-1255)
@@ -530,7 +522,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
     // factors of the last rows too (column entries of U, of L)
     double v1 = 0.0, v2 = 0.0, v3 = 0.0, a1 = 0.0, a2 = 0.0, a2p = 0.0, a3 = 0.0, a3p = 0.0, a3q = 0.0;
     for (int c = 0; c < nch; ++c) {
-        if (!warp_wait(sh.full + c % SNST, c / SNST, sh.stop)) return give_up();
+        if (!warp_wait(sh.full + c % SNST, c / SNST, sh)) return -1;
         const double* S = sh.ring + (c % SNST) * (SCH * 64);
         const int lo = c * SCH, rows = min(SCH, size - lo);
         double rb[SCH], f[SCH][HB + 1];
@@ -583,7 +575,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
     }
     v1 = v2 = v3 = a1 = a2 = a2p = a3 = a3p = a3q = 0.0;
     for (int c = nch; c < 2 * nch; ++c) {
-        if (!warp_wait(sh.full + c % SNST, c / SNST, sh.stop)) return give_up();
+        if (!warp_wait(sh.full + c % SNST, c / SNST, sh)) return -1;
         int lo, rows;
         solve_chunk(c, nch, size, lo, rows);
         const int hi = lo + rows - 1;
@@ -673,15 +665,20 @@ __device__ __forceinline__ void band_solve(const DevGrid& g, const SolveItem& p,
     const int nsb = min(16, g.NXCHOPDIM - k0);
     const int nn = max(0, g.NRCHOP + fo.pad - m);
     const int size = max(0, (m == 0 && fo.kind == 2) ? nn - 1 : nn);
+    int issued = 0;
     if (threadIdx.x >= 32) {
-        solve_producer<HB, TR, XG>(g, p.src + base, nsb, FL, FU, size, nn, sh);
+        issued = solve_producer<HB, TR, XG>(g, p.src + base, nsb, FL, FU, size, nn, sh);
     } else {
         const int rows = solve_consumer<HB, TR, XG>(g, p, fo, m, k0, nsb, size, nn, sh);
         if (threadIdx.x == 0) rows_sh = rows;
     }
     __syncthreads();
     const int rows_out = rows_sh;
-    if (rows_out < 0) return;
+    if (rows_out < 0) {  // the consumer stops in any case: without the producer's chunks, or by itself
+        if (threadIdx.x == 0 && g.err) *g.err = 1;
+        if (threadIdx.x >= 32) solve_drain(issued, sh);
+        return;
+    }
     const int end = fo.keep_tail ? rows_out : g.NRCHOPDIM, q = threadIdx.x & 15;
     double2* dst = p.dst + base + q;
     if (q >= nsb) return;
@@ -700,7 +697,6 @@ template <bool TR, bool XG>
 __device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p, const SolveForm& fo, int b) {
     extern __shared__ __align__(128) double sms[];
     __shared__ uint64_t bars[2 * SNST + 1];
-    __shared__ int stop;
     const FactorTable ft(g);
     const int m = b / ft.nkb, kb = b - m * ft.nkb;
     const int R = (max(g.NRCHOP + fo.pad, 0) + 1 + SCH - 1) / SCH * SCH;
@@ -712,9 +708,8 @@ __device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p
     sh.full = bars;
     sh.empty = bars + SNST;
     sh.whole = bars + 2 * SNST;
-    sh.stop = &stop;
+    sh.limit = g.wait;
     if (threadIdx.x == 0) {
-        stop = 0;
         for (int q = 0; q < SNST; ++q) {
             bar_init(sh.full + q, 33);
             bar_init(sh.empty + q, 1);
