@@ -330,6 +330,9 @@ int mlegs_ensemble_step(mlegs_ensemble* e, int nsteps, int graph);
 int mlegs_ensemble_tune(mlegs_ensemble* e);
 int mlegs_ensemble_tuning(const mlegs_ensemble* e, int32_t* out, int cap);
 int mlegs_ensemble_ctas(const mlegs_ensemble* e, int32_t* out);
+/* Waits for the device; returns MLEGS_ERR_TIMEOUT (once; mlegs_ensemble_last_error
+ * names the members) when a bounded wait of a member's launches ran out since the
+ * last sync, the grouped launches' included. */
 int mlegs_ensemble_sync(mlegs_ensemble* e);
 int64_t mlegs_ensemble_launch_count(const mlegs_ensemble* e);
 void* mlegs_ensemble_stream(mlegs_ensemble* e);

@@ -80,6 +80,7 @@ struct mlegs_ensemble {
     std::vector<void*> allocs;
     int64_t launches = 0, graph_launches = 0;
     int* d_next = nullptr;  // tile counters of the two GEMM groups
+    int* d_errs = nullptr;  // the members' error words, side by side
     int sms = 148;
     int ctas[2] = {3, 3};
     bool prepared = false, tuned = false;
@@ -621,6 +622,10 @@ int mlegs_ensemble_create(const mlegs_params* p, int n, mlegs_ensemble** out) {
         CK(cudaEventCreateWithFlags(&e->gev, cudaEventDisableTiming));
         CK(cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->dev));
         e->d_next = dalloc<int>(2);
+        e->d_errs = dalloc<int>(e->inst.size());
+        CK(cudaMemset(e->d_errs, 0, e->inst.size() * sizeof(int)));
+        CK(cudaDeviceSynchronize());
+        for (size_t i = 0; i < e->inst.size(); ++i) e->inst[i]->split_err = e->inst[i]->g.err = e->d_errs + i;
         e->st.resize(e->inst.size());
         for (size_t i = 0; i < e->inst.size(); ++i) {
             e->st[i].c = e->inst[i];
@@ -743,7 +748,18 @@ int mlegs_ensemble_ctas(const mlegs_ensemble* e, int32_t* out) {
 }
 
 int mlegs_ensemble_sync(mlegs_ensemble* e) {
-    return eguard(e, [&] { CK(cudaDeviceSynchronize()); });
+    return eguard(e, [&] {
+        CK(cudaDeviceSynchronize());
+        std::vector<int> h(e->inst.size());
+        CK(cudaMemcpy(h.data(), e->d_errs, h.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        std::string who;
+        for (size_t i = 0; i < h.size(); ++i)
+            if (h[i]) who += (who.empty() ? "" : ", ") + std::to_string(i);
+        if (who.empty()) return;
+        CK(cudaMemset(e->d_errs, 0, h.size() * sizeof(int)));
+        throw ApiError(MLEGS_ERR_TIMEOUT,
+                       "ensemble: a bounded pipeline wait timed out (results invalid) in member " + who);
+    });
 }
 
 int64_t mlegs_ensemble_launch_count(const mlegs_ensemble* e) { return e ? e->launches : 0; }
