@@ -1833,11 +1833,12 @@ int mlegs_project(mlegs_ctx* ctx, mlegs_field* rur, mlegs_field* rup, mlegs_fiel
                     h.src[q] = v.dst[q] = in[q]->data;
                     h.dst[q] = t[q]->data;
                     v.src[q] = t[q]->data;
-                    in[q]->space = MLEGS_PFF;
                 }
                 k_horfft_batch(ctx->g, ctx->fft, h, -1, ctx->s);
                 ctx->verfft_batch(v, -1, ctx->s);
                 for (Field* q : t) ctx->rel(q);
+                CK(cudaPeekAtLastError());
+                for (Field* q : in) q->space = MLEGS_PFF;
             }
             ctx->project(a, b2, c, F(psi), F(chi), ln_mode, ln);
             return;
@@ -2350,7 +2351,7 @@ static void user_transform(mlegs_ctx* ctx, Field* f, std::initializer_list<Stage
     // buffer of the result of stage i: the last one is the field's own
     double2* const mid[2] = {t->data, ctx->scratch};
     const double2* src = f->data;
-    int i = 0;
+    int i = 0, space = f->space;
     bool zero_ln = false;  // RTRAN zeroes LN, in both directions
     for (Stage st : stages) {
         double2* dst = (i == n - 1 && n > 1) ? f->data : mid[i];
@@ -2380,10 +2381,12 @@ static void user_transform(mlegs_ctx* ctx, Field* f, std::initializer_list<Stage
             case HORFFT_M: k_horfft_batch(ctx->g, ctx->fft, v, -1, ctx->s); break;
         }
         src = dst;
-        f->space = to[st];
+        space = to[st];
         ++i;
     }
-    if (n == 1) k_copy(f->data, src, ctx->d.elems(f->space), ctx->s);
+    if (n == 1) k_copy(f->data, src, ctx->d.elems(space), ctx->s);
     if (zero_ln) ctx->ln_zero(f);
+    CK(cudaPeekAtLastError());  // a chain that did not run leaves the field in its space
+    f->space = space;
     ctx->rel(t);
 }
