@@ -342,7 +342,8 @@ void k_solve_factor(const DevGrid& g, int kind, double alp, int pad, double* F, 
 // solve at 64x32x32 takes 11.6 us, 17-19 us in the other forms (ncu, cold cache).
 // The blocks run m ascending: longest first.
 // XG: columns too long for shared memory (NRCHOP + pad > 727 rows at SOLVE_SMEM_MAX)
-// stay in global memory, read and written a chunk at a time.
+// stay in global memory, read and written a chunk at a time, and so do the tables: its
+// shared memory is the ring alone, for any number of rows.
 namespace {
 using namespace bulk;
 
@@ -360,8 +361,8 @@ struct SolveForm {
 // xm [R][2]), the column Xs [R][16].
 struct SolveShared {
     double* ring;
-    double* at1;
-    double* xm;
+    const double* at1;
+    const double* xm;
     double2* Xs;
     uint64_t* full;   // a chunk has arrived: 32 producer lanes and the bulk copy
     uint64_t* empty;  // the consumer has read it
@@ -690,7 +691,7 @@ __device__ __forceinline__ void band_solve(const DevGrid& g, const SolveItem& p,
 // doubles of a block's shared memory for columns of `rows` rows (at least SCH, whole chunks)
 __host__ __device__ inline size_t solve_doubles(int rows, bool xg) {
     const int r = (rows + SCH - 1) / SCH * SCH;
-    return SRING + (size_t)(r + 2 * r) + (xg ? 0 : (size_t)r * 32);
+    return SRING + (xg ? 0 : (size_t)r * 35);
 }
 
 template <bool TR, bool XG>
@@ -702,9 +703,10 @@ __device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p
     const int R = (max(g.NRCHOP + fo.pad, 0) + 1 + SCH - 1) / SCH * SCH;
     SolveShared sh;
     sh.ring = sms;
-    sh.at1 = sms + SRING;
-    sh.xm = sh.at1 + R;
-    sh.Xs = (double2*)(sh.xm + 2 * R);
+    double *at1 = sms + SRING, *xm = at1 + R;
+    sh.at1 = XG ? g.at1 : at1;
+    sh.xm = XG ? g.xm : xm;
+    sh.Xs = (double2*)(xm + 2 * R);
     sh.full = bars;
     sh.empty = bars + SNST;
     sh.whole = bars + 2 * SNST;
@@ -720,12 +722,12 @@ __device__ __forceinline__ void solve_block(const DevGrid& g, const SolveItem& p
             for (int j = 0; j < 2; ++j)
                 if (p.ln_dst[j]) *p.ln_dst[j] = *p.ln_src[j];
     }
-    if (m == 0) {  // the tables of the m = 0 tails
+    if (m == 0 && !XG) {  // the tables of the m = 0 tails
         const int nr = min(R, g.NRCHOPDIM);
         if (fo.farfield)
-            for (int r = threadIdx.x; r < nr; r += 64) sh.at1[r] = g.at1[r];
+            for (int r = threadIdx.x; r < nr; r += 64) at1[r] = g.at1[r];
         if (fo.kind == 2)
-            for (int r = threadIdx.x; r < 2 * nr; r += 64) sh.xm[r] = g.xm[r];
+            for (int r = threadIdx.x; r < 2 * nr; r += 64) xm[r] = g.xm[r];
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
