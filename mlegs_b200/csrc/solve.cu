@@ -644,12 +644,21 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
         if (logfix && p.ln_out) *p.ln_out = lnv;
         if (fo.farfield && m == 0 && size > 0) {
             // a(n=0, m=0, k) -= sum_{n < NRCHOP+pad} AT1(n) a(n, 0, k) / AT1(0); the rows
-            // past the system are zero, four partial sums break the chain
+            // past the system are zero, four partial sums break the chain.  XG has FCH rows'
+            // loads in flight (one at a time, the sum was as long as the substitutions)
+            constexpr int FCH = XG ? 32 : SCH;
             double s[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int r0 = 0; r0 < size; r0 += SCH) {
+            for (int r0 = 0; r0 < size; r0 += FCH) {
+                double w[FCH], v[FCH];
 #pragma unroll
-                for (int q = 0; q < SCH; ++q)
-                    if (r0 + q < size) s[q & 3] = __fma_rn(sh.at1[r0 + q], xget(r0 + q), s[q & 3]);
+                for (int q = 0; q < FCH; ++q) {
+                    const int r = min(r0 + q, size - 1);
+                    w[q] = sh.at1[r];
+                    v[q] = xget(r);
+                }
+#pragma unroll
+                for (int q = 0; q < FCH; ++q)
+                    if (r0 + q < size) s[q & 3] = __fma_rn(w[q], v[q], s[q & 3]);
             }
             const double sum = __dadd_rn(__dadd_rn(s[0], s[1]), __dadd_rn(s[2], s[3]));
             xput(0, __dsub_rn(xget(0), __ddiv_rn(sum, sh.at1[0])));
