@@ -84,31 +84,35 @@ void k_chopdo_fff(const DevGrid& g, double2* a, int pad, cudaStream_t s) {
 
 // COPY0 of an FFF field in one pass: dst = src with the entries CHOPDO clears
 // (rows n >= NRCHOPS(m) at pad, m >= NTCHOP) written as zero, LN copied.
-// One warp per (m, n) row: the row's indices are one 32-bit division per lane and cleared
-// rows are not read (two 64-bit divisions per entry before: 25.2 -> 17.6 us at 256x256x256).
+// A team of L lanes (the 8, 16 or 32 that cover a row, L = 32 from 17 modes on) takes a row
+// or, of longer rows, 4 L entries: the row's indices are one 32-bit division per lane and
+// cleared rows are not read (two 64-bit divisions per entry before: 25.2 -> 17.6 us at
+// 256x256x256).  A whole warp per row, however short or long, took 2.1 us for 7,600 rows of
+// 9 modes and 3.2 us for 368 rows of 599, where this takes the 1.5 us of other small fields.
 __global__ void __launch_bounds__(256) copy_chop_fff_kernel(DevGrid g, double2* d, const double2* a, double* dln,
-                                                            const double* aln, int pad) {
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *dln = *aln;
+                                                            const double* aln, int pad, int lg) {
+    const int L = 1 << lg, row = blockIdx.x * (256 >> lg) + (threadIdx.x >> lg), lane = threadIdx.x & (L - 1);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *dln = *aln;
     if (row >= g.NTCHOPDIM * g.NRCHOPDIM) return;
     const int m = row / g.NRCHOPDIM, n = row - m * g.NRCHOPDIM;
     const bool clear = n >= nrchops(g, m, pad) || m >= g.NTCHOP;
     const size_t base = (size_t)row * g.NXCHOPDIM;
-    for (int k0 = lane; k0 < g.NXCHOPDIM; k0 += 32 * COPY_U) {
-        double2 v[COPY_U];
+    const int k0 = blockIdx.y * (L * COPY_U) + lane;
+    double2 v[COPY_U];
 #pragma unroll
-        for (int u = 0; u < COPY_U; ++u) {
-            v[u] = make_double2(0.0, 0.0);
-            if (!clear && k0 + 32 * u < g.NXCHOPDIM) v[u] = a[base + k0 + 32 * u];
-        }
-#pragma unroll
-        for (int u = 0; u < COPY_U; ++u)
-            if (k0 + 32 * u < g.NXCHOPDIM) d[base + k0 + 32 * u] = v[u];
+    for (int u = 0; u < COPY_U; ++u) {
+        v[u] = make_double2(0.0, 0.0);
+        if (!clear && k0 + L * u < g.NXCHOPDIM) v[u] = a[base + k0 + L * u];
     }
+#pragma unroll
+    for (int u = 0; u < COPY_U; ++u)
+        if (k0 + L * u < g.NXCHOPDIM) d[base + k0 + L * u] = v[u];
 }
 void k_copy_chop_fff(const DevGrid& g, double2* dst, const double2* src, double* dln, const double* sln, int pad,
                      cudaStream_t s) {
-    copy_chop_fff_kernel<<<nblk((size_t)g.NTCHOPDIM * g.NRCHOPDIM, 8), 256, 0, s>>>(g, dst, src, dln, sln, pad);
+    const int lg = g.NXCHOPDIM <= 8 ? 3 : g.NXCHOPDIM <= 16 ? 4 : 5;
+    const dim3 grid(nblk((size_t)g.NTCHOPDIM * g.NRCHOPDIM, 256 >> lg), nblk(g.NXCHOPDIM, COPY_U << lg));
+    copy_chop_fff_kernel<<<grid, 256, 0, s>>>(g, dst, src, dln, sln, pad, lg);
     count_launch();
 }
 
