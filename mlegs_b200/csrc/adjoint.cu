@@ -24,6 +24,9 @@
 //   IDEL2LN^T, IHELM^T  U^T then L^T substitutions with the stored factors.
 // The pointwise products' adjoints (VPRODSUB, VDOTPSUB) are kernels here.
 // FP64 contexts only.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include "ctx_internal.h"
 
 namespace mlegs {
@@ -1581,6 +1584,30 @@ int mlegs_energy_objective(mlegs_ctx* ctx, const mlegs_field* psi, const mlegs_f
     });
 }
 
+// [q, q + bytes) lies in one allocation of device `dev`, aligned to `align`.
+static bool in_device(const void* q, size_t bytes, size_t align, int dev) {
+    if ((uintptr_t)q & (align - 1)) return false;
+    static const auto query = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &qr) == cudaSuccess &&
+                        qr == cudaDriverEntryPointSuccess;
+        return ok ? (PFN_cuPointerGetAttributes_v7000)p : nullptr;
+    }();
+    unsigned type = 0, managed = 0;
+    int ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[] = {&type, &managed, &ordinal, &start, &size};
+    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)q;
+    if (!query || query(5, what, out, a) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == dev && a >= start && bytes <= size &&
+           a - start <= size - bytes;
+}
+
 int mlegs_field_device_copy(mlegs_ctx* ctx, mlegs_field* f, int to_field, int space, void* dev, double* ln_dev) {
     return guard(ctx, [&] {
         if (!dev) throw ApiError(MLEGS_ERR_ARG, "mlegs_field_device_copy: null device buffer");
@@ -1588,18 +1615,10 @@ int mlegs_field_device_copy(mlegs_ctx* ctx, mlegs_field* f, int to_field, int sp
         if (to_field && (space < 0 || space > 3))
             throw ApiError(MLEGS_ERR_TRANSFORM, "mlegs_field_device_copy: bad space");
         // this device's memory: data and LN in one launch (two copies cost twice the
-        // gaps around them); anything else (unaligned, host or another device's) by
-        // the runtime's copies
-        auto local = [&](const void* q, size_t align) {
-            if (!q) return true;
-            cudaPointerAttributes a{};
-            if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
-            return a.type == cudaMemoryTypeDevice && a.device == ctx->dev && ((uintptr_t)q & (align - 1)) == 0;
-        };
-        if (local(dev, 16) && local(ln_dev, 8)) {
+        // gaps around them); anything else (unaligned, host or another device's, past
+        // an allocation's end) by the runtime's copies, which take or refuse it
+        const size_t bytes = ctx->d.elems(to_field ? space : fd->space) * sizeof(double2);
+        if (in_device(dev, bytes, 16, ctx->dev) && (!ln_dev || in_device(ln_dev, sizeof(double), 8, ctx->dev))) {
             double2* d = (double2*)dev;
             if (to_field) {
                 k_copy_ln(fd->data, d, ctx->d.elems(space), fd->ln, ln_dev, ctx->s);
