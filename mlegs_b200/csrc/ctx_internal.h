@@ -766,6 +766,7 @@ inline int guard(mlegs_ctx* ctx, F&& fn) {
         ctx->set_error(e.what());
         rc = MLEGS_ERR_STATE;
     }
+    if (rc != MLEGS_OK) cudaGetLastError();  // reported: not the next call's
     g_launch_counter = prev;
     g_allocs = prev_allocs;
     return rc;

@@ -588,6 +588,7 @@ int eguard(mlegs_ensemble* e, Fn&& fn) {
         e->err = x.what();
         rc = MLEGS_ERR_STATE;
     }
+    if (rc != MLEGS_OK) cudaGetLastError();  // reported: not the next call's
     g_launch_counter = prev;
     g_allocs = prev_allocs;
     return rc;

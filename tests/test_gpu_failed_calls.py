@@ -85,3 +85,15 @@ def test_project(env):
         U.append(A)
     P, C = L.project(g, *U, 0.0)
     assert rel(psi.download()[0], P.E) < 1e-11 and rel(chi.download()[0], C.E) < 1e-11
+
+
+def test_an_error_is_reported_once(env):
+    """What a refused call leaves in the runtime is not the next call's error."""
+    M, ctx, g = env
+    f = ctx.field(M.FFF).upload(random_fff(g, 95).E, 0.4, M.FFF)
+    with InvalidCapture(ctx) as _:
+        with pytest.raises(M.MlegsError):
+            ctx.TOFP(f)
+        assert ctypes.CDLL("libcudart.so.12").cudaPeekAtLastError() == 0
+    ctx.TOFP(f)
+    ctx.sync()
