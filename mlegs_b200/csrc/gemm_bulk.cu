@@ -196,11 +196,11 @@ __global__ void __launch_bounds__((BNW + 1) * 32, MTW <= 3 ? 3 : 2)
                 ok = false;
             }
         }
-        if (!ok && lane == 0) {
-            // drain: the copies of stages handed over and possibly unconsumed land
-            // before the CTA's shared memory is released (bounded waits)
+        if (lane == 0) {
+            // drain: the copies of stages handed over land before the CTA's shared memory is
+            // released, whether or not a consumer stays to wait for them (bounded waits)
             for (int c = max(0, seq - NST); c < seq; ++c) bar_wait(full + (c % NST), (uint32_t)((c / NST) & 1));
-            atomicExch(&g_bulk_err, 1);
+            if (!ok) atomicExch(&g_bulk_err, 1);
         }
         return;
     }
@@ -445,9 +445,9 @@ __global__ void __launch_bounds__((FNW + 1) * 32, 3) fold_bulk_kernel(DevGrid g,
                 ok = false;
             }
         }
-        if (!ok && lane == 0) {
+        if (lane == 0) {  // drain, as in b2p_bulk_kernel
             for (int c = max(0, seq - NST); c < seq; ++c) bar_wait(full + (c % NST), (uint32_t)((c / NST) & 1));
-            atomicExch(&g_bulk_err, 1);
+            if (!ok) atomicExch(&g_bulk_err, 1);
         }
         return;
     }
