@@ -101,6 +101,12 @@ int mlegs_sync(mlegs_ctx* ctx);
  * what it has in flight, frees its tensor memory and returns, and the next
  * mlegs_sync reports MLEGS_ERR_TIMEOUT; used to test that error path. */
 int mlegs_set_wait_limit(mlegs_ctx* ctx, int64_t cycles);
+/* Fields that TOFP of several fields (CALC_BOUSSI_FORCE, the steps) takes per
+ * launch and stage: set for n > 0 (at most the number whose images the context
+ * holds: all ten, fewer on grids whose images would take more than 8 GiB), and
+ * returned.  Results do not depend on it; lets a test run the groups of a large
+ * grid on a small one. */
+int mlegs_tofp_group(mlegs_ctx* ctx, int n);
 /* Sizes (NDIMR, NDIMTH, NX, NRCHOPDIM, NTCHOPDIM, NXCHOPDIM, NRH, NR, NTH). */
 int mlegs_dims(const mlegs_ctx* ctx, int32_t out[9]);
 

@@ -48,6 +48,7 @@ SIGNATURES = {
     "mlegs_last_error": (c_char_p, [c_void_p]),
     "mlegs_sync": (c_int, [c_void_p]),
     "mlegs_set_wait_limit": (c_int, [c_void_p, c_int64]),
+    "mlegs_tofp_group": (c_int, [c_void_p, c_int]),
     "mlegs_dims": (c_int, [c_void_p, ctypes.POINTER(ctypes.c_int32)]),
     "mlegs_field_alloc": (c_int, [c_void_p, c_int, ctypes.POINTER(c_void_p)]),
     "mlegs_field_free": (c_int, [c_void_p, c_void_p]),

@@ -12,7 +12,8 @@ thread_local std::vector<void*>* mlegs_host::g_allocs = nullptr;
 
 // TOFP of several fields (tofp_pipe) goes in one launch per stage while the PFF images
 // between the stages stay within PIPE_BYTES, 5% of the device's memory; larger grids run
-// groups of PIPE_MIN fields.  One launch was the faster form at every size measured
+// groups of PIPE_MIN fields, or of the 3 to 5 whose images fit in three field buffers.
+// One launch was the faster form at every size measured
 // (CALC_BOUSSI_FORCE, against groups of three with the two stages on two streams, which
 // held as many images as PIPE_MIN): 61 against 81 us at 64x32x32, 218 against 236 us at
 // 100x64x128, 478 against 501 us at 128x128x128, 1447 against 1481 us at 192x128x256.
@@ -431,10 +432,12 @@ void mlegs_ctx::init(const mlegs_params& prm) {
     lnslots = dalloc<double>(nslots);
     CK(cudaMemsetAsync(lnslots, 0, nslots * sizeof(double), s));
     scratch = dalloc<double2>(d.cap());
-    pipe_group = BATCH * d.pff() * sizeof(double2) <= PIPE_BYTES ? BATCH : PIPE_MIN;
+    pipe_images = BATCH * d.pff() * sizeof(double2) <= PIPE_BYTES ? BATCH
+                                                                 : std::min<int>(PIPE_MIN, 3 * d.cap() / d.pff());
+    pipe_group = pipe_images;
     {
-        double2* slab = dalloc<double2>(pipe_group * d.pff());
-        for (int q = 0; q < pipe_group; ++q) pbuf[q] = slab + q * d.pff();
+        double2* slab = dalloc<double2>(pipe_images * d.pff());
+        for (int q = 0; q < pipe_images; ++q) pbuf[q] = slab + q * d.pff();
     }
     size_t nsys = (size_t)d.NTCHOPDIM * d.NXCHOPDIM;
     solve_scr = dalloc<double>((size_t)d.NRCHOPDIM * 4 * nsys);
@@ -1428,6 +1431,12 @@ int mlegs_set_wait_limit(mlegs_ctx* ctx, int64_t cycles) {
     if (!ctx || cycles < 0) return MLEGS_ERR_ARG;
     ctx->split_wait = ctx->g.wait = ctx->gT.wait = (uint64_t)cycles;
     return MLEGS_OK;
+}
+
+int mlegs_tofp_group(mlegs_ctx* ctx, int n) {
+    if (!ctx || n < 0) return -1;
+    if (n > 0) ctx->pipe_group = std::min(n, ctx->pipe_images);
+    return ctx->pipe_group;
 }
 
 int mlegs_sync(mlegs_ctx* ctx) {

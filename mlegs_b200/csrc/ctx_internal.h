@@ -69,9 +69,9 @@ struct mlegs_ctx {
     cudaStream_t s2 = nullptr;         // second stream (nonlin, the ETD step's PC2VOR)
     cudaEvent_t evs[64] = {};          // fork/join events, used in rotation
     int ev_next = 0;
-    // TOFP of several fields (tofp_pipe): fields per launch, and as many PFF images
-    // between RTRAN(+1) and VERFFT(+1)
-    int pipe_group = 1;
+    // TOFP of several fields (tofp_pipe): fields per launch, and the PFF images between
+    // RTRAN(+1) and VERFFT(+1), at least as many
+    int pipe_group = 1, pipe_images = 1;
     double2* pbuf[BATCH] = {};
     int dev = 0;
     std::string err;
@@ -347,7 +347,7 @@ struct mlegs_ctx {
                    const double2* const* src = nullptr, const double* const* ln = nullptr) {
         if (!src)
             for (int i = 0; i < n; ++i) require(fs[i], MLEGS_FFF, "RTRAN");
-        const int step = split_S ? 3 : pipe_group;
+        const int step = split_S ? std::min(3, pipe_group) : pipe_group;
         if (split_S) order(s, s2);
         for (int i0 = 0, img = 0; i0 < n; i0 += step, img += step) {
             const int cnt = std::min(step, n - i0);
