@@ -13,10 +13,10 @@ thread_local std::vector<void*>* mlegs_host::g_allocs = nullptr;
 // TOFP of several fields (tofp_pipe) goes in one launch per stage while the PFF images
 // between the stages stay within PIPE_BYTES, 5% of the device's memory; larger grids run
 // groups of PIPE_MIN fields, or of the 3 to 5 whose images fit in three field buffers.
-// One launch was the faster form at every size measured
-// (CALC_BOUSSI_FORCE, against groups of three with the two stages on two streams, which
-// held as many images as PIPE_MIN): 61 against 81 us at 64x32x32, 218 against 236 us at
-// 100x64x128, 478 against 501 us at 128x128x128, 1447 against 1481 us at 192x128x256.
+// One launch for all is the fastest form at every size: CALC_BOUSSI_FORCE in groups of 10,
+// 6 and 3 (a graph of ten calls, one context) takes 45.5, 51.1 and 63.5 us at 64x32x32, 188,
+// 194 and 213 us at 100x64x128, 460, 465 and 480 us at 128x128x128, 1428, 1438 and 1451 us
+// at 192x128x256.
 static constexpr size_t PIPE_BYTES = (size_t)8 << 30;
 static constexpr int PIPE_MIN = 6;
 
@@ -973,8 +973,9 @@ void mlegs_ctx::hyp3adj(const Field* PSI, const Field* CHI, const Field* B) {
 void mlegs_ctx::nonlin(const Field* B, Field* RUR, Field* RUP, Field* UZ, Field* ROR, Field* ROP, Field* OZ,
                        Field* BN, cudaEvent_t vor_ready, Field* PSIN, Field* CHIN) {
     Field *RBR = tmp(), *RBP = tmp(), *BZ = tmp();
-    // GRAD(B) on s2, beside the first RTRAN(+1) GEMMs on s; ROR, ROP, OZ may
-    // still be in the making on s2 (vor_ready)
+    // GRAD(B) on s2, beside the first RTRAN(+1) GEMMs on s where those are one launch a
+    // field (split-BF16; the FP64 form's one launch waits for every field); ROR, ROP, OZ
+    // may still be in the making on s2 (vor_ready)
     cudaEvent_t ef = next_event();
     CK(cudaEventRecord(ef, s));
     CK(cudaStreamWaitEvent(s2, ef, 0));
@@ -1307,7 +1308,7 @@ void mlegs_ctx::step_etdab_cn() {
     }
     Field *RURN = tmp(), *RUPN = tmp(), *UZN = tmp(), *RORN = tmp(), *ROPN = tmp(), *OZN = tmp(), *BN = tmp();
     pc2vel(psi, chi, RURN, RUPN, UZN, 3);
-    // PC2VOR on s2: the RTRAN(+1) of the velocity starts beside it
+    // PC2VOR on s2: the split-BF16 RTRAN(+1) of the velocity starts beside it
     cudaEvent_t ef = next_event();
     CK(cudaEventRecord(ef, s));
     CK(cudaStreamWaitEvent(s2, ef, 0));

@@ -110,7 +110,7 @@ struct mlegs_ctx {
     int split_S = 0;                 // slices per operand; 0 = FP64 GEMMs
     uint8_t* split_img = nullptr;    // PF slice images for RTRAN(+1)
     int* split_eA = nullptr;         // PF row scale exponents
-    int* split_err = nullptr;        // raised by a timed-out wait in a tensor-core kernel
+    int* split_err = nullptr;        // raised by a timed-out wait in a split GEMM or a banded solve
     uint64_t split_wait = 0;         // limit of those waits in SM cycles (0: the kernel's default)
     uint8_t* fimg[4] = {};           // weight slice images: 0 PF (RTRAN -1), 1 V, 2 D, 3 T (PROJECT)
     int* feA[4] = {};

@@ -10,15 +10,15 @@
 // ordinary context (its own fields, tables and streams), and a step is cut at
 // those calls into five phases:
 //   0  GRAD / PC2VEL / PC2VOR at CHOPSET(3), W = B            | grouped RTRAN(+1) x 10
-//   1  VERFFT(+1), theta stage, VERFFT(-1), VEL2PLN             | grouped PROJECT folds + RTRAN(-1)
-//   2  far-field fix, B_N                                       | grouped IDEL2LN solves
+//   1  VERFFT(+1), theta stage, VERFFT(-1)                      | grouped PROJECT folds + RTRAN(-1)
+//   2  VEL2PLN, far-field fix                                   | grouped IDEL2LN solves
 //   3  AB2 update, history, VISC2 right-hand sides (DEL2)       | grouped IHELM solves
-//   4  CHOPDO, CALC_BOUSSI_HYPERV
+//   4  CALC_BOUSSI_HYPERV
 // The per-instance work of a phase runs on each instance's stream; each
 // grouped launch runs on the ensemble's stream after all instances reach it,
 // over every instance's problems at once: persistent CTAs take (problem, m,
 // column tile) work items from a global counter (gemm_dmma.cu), the solves one
-// block per 64 systems (solve.cu).  The arithmetic is the single-grid path's,
+// block per 16 systems (solve.cu).  The arithmetic is the single-grid path's,
 // tile for tile.  A step is captured once as a CUDA graph over all streams.
 //
 // Autotuner: the column-tile width of each class of GEMM problems -- key
@@ -208,7 +208,7 @@ void phase0(mlegs_ensemble& E, EnsInst& I) {
 }
 
 // Phase 1: VERFFT(+1) of the ten images, the theta stage with the linear terms,
-// PROJECT's VERFFT(-1) and VEL2PLN, TOFF(B_N) up to PFF; fold problems.
+// the four VERFFT(-1); fold problems (PROJECT, RTRAN(-1) of B_N).
 void phase1(mlegs_ensemble& E, EnsInst& I) {
     mlegs_ctx* c = I.c;
     const DevGrid& g = c->g;

@@ -587,9 +587,9 @@ void launch_b2p_bulk_n(const DevGrid& g, const B2PBatch& f, int per_sm, cudaStre
     count_launch();
 }
 
-// Three stages at three CTAs per SM (55 KB each at MTW = 3) leave room on every
-// SM for a VERFFT(+1) CTA, which runs beside the GEMM on the other stream in
-// TOFP; four stages filled the SM (545 vs 541 steps/s at 192x128x256).
+// Three stages of the ring (55 KB a CTA at MTW = 3): a fourth is worth 0.3% of a
+// 256x256x256 round trip and 0.5% of a right-hand side at 100x64x128 (558.5 against 556.5 us,
+// 169.0 against 168.2), and nothing in the ETD step at 192x128x256 (1723 us with either).
 template <int MTW>
 void launch_b2p_bulk(const DevGrid& g, const B2PBatch& f, cudaStream_t s) {
     launch_b2p_bulk_n<MTW, 3>(g, f, MTW <= 3 ? 3 : 2, s);

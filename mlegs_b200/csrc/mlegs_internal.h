@@ -189,9 +189,12 @@ struct SolveBatch {
 // PFF line, stride NXCHOPDIM) applied to PSI's (0, 0) column, and the far-field fix of
 // PSI's m = 0 columns over NRCHOP rows.  VEL2PLN adds PLN u to the line before the
 // products, a fixed u: dvec is the change of PSI's column per unit of PLN.
-// CALC_BOUSSI_FORCE returns PSI as it is.  Where PSI goes on through PC2VEL and IDEL2LN
-// (the ETD step, PROJECT itself) the line is changed before the products, as the formulas
-// stand: IDEL2LN magnifies a last-bit change some 1e5 times.
+// CALC_BOUSSI_FORCE, made of launches as short as these two, takes this form.  The two
+// formulas differ in PSI's last bits, which an AB2-CN run carries on into the next step:
+// 1e-15 to 6e-13 of the fields over ten steps, errors against 64-bit references the same.
+// PROJECT and the ETD step change the line before the products, as the formulas stand: there
+// IDEL2LN takes PSI's change on in the same step and magnifies it to 4e-10 of the field's
+// largest value at 192x128x256.
 struct ProjectTail {
     double2* psi;
     const double2* line;
@@ -239,7 +242,8 @@ void k_fold_table(const DevGrid& g, const double* W, int src_rows, int wt_rows, 
 bool fold_bulk_supported(const DevGrid& g, int wt_rows);
 void k_fold_bulk(const DevGrid& g, const FoldSeg* seg, const int* first, int nout, double2* const* outs, int wt_rows,
                  const int* pads, int accumulate, cudaStream_t s);
-// FP64 tensor-path (mma.sync m8n8k4.f64) forms used by k_rtran_b2p / k_fold_gemm when supported.
+// FP64 tensor-path (mma.sync m8n8k4.f64) form that k_fold_gemm takes when supported, where
+// the bulk-copy one above has no table or is not.
 bool dmma_supported(const DevGrid& g);
 void k_fold_gemm_dmma(const DevGrid& g, const double* Wt, int wt_rows, const double2* in, double2* out, int mode,
                       int scale, int accumulate, int pad, cudaStream_t s);
