@@ -376,6 +376,15 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, int phase, const SolveS
     return __all_sync(0xffffffffu, bar_wait(bar, (uint32_t)(phase & 1), sh.limit));
 }
 
+// The stage back to the producing warp, whose next bulk copy writes over it through the
+// async proxy: every lane's reads, which may still be in flight here (their values are used
+// further down), come before that by the fence.
+__device__ __forceinline__ void give_back(uint64_t* empty) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) bar_arrive(empty);
+}
+
 // Chunk c of 2 nch: rows [lo, lo + rows), ascending in the first pass, descending in the second.
 __device__ __forceinline__ void solve_chunk(int c, int nch, int size, int& lo, int& rows) {
     if (c < nch) {
@@ -534,8 +543,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
             if constexpr (TR) row_u(S + q * WU, f[q]);
             else row_l(S + q * WL, f[q]);
         }
-        __syncwarp();
-        if (lane == 0) bar_arrive(sh.empty + c % SNST);
+        give_back(sh.empty + c % SNST);
         if (logfix && c == 0) {
             const double cf[3] = {4.0 / 3, -2.0, 2.0 / 3};
 #pragma unroll
@@ -589,8 +597,7 @@ __device__ int solve_consumer(const DevGrid& g, const SolveItem& p, const SolveF
             if constexpr (TR) row_l(S + (r - lo) * WL, f[q]);
             else row_u(S + (r - lo) * WU, f[q]);
         }
-        __syncwarp();
-        if (lane == 0) bar_arrive(sh.empty + c % SNST);
+        give_back(sh.empty + c % SNST);
         if constexpr (!TR) {
 #pragma unroll
             for (int q = 0; q < SCH; ++q) vb[q] = __dmul_rn(vb[q], f[q][0]);
